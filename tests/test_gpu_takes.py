@@ -195,3 +195,17 @@ def test_exclusive_scan_matches_cumsum(cuda, n):
                "fbp_scan_i32")
     ref = np.concatenate([[0], np.cumsum(x, dtype=np.int64)]).astype(np.int32)
     np.testing.assert_array_equal(out.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("m,n", [(1, 1), (12288, 5000), (12289, 5000)])
+def test_points_per_box_counts(cuda, m, n):
+    """model_count against numpy, up to the most boxes counted in shared
+    memory and one more: the first box holds every point, the others a few."""
+    rng = np.random.default_rng(m)
+    lo = np.concatenate([[0.0], rng.uniform(0, 1, m - 1)]).astype(np.float32).reshape(m, 1)
+    hi = np.concatenate([[1.0], lo[1:, 0] + 1e-3]).astype(np.float32).reshape(m, 1)
+    x = rng.uniform(0, 1, (n, 1)).astype(np.float32)
+    t = T.PointTakes(T.grid_of(boxes_static(lo, hi)), n)
+    t.build(torch.from_numpy(x).cuda())
+    ref = np.array([((x >= lo[j]) & (x <= hi[j])).sum() for j in range(m)])
+    np.testing.assert_array_equal(_np(t.model_count), ref)
