@@ -120,6 +120,7 @@ struct Cfg {
     static constexpr int NS = d2_slots(D2);
     static constexpr int J = 1 + XD + NS;
     static constexpr bool TWO = H2 > 0;
+    static constexpr bool W2S = TWO;          // SParams holds W2
     static constexpr int HL = TWO ? H2 : H1;  // width feeding the output layer
     // packed layout per layer: W (fan_out, fan_in), b (fan_out), then EXTRA
     // vectors (fan_out) of activation parameters (the output layer's unused)
@@ -145,6 +146,14 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
+
+// tanh_fast of two values (the same results)
+__device__ __forceinline__ float2 tanh_fast2(float2 x) {
+    const float2 e = make_float2(ex2_ftz(fabsf(x.x) * kTanhScale), ex2_ftz(fabsf(x.y) * kTanhScale));
+    const float2 d = add2(e, dup2(1.0f)), n = fma2(e, dup2(-1.0f), dup2(1.0f));
+    const float2 t = mul2(n, make_float2(rcp_ftz(d.x), rcp_ftz(d.y)));
+    return make_float2(copysignf(t.x, x.x), copysignf(t.y, x.y));
+}
 
 // Work-item schedule of the persistent jet kernels: with pr.item_ctr null CTA b
 // takes items b, b + gridDim.x, ...; otherwise each CTA takes the next index
@@ -177,8 +186,8 @@ struct SParams {
     float cw[C::H1 * C::XD];   // W1[n][d] / sd[d]: first-layer tangent along d
     float c2[C::H1 * (C::NS > 0 ? C::NS : 1)];  // per slot s: sum of cw[n][d]^2 over its dims
     // 16-byte aligned: the layer-2 loops read pairs of neighbouring weights
-    alignas(16) float W2t[C::TWO ? C::H1 * C::H2 : 4];  // [n][k]
-    alignas(16) float W2[C::TWO ? C::H2 * C::H1 : 4];   // [k][n]
+    alignas(16) float W2t[C::W2S ? C::H1 * C::H2 : 4];  // [n][k]
+    alignas(16) float W2[C::W2S ? C::H2 * C::H1 : 4];   // [k][n]
     alignas(16) float b2[C::TWO ? C::H2 : 4];
     alignas(16) float W3[C::HL];
     float b3;
@@ -212,11 +221,13 @@ __device__ __forceinline__ void load_params(SParams<C>& S, const fbp_net& net, i
     for (int i = threadIdx.x; i < C::H1 * C::XD; i += blockDim.x) S.W1[i] = th[C::oW1 + i];
     for (int i = threadIdx.x; i < C::H1; i += blockDim.x) S.b1[i] = th[C::ob1 + i];
     if constexpr (C::TWO) {
-        for (int i = threadIdx.x; i < C::H2 * C::H1; i += blockDim.x) {
-            const float v = th[C::oW2 + i];
-            const int k = i / C::H1, n = i - k * C::H1;
-            S.W2[i] = v;
-            if constexpr (W2T) S.W2t[n * C::H2 + k] = v;
+        if constexpr (C::W2S) {
+            for (int i = threadIdx.x; i < C::H2 * C::H1; i += blockDim.x) {
+                const float v = th[C::oW2 + i];
+                const int k = i / C::H1, n = i - k * C::H1;
+                S.W2[i] = v;
+                if constexpr (W2T) S.W2t[n * C::H2 + k] = v;
+            }
         }
         for (int i = threadIdx.x; i < C::H2; i += blockDim.x) S.b2[i] = th[C::ob2 + i];
     }
@@ -405,11 +416,10 @@ __device__ __forceinline__ void window_1d(const SParams<C>& S, int d, float xn, 
     }
 }
 
+// The window's jet from its 1D factors (value, first and second derivative per dim).
 template <class C>
-__device__ __forceinline__ void window_jet(const SParams<C>& S, const float (&xn)[C::XD], float (&w)[C::J]) {
-    float c0[C::XD], c1[C::XD], c2[C::XD];
-#pragma unroll
-    for (int d = 0; d < C::XD; ++d) window_1d<C>(S, d, xn[d], c0[d], c1[d], c2[d]);
+__device__ __forceinline__ void window_product(const SParams<C>& S, const float (&c0)[C::XD], const float (&c1)[C::XD],
+                                               const float (&c2)[C::XD], float (&w)[C::J]) {
     float prod = 1.f;
 #pragma unroll
     for (int d = 0; d < C::XD; ++d) prod *= c0[d];
@@ -437,6 +447,14 @@ __device__ __forceinline__ void window_jet(const SParams<C>& S, const float (&xn
             }
         w[1 + C::XD + s] = f * acc;
     }
+}
+
+template <class C>
+__device__ __forceinline__ void window_jet(const SParams<C>& S, const float (&xn)[C::XD], float (&w)[C::J]) {
+    float c0[C::XD], c1[C::XD], c2[C::XD];
+#pragma unroll
+    for (int d = 0; d < C::XD; ++d) window_1d<C>(S, d, xn[d], c0[d], c1[d], c2[d]);
+    window_product<C>(S, c0, c1, c2, w);
 }
 
 // Jet of the product u w (first J entries of a pair record).

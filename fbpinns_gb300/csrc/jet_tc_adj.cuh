@@ -1,255 +1,175 @@
-// Tensor-core (tcgen05, 3xTF32) variant of the per-pair adjoint kernel for
-// tanh networks with two 16-wide hidden layers.
+// Tensor-core (tcgen05, 3xTF32) per-pair adjoint for tanh networks with two
+// hidden layers of equal width H = 16 or 32.
 //
-// The adjoint recomputes each pair's layer-2 pre-activation jet z_c =
-// W2 v_c (+ b2) before back-propagating through it.  That contraction is the
-// forward's: J GEMMs of M = 128 pairs, N = 16, K = 16 per tile with the
-// pair-dependent A operands a, tp, tpp of the first layer and the per-neuron
-// scales folded into B_c = W2 diag(f_c) (see jet_tc.cuh).  Here it runs on the
-// tensor cores; per tile of 128 pairs (thread = pair = TMEM lane):
+// Of the adjoint's three layer-2 contractions, two have the pairs as rows and
+// run on the tensor cores with the pair-dependent operand in tensor memory
+// (the thread of a pair writes its own TMEM lane, so it costs no shared-memory
+// traffic, and an MMA with A in TMEM takes N/2 cycles where one with A in
+// shared memory takes at least 40):
+//   GEMM 1  z_c = B_c v      B_c = W2 diag(f_c), v = a, tp or tpp of layer 1,
+//           f_c = 1, W1[:, d] / sd_d, or the slot's sum of their squares
+//   GEMM 2  T_0 = W2^T z2bar_0, T_1 = sum_d B_{1+d}^T z2bar_{1+d},
+//           T_2 = sum_s B_s^T z2bar_s
+// With T the layer-1 adjoint is z1bar = T_0 tp + T_1 tpp + T_2 tppp per neuron
+// (tpp = -2 a tp with the -2 in the B operands); vbar is not formed.  The third contraction sums over the pairs,
+//   S_c[k][n] = sum_pairs z2bar_c[k] m_c[n],   m = a, tp or tpp,
+// and runs on warp-level MMAs (mma.sync, 3xTF32) from shared-memory rows while
+// GEMM 2 is under way: tcgen05 would want at least 64 rows (c, k) by all three
+// m, so that two thirds of its products are thrown away, with both operands
+// split and transposed in shared memory (21 cycles per pair at H = 32, J = 4,
+// against 24); packed FP32 FMAs need 1.1 words of shared memory per FMA pair
+// and lane, over twice what it delivers (0.465 ms instead of 0.373 at
+// 2.34e6 pairs, H = 16).  From S follow, once per work item,
+//   W2bar = sum_c f_c S_c   and the tangent part of W1bar,
+//   sum_pairs cwbar_d[n] = sum_k W2[k][n] (S_{1+d} + 2 cw_d sum_{s with d} S_s).
 //
-//   stage A: seeds -> o-bar (registers); layer 1 -> the a1 row and the A
-//            operands; one thread issues the MMAs of the tile into TMEM
-//   wait for the MMAs (bounded), tcgen05.ld the z-jets
-//   phase A2: tanh jets of layer 2 and their adjoint -> z2-bar rows, the
-//            W3-bar and b3-bar sums
-//   phases B, C (each warp on its 32 pairs): v-bar = W2^T z2-bar and the
-//            layer-1 adjoint; W2-bar.
+// A tile is 128 pairs; NPT = H / 8 threads share a pair (eight neurons each),
+// so a CTA has 256 or 512 threads, two CTAs or one fill an SM's tensor memory,
+// and 16 warps are resident.  The sums over pairs stay in registers for the
+// whole work item (S_c as 4 x 2 blocks per lane, the biases', W3's and W1's
+// value part per thread) and are reduced once, in a fixed order.
 //
-// Phases B and C, the W3/W1/bias reduce-scatters and the per-item gradient
-// partials are those of adjoint_pairs_kernel (jet.cuh); the z-jets come from
-// the tensor cores instead of FFMA2 loops, so the CUDA cores drop a third of
-// their layer-2 FMAs.  Three CTAs share an SM (about 74 KB of shared memory
-// each: the z2-bar rows reuse the A-operand region), so CUDA-core phases run
-// while other CTAs wait for their MMAs.  Waits on the MMA-completion mbarrier are bounded as in the forward
-// kernel: on a time-out the CTA records FBP_STATUS_TC_TIMEOUT, stops, waits
-// once more and frees its TMEM.
+// What bounds it: issue slots (51% busy at H = 16, 43% at H = 32: elementwise
+// jets, splits, the S_c loop) with 16 warps to hide the tiles' barriers; for
+// H = 32 also the warp-level MMAs of S_c (24 cycles per pair at J = 4).
+// Measured on a GB300, against the FMA adjoint (jet.cuh): 2.34e6 pairs of
+// 2-16-16-1 networks, J = 4, 0.466 -> 0.337 ms; a training step of 4096
+// networks 2-32-32-1 on 2.1e6 points 17.0 -> 11.9 ms, of 900 networks 3-32-32-1
+// (J = 6) on 58^3 points 6.44 -> 4.40 ms with the same forward.
+//
+// Waits on the MMA-completion mbarriers are bounded: on a time-out the kernel
+// records FBP_STATUS_TC_TIMEOUT, stops, waits once more and frees its TMEM.
 #pragma once
 
-#include "jet_tc.cuh"
+#include "tc_ops.cuh"
 
 namespace fbp {
 
 template <class C>
+struct TcAdj {
+    static_assert(C::TWO && C::H1 == C::H2 && (C::H1 == 16 || C::H1 == 32) && C::EXTRA == 0 && C::J <= 6,
+                  "tensor-core adjoint shape");
+    static constexpr int H = C::H1, J = C::J, XD = C::XD, NS = C::NS;
+    static constexpr int NPT = H / 8;      // threads per pair
+    static constexpr int T = 128 * NPT;    // threads per CTA
+    static constexpr int NW = T / 32;
+    static constexpr int NA = NS > 0 ? 3 : 2;  // A operands a, tp (, tpp); also the GEMM 2 groups
+    static constexpr int OP = 2 * H;           // TMEM columns of an operand: hi, lo
+    // TMEM columns: [A operands | z | (z2bar operands past the NA-th) | T].  z2bar
+    // operands 0 .. NA-1 take the A operands' columns (free once GEMM 1 is
+    // done); the others follow z where the columns suffice, else they take z's
+    // own columns after a barrier (OVER).
+    static constexpr int COLS = 16 * H;
+    static constexpr int MORE = (J > NA ? J - NA : 0) * OP;
+    static constexpr bool OVER = NA * OP + J * H + MORE + NA * H > COLS;
+    static constexpr int cZ = NA * OP;
+    static constexpr int cM = OVER ? cZ : cZ + J * H;
+    static constexpr int cT = OVER ? cZ + J * H : cM + MORE;
+    static_assert(cT + NA * H <= COLS && (!OVER || MORE <= J * H), "TMEM columns");
+    __host__ __device__ static constexpr int zcol(int c) { return c < NA ? c * OP : cM + (c - NA) * OP; }
+    // shared-memory rows: z2bar [c][k] (row stride 4 mod 32 words: 16-byte
+    // accesses of eight consecutive rows hit different banks), a [n]
+    static constexpr int ZS = (J * H + 31) / 32 * 32 + 4, AS = H + 4;
+    // S_c blocks: a warp has 16 k x 8 NQ n (NQ = 1 where J blocks of two would
+    // not fit the registers); SUB warps cover H x H, PG groups of warps split
+    // the tile's pairs
+    static constexpr int NQ = J > 4 ? 1 : 2;
+    static constexpr int KB = H / 16, SUB = KB * (H / (8 * NQ)), PG = NW / SUB, PPG = 128 / PG;
+    // per-thread sums of b1 and W1's value part, kept in shared memory between
+    // tiles (as float4, conflict-free) where it has the room
+    static constexpr int NST = 2 * (1 + XD);
+    static constexpr int BASE = 4 * (4 * J * H * H + 128 * (ZS + AS) + 2 * (XD + J) * 128 + 4 * NPT * 48);
+    static constexpr bool STASH = BASE + NST * T * 16 <= (H == 16 ? 110 : 222) * 1024;
+};
+
+template <class C>
 struct TcAdjSmem {
-    static_assert(C::TWO && C::H1 == 16 && C::H2 == 16 && C::J <= 8 && C::EXTRA == 0, "tensor-core adjoint shape");
-    static constexpr int COLS = pow2_at_least(C::J * 16 < 32 ? 32 : C::J * 16);  // one z-jet accumulator set
-    static constexpr int NA = TcSmem<C>::NA;
-    float a[NA][2][TC_TILE * 16];  // A operands a, tp (, tpp): hi, lo
-    float b[C::J][2][16 * 16];     // B_c = W2 diag(f_c): hi, lo
-    uint64_t mbar;
+    using A = TcAdj<C>;
+    float b1[2][A::J * A::H * A::H];  // GEMM 1 B (hi, lo): component c's rows k at c H + k, K = n
+    float b2[2][A::J * A::H * A::H];  // GEMM 2 B: component c's H x H matrix, rows n, K = k
+    float zb[128 * A::ZS];            // z2bar rows; at the item's end the S_c of the pair groups
+    float a1[128 * A::AS];            // layer-1 activations
+    float xo[2][A::XD + A::J][128];   // per pair of this and the next tile: normalised point, o-bar jet
+    float red[4 * A::NPT][48];        // per warp: the item's sums over its lanes
+    float4 stash[A::STASH ? A::NST : 1][A::STASH ? A::T : 1];
+    float red3[4];
+    uint64_t mbar[2];
     uint32_t tmem_base;
-    uint32_t pad_;
 };
 
-// One warp's rows and gradient sums (the warp owns 32 lanes = pairs of a
-// tile).  Its z2-bar rows live in the A-operand region of TcAdjSmem: they are
-// written after the tile's MMAs have completed and read before the next tile
-// is staged, so the two never hold data at the same time.
-template <class C>
-struct __align__(16) TcAdjWarp {
-    float a1[32 * AdjW<C>::AS];  // layer-1 activations [t][n]
-    float gW2[C::H2 * C::H1];
-    float gW1[C::H1 * C::XD];
-    float gb1[C::H1];
-    float gb2[C::H2];
-    float gW3[C::HL];
-    float gb3;
-};
-
-// Phase B of one warp tile: v-bar = W2^T z2-bar (own row), the layer-1 jet
-// adjoint, and the W1-bar / b1-bar terms summed over the warp.
-template <class C>
-__device__ __forceinline__ void tc_adj_phase_b(const SParams<C>& S, TcAdjWarp<C>& R, const float* zb,
-                                               const float* a1row, bool act, const float (&xn)[C::XD], int lane) {
-    using A = AdjW<C>;
-    constexpr int J = C::J, XD = C::XD, H1 = C::H1, H2 = C::H2;
-    constexpr int RN = XD + 1;
-    constexpr int NC = 32 / RN >= 8 ? 8 : 4;
-    static_assert(NC * RN <= 32 && H1 % NC == 0 && NC % 2 == 0, "layer-1 chunk");
-#pragma unroll 1
-    for (int n0 = 0; n0 < H1; n0 += NC) {
-        float r1[32];
+// The MMAs of one operand group, issued by one thread: GEMM 1's operand o
+// (value, tangents or second derivatives) or GEMM 2's group g.  Small
+// products first, so that the large ones are added (and rounded) last.
+template <class C, int O>
+__device__ __forceinline__ void tc_adj_issue1(uint32_t tmem, uint32_t b_hi, uint32_t b_lo) {
+    using A = TcAdj<C>;
+    constexpr int H = A::H, c0 = O == 0 ? 0 : (O == 1 ? 1 : 1 + A::XD), nc = O == 0 ? 1 : (O == 1 ? A::XD : A::NS);
+    constexpr uint32_t idesc = umma_idesc_tf32(128, nc * H), rows = (uint32_t)(c0 * (H / 8)) * KMajor<H>::SBO;
+    const uint32_t d = tmem + A::cZ + c0 * H, a = tmem + O * A::OP;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) r1[i] = 0.f;
-        if (act) {
-            float2 vb2[NC / 2][J];
+    for (int p = 0; p < 3; ++p)
 #pragma unroll
-            for (int q = 0; q < NC / 2; ++q)
-#pragma unroll
-                for (int c = 0; c < J; ++c) vb2[q][c] = make_float2(0.f, 0.f);
-            const float* zrow = zb + lane * A::ZS;
-#pragma unroll 1
-            for (int k0 = 0; k0 < H2; k0 += 4) {
-                float4 z4[J];
-#pragma unroll
-                for (int c = 0; c < J; ++c) z4[c] = *reinterpret_cast<const float4*>(zrow + c * H2 + k0);
-#pragma unroll
-                for (int kq = 0; kq < 4; ++kq) {
-                    const float2* w2 = reinterpret_cast<const float2*>(&S.W2[(k0 + kq) * H1 + n0]);
-#pragma unroll
-                    for (int q = 0; q < NC / 2; ++q) {
-                        const float2 w = w2[q];
-#pragma unroll
-                        for (int c = 0; c < J; ++c) {
-                            const float zc = kq == 0 ? z4[c].x : kq == 1 ? z4[c].y : kq == 2 ? z4[c].z : z4[c].w;
-                            vb2[q][c] = fma2(w, make_float2(zc, zc), vb2[q][c]);
-                        }
-                    }
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < NC; ++q) {
-                const int n = n0 + q;
-                float vb[J];
-#pragma unroll
-                for (int c = 0; c < J; ++c) vb[c] = (q & 1) ? vb2[q / 2][c].y : vb2[q / 2][c].x;
-                float a, tp, tpp, tppp;
-                C::AF1::derivs(a1row[n], 1.0f, 1.0f, a, tp, tpp, tppp);
-                float tpb = 0.f, tppb = 0.f, cwb[XD];
-#pragma unroll
-                for (int d = 0; d < XD; ++d) {
-                    tpb += vb[1 + d] * S.cw[n * XD + d];
-                    cwb[d] = vb[1 + d] * tp;
-                }
-#pragma unroll
-                for (int s = 0; s < C::NS; ++s) {
-                    const float g = vb[1 + XD + s];
-                    tppb += g * S.c2[n * C::NS + s];
-#pragma unroll
-                    for (int d = 0; d < XD; ++d)
-                        if ((C::slot_dims(s) >> d) & 1) cwb[d] += 2.0f * g * tpp * S.cw[n * XD + d];
-                }
-                const float z1b = vb[0] * tp + tpb * tpp + tppb * tppp;
-#pragma unroll
-                for (int d = 0; d < XD; ++d) r1[q * RN + d] = fmaf(z1b, xn[d], cwb[d] * S.inv_sd[d]);
-                r1[q * RN + XD] = z1b;
-            }
-        }
-        warp_reduce_scatter<32>(r1, lane);
-        if (lane < NC * RN) {
-            const int q = lane / RN, d = lane - q * RN;
-            if (d < XD)
-                R.gW1[(n0 + q) * XD + d] += r1[0];
-            else
-                R.gb1[n0 + q] += r1[0];
-        }
-    }
+        for (int ks = 0; ks < H / 8; ++ks)
+            umma_tf32_ta(d, a + (p == 0 ? H : 0) + 8 * ks,
+                         umma_desc((p == 1 ? b_lo : b_hi) + rows + ks * 256, KMajor<H>::LBO, KMajor<H>::SBO), idesc,
+                         p + ks > 0);
 }
 
-// Phase C of one warp tile: W2-bar and b2-bar over its nt pairs (lane = a
-// KB x NB block of W2-bar; rows in pairs share packed FMAs).
-template <class C>
-__device__ __forceinline__ void tc_adj_phase_c(const SParams<C>& S, TcAdjWarp<C>& R, const float* zb,
-                                               const float* a1rows, int nt, int lane) {
-    using A = AdjW<C>;
-    constexpr int J = C::J, XD = C::XD, H1 = C::H1, H2 = C::H2;
-#pragma unroll 1
-    for (int ps = 0; ps < A::PASSES; ++ps) {
-        const int b = ps * 32 + lane;
-        if (b >= A::NBLK) continue;
-        const int nb = b % (H1 / A::NB), kb = b / (H1 / A::NB);
-        const int n0 = nb * A::NB, k0 = kb * A::KB;
-        float2 sacc[A::KB / 2][A::NB][J];
+template <class C, int G>
+__device__ __forceinline__ void tc_adj_issue2(uint32_t tmem, uint32_t b_hi, uint32_t b_lo) {
+    using A = TcAdj<C>;
+    constexpr int H = A::H, c0 = G == 0 ? 0 : (G == 1 ? 1 : 1 + A::XD), nc = G == 0 ? 1 : (G == 1 ? A::XD : A::NS);
+    constexpr uint32_t idesc = umma_idesc_tf32(128, H);
+    const uint32_t d = tmem + A::cT + G * H;
 #pragma unroll
-        for (int i = 0; i < A::KB / 2; ++i)
+    for (int p = 0; p < 3; ++p)
 #pragma unroll
-            for (int q = 0; q < A::NB; ++q)
+        for (int c = c0; c < c0 + nc; ++c)
 #pragma unroll
-                for (int c = 0; c < J; ++c) sacc[i][q][c] = make_float2(0.f, 0.f);
-        float b2s[A::KB];
-#pragma unroll
-        for (int i = 0; i < A::KB; ++i) b2s[i] = 0.f;
-        constexpr int UC = FBP_ADJ_UNROLL_C;  // (pragma arguments are not macro-expanded)
-#pragma unroll UC
-        for (int t = 0; t < nt; ++t) {
-            float m[A::NB][3];
-#pragma unroll
-            for (int q = 0; q < A::NB; ++q) {
-                float a, tp, tpp, tppp;
-                C::AF1::derivs(a1rows[t * A::AS + n0 + q], 1.0f, 1.0f, a, tp, tpp, tppp);
-                m[q][0] = a;
-                m[q][1] = tp;
-                m[q][2] = tpp;
-            }
-            const float* zr = zb + t * A::ZS + k0;
-#pragma unroll
-            for (int c = 0; c < J; ++c) {
-                float2 z2[A::KB / 2];
-                if constexpr (A::KB == 2) {
-                    z2[0] = *reinterpret_cast<const float2*>(zr + c * H2);
-                } else {
-#pragma unroll
-                    for (int h = 0; h < A::KB / 4; ++h) {
-                        const float4 z4 = *reinterpret_cast<const float4*>(zr + c * H2 + 4 * h);
-                        z2[2 * h] = make_float2(z4.x, z4.y);
-                        z2[2 * h + 1] = make_float2(z4.z, z4.w);
-                    }
-                }
-                const int mi = c == 0 ? 0 : (c <= XD ? 1 : 2);
-                if (c == 0) {
-#pragma unroll
-                    for (int i = 0; i < A::KB / 2; ++i) {
-                        b2s[2 * i] += z2[i].x;
-                        b2s[2 * i + 1] += z2[i].y;
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < A::NB; ++q) {
-                    const float2 mm = make_float2(m[q][mi], m[q][mi]);
-#pragma unroll
-                    for (int i = 0; i < A::KB / 2; ++i) sacc[i][q][c] = fma2(z2[i], mm, sacc[i][q][c]);
-                }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < A::KB; ++i)
-#pragma unroll
-            for (int q = 0; q < A::NB; ++q) {
-                const int n = n0 + q;
-                float s[J];
-#pragma unroll
-                for (int c = 0; c < J; ++c) s[c] = (i & 1) ? sacc[i / 2][q][c].y : sacc[i / 2][q][c].x;
-                float v = s[0];
-#pragma unroll
-                for (int d = 0; d < XD; ++d) v = fmaf(S.cw[n * XD + d], s[1 + d], v);
-#pragma unroll
-                for (int ss = 0; ss < C::NS; ++ss) v = fmaf(S.c2[n * C::NS + ss], s[1 + XD + ss], v);
-                R.gW2[(k0 + i) * H1 + n] += v;
-            }
-        if (nb == 0) {
-#pragma unroll
-            for (int i = 0; i < A::KB; ++i) R.gb2[k0 + i] += b2s[i];
-        }
-    }
+            for (int ks = 0; ks < H / 8; ++ks)
+                umma_tf32_ta(d, tmem + A::zcol(c) + (p == 0 ? H : 0) + 8 * ks,
+                             umma_desc((p == 1 ? b_lo : b_hi) + c * H * H * 4 + ks * 256, KMajor<H>::LBO,
+                                       KMajor<H>::SBO),
+                             idesc, p + (c - c0) + ks > 0);
 }
 
+// Runs F<0>, F<1> (, F<2>) on lane 0 of warps 0, 1 (, 2): one thread needs about
+// 45 cycles per MMA it issues, so the groups go out in parallel.
+#define FBP_TC_ISSUE(F, hi, lo, bar)                            \
+    if (lane == 0 && warp < A::NA && !test_no_mma) {            \
+        if (warp == 0) F<C, 0>(tmem, hi, lo);                   \
+        if (warp == 1) F<C, 1>(tmem, hi, lo);                   \
+        if constexpr (A::NA > 2)                                \
+            if (warp == 2) F<C, A::NA - 1>(tmem, hi, lo);       \
+        umma_commit(bar);                                       \
+    }
+
 template <class C>
-__global__ void __launch_bounds__(TC_TILE) adjoint_pairs_tc_kernel(fbp_net net, const float* __restrict__ x,
-                                                                    fbp_pairs pr, const float* __restrict__ slot_out,
-                                                                    float* __restrict__ grad_part,
-                                                                    int32_t* __restrict__ status) {
-    using A = AdjW<C>;
-    constexpr int J = C::J, XD = C::XD, H1 = 16, H2 = 16, RS = rec_stride(J);
-    constexpr int NA = TcAdjSmem<C>::NA;
-    static_assert(sizeof(TcAdjWarp<C>) % 16 == 0 && A::ZS % 4 == 0, "16-byte rows");
-    static_assert((TC_TILE / 32) * 32 * A::ZS <= (int)sizeof(TcAdjSmem<C>::a) / 4, "z2-bar rows fit the A region");
+__global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kernel(fbp_net net,
+                                                                                    const float* __restrict__ x,
+                                                                                    fbp_pairs pr,
+                                                                                    const float* __restrict__ slot_out,
+                                                                                    float* __restrict__ grad_part,
+                                                                                    int32_t* __restrict__ status) {
+    using A = TcAdj<C>;
+    constexpr int J = C::J, XD = C::XD, NS = C::NS, H = A::H, RS = rec_stride(J), NPT = A::NPT, NA = A::NA;
+    static_assert(A::PG * J * H * H <= 128 * A::ZS && J * H * (H + 1) <= 128 * A::ZS, "S_c fit the z2bar rows");
     __shared__ SParams<C> S;
+    __shared__ int s_item;
     extern __shared__ float4 dyn_smem[];
     TcAdjSmem<C>& T = *reinterpret_cast<TcAdjSmem<C>*>(dyn_smem);
-    TcAdjWarp<C>* RW = reinterpret_cast<TcAdjWarp<C>*>(reinterpret_cast<char*>(dyn_smem) +
-                                                       ((sizeof(TcAdjSmem<C>) + 15) / 16) * 16);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    TcAdjWarp<C>& R = RW[warp];
-    float* zb = &T.a[0][0][0] + warp * 32 * A::ZS;  // this warp's z2-bar rows (in the A region)
-    const uint32_t mbar = smem_u32(&T.mbar);
+    const int h = warp >> 2, r = (warp & 3) * 32 + lane;  // neurons [8h, 8h + 8) of the tile's pair r
+    const int n0 = 8 * h;
+    const uint32_t mbar1 = smem_u32(&T.mbar[0]), mbar2 = smem_u32(&T.mbar[1]);
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar1), "r"(NA) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar2), "r"(NA) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&T.tmem_base)),
-                     "r"(TcAdjSmem<C>::COLS)
+                     "r"(A::COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -257,274 +177,441 @@ __global__ void __launch_bounds__(TC_TILE) adjoint_pairs_tc_kernel(fbp_net net, 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = T.tmem_base;
-    constexpr uint32_t idesc = umma_idesc_tf32(TC_TILE, H2);
+    const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)n0;  // this thread's lane and columns
+    const uint32_t b1h = smem_u32(&T.b1[0][0]), b1l = smem_u32(&T.b1[1][0]);
+    const uint32_t b2h = smem_u32(&T.b2[0][0]), b2l = smem_u32(&T.b2[1][0]);
     const bool test_no_mma = (*(volatile int32_t*)status & FBP_STATUS_TC_TEST_NO_MMA) != 0;
     const uint64_t wait_ns = test_no_mma ? TC_TEST_WAIT_NS : TC_WAIT_NS;
+    // this lane's block of the S_c loop
+    const int sk = 16 * (warp % A::SUB % A::KB) + (lane >> 2), sn = 8 * A::NQ * (warp % A::SUB / A::KB);
+    const int sp = (warp / A::SUB) * A::PPG;  // first pair of the warp's group
     uint32_t phase = 0;
     bool failed = false;
-    __shared__ int s_item;
     const int nit = (int)min((int64_t)*pr.n_items, pr.items_cap);
-    for (int it = first_item(pr, &s_item); it < nit && !failed; it = next_item(pr, it, &s_item)) {
+    int next;  // the item after this one, claimed at this one's start (see first_item)
+    for (int it = first_item(pr, &s_item); it < nit && !failed; it = next) {
         const int j = pr.items[3 * (size_t)it], beg = pr.items[3 * (size_t)it + 1], cnt = pr.items[3 * (size_t)it + 2];
+        const float* __restrict__ w2g = net.theta + (size_t)j * C::P + C::oW2;
+        constexpr int PT = H * H / A::T;  // entries of W2 per thread
+        int4 rec = make_int4(0, 0, -1, 0);
+        float xr[XD] = {}, w2[PT];
+        float4 sd[(J + 3) / 4] = {};
+        if (h == 0 && r < cnt) rec = pair_rec(pr, beg + r);
+#pragma unroll
+        for (int e = 0; e < PT; ++e) {
+            int k, n;
+            KMajor<H>::at(tid + e * A::T, k, n);
+            w2[e] = w2g[k * H + n];
+        }
         __syncthreads();
-        load_params<C>(S, net, j);
-        for (int i = tid; i < J * H2 * H1; i += blockDim.x) {  // B_c = W2 diag(f_c), hi / lo
-            const int c = i / (H2 * H1), r = i - c * (H2 * H1);
-            const int k = r / H1, n = r - k * H1;
-            float f = 1.0f;
-            if (c >= 1 && c <= XD) f = S.cw[n * XD + (c - 1)];
-            if (c > XD) f = S.c2[n * C::NS + (c - 1 - XD)];
-            float hi, lo;
-            split_tf32(S.W2[r] * f, hi, lo);
-            const uint32_t off = kmajor16_off(k, n) >> 2;
-            T.b[c][0][off] = hi;
-            T.b[c][1][off] = lo;
-        }
-        for (int i = lane; i < H2 * H1; i += 32) R.gW2[i] = 0.f;
-        for (int i = lane; i < H1 * XD; i += 32) R.gW1[i] = 0.f;
-        if (lane < H1) R.gb1[lane] = 0.f;
-        if (lane < H2) R.gb2[lane] = 0.f;
-        if (lane < H2) R.gW3[lane] = 0.f;
-        if (lane == 0) R.gb3 = 0.f;
-        // the first tile's pair (later tiles are prefetched while MMAs run)
-        int4 rec_n = make_int4(0, 0, -1, 0);
-        float xr_n[XD];
-#pragma unroll
-        for (int d = 0; d < XD; ++d) xr_n[d] = 0.f;
-        if (tid < cnt) {
-            rec_n = pair_rec(pr, beg + tid);
-#pragma unroll
-            for (int d = 0; d < XD; ++d) xr_n[d] = x[(size_t)rec_n.y * XD + d];
-        }
-        const int ntile = (cnt + TC_TILE - 1) / TC_TILE;
-        for (int ti = 0; ti < ntile; ++ti) {
-            const int t0 = ti * TC_TILE;
-            const bool act = t0 + tid < cnt;
-            const int nt = max(0, min(32, cnt - (t0 + warp * 32)));  // pairs of this warp's part
+        if (tid == 0 && pr.item_ctr) s_item = atomicAdd(pr.item_ctr, 1);
+        // pair t of the item: normalised point and o-bar jet (from the seeds of its slot)
+        auto prep = [&](int buf, bool act) {
             float xn[XD], ob[J];
 #pragma unroll
-            for (int d = 0; d < XD; ++d) xn[d] = (xr_n[d] - S.mu[d]) * S.inv_sd[d];
+            for (int d = 0; d < XD; ++d) xn[d] = act ? (xr[d] - S.mu[d]) * S.inv_sd[d] : 0.f;
 #pragma unroll
             for (int c = 0; c < J; ++c) ob[c] = 0.f;
-            float* a1row = &R.a1[lane * A::AS];
-            // every warp has read its z2-bar rows (the previous tile's phase C)
-            // before the A operands overwrite that region
-            __syncthreads();
-            // ---- stage A: seeds -> o-bar; layer 1 -> A operands and a1 row ----
             if (act) {
-                float w[J];
+                float w[J], nb[J], ub[J];
                 window_jet<C>(S, xn, w);
-                const int slot = rec_n.z;
-                const bool ok = slot >= 0 && slot < pr.slots_cap;  // overflowed slots carry no seed
-                float nb[J];
-                const float4* src = reinterpret_cast<const float4*>(slot_out + (size_t)(ok ? slot : 0) * RS);
+                const bool ok = rec.z >= 0 && rec.z < pr.slots_cap;  // overflowed slots carry no seed
 #pragma unroll
-                for (int q = 0; q < (J + 3) / 4; ++q) {
-                    const float4 v = src[q];
-                    if (4 * q + 0 < J) nb[4 * q + 0] = ok ? v.x : 0.f;
-                    if (4 * q + 1 < J) nb[4 * q + 1] = ok ? v.y : 0.f;
-                    if (4 * q + 2 < J) nb[4 * q + 2] = ok ? v.z : 0.f;
-                    if (4 * q + 3 < J) nb[4 * q + 3] = ok ? v.w : 0.f;
+                for (int c = 0; c < J; ++c) {
+                    const float4 v = sd[c / 4];
+                    nb[c] = !ok ? 0.f : (c % 4 == 0 ? v.x : c % 4 == 1 ? v.y : c % 4 == 2 ? v.z : v.w);
                 }
-                float ub[J];
                 product_jet_adj<C>(nb, w, ub);
 #pragma unroll
                 for (int c = 0; c < J; ++c) ob[c] = ub[c] * S.sd_u;
             }
 #pragma unroll
-            for (int n4 = 0; n4 < H1; n4 += 4) {
-                float2 av[NA][2];
+            for (int d = 0; d < XD; ++d) T.xo[buf][d][r] = xn[d];
 #pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const int n = n4 + 2 * q;
+            for (int c = 0; c < J; ++c) T.xo[buf][XD + c][r] = ob[c];
+        };
+        auto fetch = [&]() {
+#pragma unroll
+            for (int d = 0; d < XD; ++d) xr[d] = x[(size_t)rec.y * XD + d];
+            const bool ok = rec.z >= 0 && rec.z < pr.slots_cap;
+            const float4* src = reinterpret_cast<const float4*>(slot_out + (size_t)(ok ? rec.z : 0) * RS);
+#pragma unroll
+            for (int q = 0; q < (J + 3) / 4; ++q) sd[q] = src[q];
+        };
+        if (h == 0 && r < cnt) fetch();
+        load_params<C, false>(S, net, j);
+        if (h == 0) prep(0, r < cnt);  // the first tile's pairs
+        // B operands
+#pragma unroll
+        for (int e = 0; e < PT; ++e) {
+            const int o = tid + e * A::T;
+            int k, n;
+            KMajor<H>::at(o, k, n);
+            const int ot = KMajor<H>::off(n, k);
+#pragma unroll
+            for (int c = 0; c < J; ++c) {
+                const float f = c == 0 ? 1.0f : (c <= XD ? S.cw[n * XD + (c - 1)] : S.c2[n * NS + (c - 1 - XD)]);
+                float hi, lo;
+                split_tf32_rn(w2[e] * f, hi, lo);
+                // the factor -2 of tpp = -2 a tp: with the second-derivative
+                // operands of GEMM 1, with the tangents of GEMM 2 (T_1 tpp)
+                const float s1 = c > XD ? -2.0f : 1.0f, s2 = c >= 1 && c <= XD ? -2.0f : 1.0f;
+                T.b1[0][c * H * H + o] = s1 * hi;  // rows k, K = n
+                T.b1[1][c * H * H + o] = s1 * lo;
+                T.b2[0][c * H * H + ot] = s2 * hi;  // rows n, K = k
+                T.b2[1][c * H * H + ot] = s2 * lo;
+            }
+        }
+        if (h == 1 && 128 + r < cnt) rec = pair_rec(pr, beg + 128 + r);  // the second tile's pairs
+        fence_async_smem();
+        float sacc[J][A::NQ][4];  // S_c, 16 k x 8 NQ n as MMA accumulators (c > XD: over tpp / -2)
+        float2 g3[4], gb2[4], gb1[4], gw1[XD][4];
+        float g3b = 0.f;
+#pragma unroll
+        for (int c = 0; c < J; ++c)
+#pragma unroll
+            for (int q = 0; q < A::NQ; ++q)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) sacc[c][q][i] = 0.f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            g3[q] = gb2[q] = gb1[q] = dup2(0.f);
+#pragma unroll
+            for (int d = 0; d < XD; ++d) gw1[d][q] = dup2(0.f);
+        }
+        auto stash = [&](bool load) {  // gb1 and gw1 from / to shared memory
+#pragma unroll
+            for (int i = 0; i < A::NST; ++i) {
+                float2(&v)[4] = i < 2 ? gb1 : gw1[i < 2 ? 0 : i / 2 - 1];
+                if (load) {
+                    const float4 w = T.stash[A::STASH ? i : 0][A::STASH ? tid : 0];
+                    v[2 * (i & 1)] = make_float2(w.x, w.y);
+                    v[2 * (i & 1) + 1] = make_float2(w.z, w.w);
+                } else {
+                    T.stash[A::STASH ? i : 0][A::STASH ? tid : 0] =
+                        make_float4(v[2 * (i & 1)].x, v[2 * (i & 1)].y, v[2 * (i & 1) + 1].x, v[2 * (i & 1) + 1].y);
+                }
+            }
+        };
+        if constexpr (A::STASH) stash(false);
+        __syncthreads();
+        const int ntile = (cnt + 127) / 128;
+        for (int ti = 0; ti < ntile; ++ti) {
+            const int buf = ti & 1;
+            float* zrow = &T.zb[r * A::ZS + n0];
+            float* arow = &T.a1[r * A::AS + n0];
+            // the next tile's pairs: the groups of threads take turns; the record was
+            // fetched a tile ago
+            const bool mypre = ti + 1 < ntile && h == (ti + 1) % NPT, nact = (ti + 1) * 128 + r < cnt;
+            if (mypre && nact) fetch();
+            // ---- layer 1 of this thread's neurons -> A operands and the a row ----
+            {
+                float a[8], tp[8], tpp[8];
+                float xn[XD];
+#pragma unroll
+                for (int d = 0; d < XD; ++d) xn[d] = T.xo[buf][d][r];
+#pragma unroll
+                for (int q = 0; q < 8; q += 2) {
+                    const int n = n0 + q;
                     float2 z = *reinterpret_cast<const float2*>(&S.b1[n]);
 #pragma unroll
                     for (int d = 0; d < XD; ++d)
                         z = fma2(make_float2(S.W1[n * XD + d], S.W1[(n + 1) * XD + d]), dup2(xn[d]), z);
-                    const float2 a = make_float2(tanh_fast(z.x), tanh_fast(z.y));
-                    const float2 tp = fma2(make_float2(-a.x, -a.y), a, dup2(1.0f));
-                    av[0][q] = a;
-                    av[1][q] = tp;
-                    if constexpr (NA > 2) av[NA - 1][q] = mul2(mul2(dup2(-2.0f), a), tp);
-                    a1row[n] = a.x;
-                    a1row[n + 1] = a.y;
-                }
-                const uint32_t off = kmajor16_off(tid, n4) >> 2;
-#pragma unroll
-                for (int o = 0; o < NA; ++o) {
-                    float2 h[2], l[2];
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        h[q] = make_float2(__uint_as_float(__float_as_uint(av[o][q].x) & 0xFFFFE000u),
-                                           __uint_as_float(__float_as_uint(av[o][q].y) & 0xFFFFE000u));
-                        l[q] = add2(av[o][q], make_float2(-h[q].x, -h[q].y));  // v - hi, exact
+                    const float2 av = tanh_fast2(z);
+                    const float2 t1 = fma2(make_float2(-av.x, -av.y), av, dup2(1.0f));
+                    a[q] = av.x, a[q + 1] = av.y;
+                    tp[q] = t1.x, tp[q + 1] = t1.y;
+                    if constexpr (NS > 0) {
+                        const float2 t2 = mul2(av, t1);  // tpp / -2; the factor is in B
+                        tpp[q] = t2.x, tpp[q + 1] = t2.y;
                     }
-                    *reinterpret_cast<float4*>(&T.a[o][0][off]) = make_float4(h[0].x, h[0].y, h[1].x, h[1].y);
-                    *reinterpret_cast<float4*>(&T.a[o][1][off]) = make_float4(l[0].x, l[0].y, l[1].x, l[1].y);
                 }
+                *reinterpret_cast<float4*>(arow) = make_float4(a[0], a[1], a[2], a[3]);
+                *reinterpret_cast<float4*>(arow + 4) = make_float4(a[4], a[5], a[6], a[7]);
+                tmem_st_split8(mine, H, a);
+                tmem_st_split8(mine + A::OP, H, tp);
+                if constexpr (NS > 0) tmem_st_split8(mine + 2 * A::OP, H, tpp);
             }
-            fence_async_smem();
+            tmem_wait_st();
             tc_fence_before();
             __syncthreads();
             tc_fence_after();
-            if (tid == 0 && !test_no_mma) {
-#pragma unroll
-                for (int c = 0; c < J; ++c) {
-                    const int o = tc_a_of<C>(c);
-                    const uint32_t ah = smem_u32(&T.a[o][0][0]), al = smem_u32(&T.a[o][1][0]);
-                    const uint32_t bh = smem_u32(&T.b[c][0][0]), bl = smem_u32(&T.b[c][1][0]);
-                    const uint32_t d = tmem + (uint32_t)(c * 16);
-#pragma unroll
-                    for (int ks = 0; ks < 2; ++ks) {
-                        const uint32_t ko = ks * 256;  // two 16-byte K chunks per MMA (K = 8)
-                        umma_tf32(d, umma_desc(ah + ko, 128, 512), umma_desc(bh + ko, 128, 512), idesc, ks > 0);
-                        umma_tf32(d, umma_desc(ah + ko, 128, 512), umma_desc(bl + ko, 128, 512), idesc, 1);
-                        umma_tf32(d, umma_desc(al + ko, 128, 512), umma_desc(bh + ko, 128, 512), idesc, 1);
-                    }
-                }
-                umma_commit(mbar);
-            }
-            // prefetch the next tile's pair while the MMAs run
-            const int tn = t0 + TC_TILE + tid;
-            if (tn < cnt) {
-                rec_n = pair_rec(pr, beg + tn);
-#pragma unroll
-                for (int d = 0; d < XD; ++d) xr_n[d] = x[(size_t)rec_n.y * XD + d];
-            }
-            // ---- wait for the tile's z-jets (the verdict is CTA-uniform) ----
-            failed = __syncthreads_or(!mbar_wait_bounded(mbar, phase, wait_ns));
-            if (failed) {
-                if (tid == 0) atomicOr(status, FBP_STATUS_TC_TIMEOUT);
-                break;
-            }
-            phase ^= 1u;
+            FBP_TC_ISSUE(tc_adj_issue1, b1h, b1l, mbar1)
+            __syncwarp();
+            if (mypre) prep(buf ^ 1, nact);
+            // (a time-out counts at the tile's last barrier, where the verdict is CTA-uniform)
+            bool late = !mbar_wait_warp(mbar1, phase, wait_ns, lane);
             tc_fence_after();
-            // ---- phase A2: tanh jets of layer 2 and their adjoint -> z2-bar rows ----
+            // ---- tanh jets of layer 2 and their adjoint -> z2bar ----
             {
-                float acc[J][16];
+                float acc[J][8];
 #pragma unroll
-                for (int c = 0; c < J; ++c)
-                    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c * 16), acc[c]);
+                for (int c = 0; c < J; ++c) tmem_ld8(mine + A::cZ + c * H, acc[c]);
                 tmem_wait_ld();
-                float e3[16];
-                float* zrow = zb + lane * A::ZS;
+                if constexpr (A::OVER) {  // every thread has read its z before z2bar takes the columns
+                    tc_fence_before();
+                    __syncthreads();
+                    tc_fence_after();
+                }
+                float ob[J];
 #pragma unroll
-                for (int k = 0; k < H2; k += 2) {
+                for (int c = 0; c < J; ++c) ob[c] = T.xo[buf][XD + c][r];
+                if (h == 0) g3b += ob[0];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int k = n0 + 2 * q;
                     float2 z[J];
 #pragma unroll
-                    for (int c = 0; c < J; ++c) z[c] = make_float2(acc[c][k], acc[c][k + 1]);
+                    for (int c = 0; c < J; ++c) z[c] = make_float2(acc[c][2 * q], acc[c][2 * q + 1]);
                     z[0] = add2(z[0], *reinterpret_cast<const float2*>(&S.b2[k]));
-                    const float2 a = make_float2(tanh_fast(z[0].x), tanh_fast(z[0].y));
+                    const float2 a = tanh_fast2(z[0]);
                     const float2 tp = fma2(make_float2(-a.x, -a.y), a, dup2(1.0f));
-                    const float2 tpp = mul2(mul2(dup2(-2.0f), a), tp);
-                    // tppp = tp (6 a^2 - 2)
-                    const float2 tppp = mul2(tp, fma2(mul2(dup2(6.0f), a), a, dup2(-2.0f)));
-                    float2 q2[C::NS > 0 ? C::NS : 1];  // sum of z_d^2 over each slot's dims
-                    float2 g[J];
-                    g[0] = a;
-#pragma unroll
-                    for (int d = 0; d < XD; ++d) g[1 + d] = mul2(tp, z[1 + d]);
-#pragma unroll
-                    for (int s = 0; s < C::NS; ++s) {
-                        float2 q = dup2(0.f);
-#pragma unroll
-                        for (int d = 0; d < XD; ++d)
-                            if ((C::slot_dims(s) >> d) & 1) q = fma2(z[1 + d], z[1 + d], q);
-                        q2[s] = q;
-                        g[1 + XD + s] = fma2(tp, z[1 + XD + s], mul2(tpp, q));
-                    }
-                    // W3-bar terms sum_c ob_c g_c and the sensitivities gb_c = W3 ob_c
-                    float2 s3 = dup2(0.f);
-#pragma unroll
-                    for (int c = 0; c < J; ++c) s3 = fma2(dup2(ob[c]), g[c], s3);
-                    e3[k] = s3.x;
-                    e3[k + 1] = s3.y;
+                    const float2 m2 = mul2(a, tp), tpp = mul2(dup2(-2.0f), m2);
+                    const float2 tppp = mul2(tp, fma2(dup2(-6.0f), tp, dup2(4.0f)));  // tp (6 a^2 - 2), a^2 = 1 - tp
+                    // the sensitivities of sigma' and sigma'' over W3: P = sum_d ob_d z_d +
+                    // sum_s ob_s z_s, Q = sum_s ob_s sum_d z_d^2; then W3-bar += ob_0 a +
+                    // tp P + tpp Q, z2bar_0 = W3 (ob_0 tp + tpp P + tppp Q), z2bar_d =
+                    // W3 (ob_d tp + 2 ob_s tpp z_d), z2bar_s = W3 ob_s tp
                     const float2 w3 = *reinterpret_cast<const float2*>(&S.W3[k]);
-                    float2 gb[J];
+                    const float2 wtp = mul2(w3, tp), w4 = mul2(dup2(-4.0f), mul2(w3, m2));  // 2 W3 tpp
+                    float2 P = mul2(dup2(ob[1]), z[1]), Q = dup2(0.f), zb[J];
 #pragma unroll
-                    for (int c = 0; c < J; ++c) gb[c] = mul2(w3, dup2(ob[c]));
-                    // adjoint of the tanh jet (tanh_jet_adj, two neurons at once)
-                    float2 tpb = dup2(0.f), tppb = dup2(0.f), zb[J];
+                    for (int d = 1; d < XD; ++d) P = fma2(dup2(ob[1 + d]), z[1 + d], P);
 #pragma unroll
-                    for (int d = 0; d < XD; ++d) {
-                        tpb = fma2(gb[1 + d], z[1 + d], tpb);
-                        zb[1 + d] = mul2(gb[1 + d], tp);
-                    }
+                    for (int d = 0; d < XD; ++d) zb[1 + d] = mul2(dup2(ob[1 + d]), wtp);
 #pragma unroll
-                    for (int s = 0; s < C::NS; ++s) {
-                        const float2 gs = gb[1 + XD + s];
-                        tpb = fma2(gs, z[1 + XD + s], tpb);
-                        zb[1 + XD + s] = mul2(gs, tp);
-                        tppb = fma2(gs, q2[s], tppb);
-                        const float2 g2 = mul2(mul2(dup2(2.0f), gs), tpp);
+                    for (int s = 0; s < NS; ++s) {
+                        const float2 os = dup2(ob[1 + XD + s]), o4 = mul2(os, w4);
+                        float2 q2 = dup2(0.f);  // sum of z_d^2 over the slot's dims
+                        bool first = true;
 #pragma unroll
                         for (int d = 0; d < XD; ++d)
-                            if ((C::slot_dims(s) >> d) & 1) zb[1 + d] = fma2(g2, z[1 + d], zb[1 + d]);
+                            if ((C::slot_dims(s) >> d) & 1) {
+                                q2 = first ? mul2(z[1 + d], z[1 + d]) : fma2(z[1 + d], z[1 + d], q2);
+                                first = false;
+                                zb[1 + d] = fma2(o4, z[1 + d], zb[1 + d]);
+                            }
+                        P = fma2(os, z[1 + XD + s], P);
+                        Q = s == 0 ? mul2(os, q2) : fma2(os, q2, Q);
+                        zb[1 + XD + s] = mul2(os, wtp);
                     }
-                    zb[0] = fma2(tppb, tppp, fma2(tpb, tpp, mul2(gb[0], tp)));
+                    float2 s3 = fma2(tp, P, fma2(dup2(ob[0]), a, g3[q]));
+                    float2 z0 = fma2(tpp, P, mul2(dup2(ob[0]), tp));
+                    if constexpr (NS > 0) {
+                        s3 = fma2(tpp, Q, s3);
+                        z0 = fma2(tppp, Q, z0);
+                    }
+                    zb[0] = mul2(w3, z0);
+                    g3[q] = s3;
+                    gb2[q] = add2(gb2[q], zb[0]);
 #pragma unroll
-                    for (int c = 0; c < J; ++c) *reinterpret_cast<float2*>(zrow + c * H2 + k) = zb[c];
+                    for (int c = 0; c < J; ++c) acc[c][2 * q] = zb[c].x, acc[c][2 * q + 1] = zb[c].y;
                 }
-                warp_reduce_scatter<16>(e3, lane);  // lanes without a pair have ob = 0
-                if (!(lane & 1)) R.gW3[lane >> 1] += e3[0];
-                float b3 = ob[0];
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) b3 += __shfl_xor_sync(0xffffffffu, b3, o);
-                if (lane == 0) R.gb3 += b3;
+                for (int c = 0; c < J; ++c) {
+                    *reinterpret_cast<float4*>(zrow + c * H) = make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
+                    *reinterpret_cast<float4*>(zrow + c * H + 4) =
+                        make_float4(acc[c][4], acc[c][5], acc[c][6], acc[c][7]);
+                    tmem_st_split8(mine + A::zcol(c), H, acc[c]);
+                }
             }
-            __syncwarp();  // z2-bar and a1 rows of the warp's pairs are written
-            // ---- phases B and C (warp-level) ----
-            tc_adj_phase_b<C>(S, R, zb, a1row, act, xn, lane);
-            tc_adj_phase_c<C>(S, R, zb, R.a1, nt, lane);
-            __syncwarp();  // every lane has read the rows before the next tile rewrites them
+            tmem_wait_st();
+            tc_fence_before();
+            __syncthreads();
+            tc_fence_after();
+            FBP_TC_ISSUE(tc_adj_issue2, b2h, b2l, mbar2)
+            __syncwarp();
+            if (h == (ti + 2) % NPT && (ti + 2) * 128 + r < cnt) rec = pair_rec(pr, beg + (ti + 2) * 128 + r);
+            // ---- S_c over the warp's pairs, eight at a time, while GEMM 2 runs ----
+            // (K index t of the MMA is pair p + 2t, t + 4 pair p + 2t + 1: loads
+            // without bank conflicts.  The MMA's sums are truncated, so each group
+            // of eight pairs starts from zero and is added in FP32.)
+            {
+                auto split = [](float2 v, float* hi, float* lo) {
+                    float2 a, b;
+                    split2_tf32_rn(v, a, b);
+                    hi[0] = a.x, hi[1] = a.y, lo[0] = b.x, lo[1] = b.y;
+                };
+                const int np = min(A::PPG, cnt - (ti * 128 + sp));
+                const int p2 = sp + 2 * (lane & 3);
+                const float* zr = &T.zb[p2 * A::ZS + sk];
+                const float* ar = &T.a1[p2 * A::AS + sn + (lane >> 2)];
+#pragma unroll 1
+                for (int p = 0; p < np; p += 8, zr += 8 * A::ZS, ar += 8 * A::AS) {
+                    float bh[NA][A::NQ][2], bl[NA][A::NQ][2];
+#pragma unroll
+                    for (int q = 0; q < A::NQ; ++q) {
+                        const float2 a = make_float2(ar[8 * q], ar[A::AS + 8 * q]);
+                        const float2 tp = fma2(make_float2(-a.x, -a.y), a, dup2(1.0f));
+                        split(a, bh[0][q], bl[0][q]);
+                        split(tp, bh[1][q], bl[1][q]);
+                        if constexpr (NS > 0) split(mul2(a, tp), bh[NA - 1][q], bl[NA - 1][q]);  // tpp / -2
+                    }
+#pragma unroll
+                    for (int c = 0; c < J; ++c) {
+                        const int o = c == 0 ? 0 : (c <= XD ? 1 : NA - 1);
+                        float ah[4], al[4];
+                        split(make_float2(zr[c * H], zr[c * H + 8]), ah, al);
+                        split(make_float2(zr[A::ZS + c * H], zr[A::ZS + c * H + 8]), ah + 2, al + 2);
+#pragma unroll
+                        for (int q = 0; q < A::NQ; ++q) {
+                            float d[4];
+                            mma_tf32<true>(d, al, bh[o][q]);
+                            mma_tf32(d, ah, bl[o][q]);
+                            mma_tf32(d, ah, bh[o][q]);
+#pragma unroll
+                            for (int i = 0; i < 4; i += 2) {
+                                const float2 v = add2(make_float2(sacc[c][q][i], sacc[c][q][i + 1]), make_float2(d[i], d[i + 1]));
+                                sacc[c][q][i] = v.x, sacc[c][q][i + 1] = v.y;
+                            }
+                        }
+                    }
+                }
+            }
+            late |= !mbar_wait_warp(mbar2, phase, wait_ns, lane);
+            failed = __syncthreads_or(late);
+            if (failed) break;
+            phase ^= 1u;
+            tc_fence_after();
+            // ---- layer-1 adjoint: b1-bar and the value part of W1-bar ----
+            {
+                float tb[NA][8];
+#pragma unroll
+                for (int g = 0; g < NA; ++g) tmem_ld8(mine + A::cT + g * H, tb[g]);
+                float xn[XD];
+#pragma unroll
+                for (int d = 0; d < XD; ++d) xn[d] = T.xo[buf][d][r];
+                if constexpr (A::STASH) stash(true);
+                tmem_wait_ld();
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float2 a = *reinterpret_cast<const float2*>(arow + 2 * q);
+                    const float2 tp = fma2(make_float2(-a.x, -a.y), a, dup2(1.0f));
+                    // z1bar = tp (T_0 + a T_1 + (6 a^2 - 2) T_2), T_1 over B times -2
+                    float2 z1 = fma2(a, make_float2(tb[1][2 * q], tb[1][2 * q + 1]),
+                                     make_float2(tb[0][2 * q], tb[0][2 * q + 1]));
+                    if constexpr (NS > 0)
+                        z1 = fma2(fma2(dup2(-6.0f), tp, dup2(4.0f)),
+                                  make_float2(tb[NA - 1][2 * q], tb[NA - 1][2 * q + 1]), z1);
+                    z1 = mul2(z1, tp);
+                    gb1[q] = add2(gb1[q], z1);
+#pragma unroll
+                    for (int d = 0; d < XD; ++d) gw1[d][q] = fma2(z1, dup2(xn[d]), gw1[d][q]);
+                }
+                if constexpr (A::STASH) stash(false);
+            }
         }
         if (failed) break;
-        __syncthreads();
-        // combine the warps' sums (fixed warp order) into the item's gradient partial
+        // ---- the item's gradient partial: sums over lanes, warps and pair groups in a fixed order ----
         float* dst = grad_part + (size_t)it * C::P;
-        constexpr int NW = TC_TILE / 32;
-        for (int i = tid; i < H1 * XD; i += blockDim.x) {
-            float v = 0.f;
+        if constexpr (A::STASH) stash(true);
+        {
+            float v[32];
 #pragma unroll
-            for (int w = 0; w < NW; ++w) v += RW[w].gW1[i];
-            dst[C::oW1 + i] = v;
+            for (int q = 0; q < 4; ++q) {
+                v[2 * q] = g3[q].x, v[2 * q + 1] = g3[q].y;
+                v[8 + 2 * q] = gb2[q].x, v[8 + 2 * q + 1] = gb2[q].y;
+                v[16 + 2 * q] = gb1[q].x, v[16 + 2 * q + 1] = gb1[q].y;
+                v[24 + 2 * q] = gw1[0][q].x, v[24 + 2 * q + 1] = gw1[0][q].y;
+            }
+            warp_reduce_scatter<32>(v, lane);
+            T.red[warp][lane] = v[0];
+            if constexpr (XD > 1) {
+                float u[16];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    u[2 * q] = gw1[1][q].x, u[2 * q + 1] = gw1[1][q].y;
+                    u[8 + 2 * q] = XD > 2 ? gw1[XD - 1][q].x : 0.f, u[8 + 2 * q + 1] = XD > 2 ? gw1[XD - 1][q].y : 0.f;
+                }
+                warp_reduce_scatter<16>(u, lane);
+                if (!(lane & 1)) T.red[warp][32 + (lane >> 1)] = u[0];
+            }
+            if (h == 0) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) g3b += __shfl_xor_sync(0xffffffffu, g3b, o);
+                if (lane == 0) T.red3[warp] = g3b;
+            }
         }
-        for (int i = tid; i < H1; i += blockDim.x) {
-            float v = 0.f;
+        // pair groups' S_c: [group][c][k][n]
 #pragma unroll
-            for (int w = 0; w < NW; ++w) v += RW[w].gb1[i];
-            dst[C::ob1 + i] = v;
-        }
-        for (int i = tid; i < H2 * H1; i += blockDim.x) {
-            float v = 0.f;
+        for (int c = 0; c < J; ++c)
 #pragma unroll
-            for (int w = 0; w < NW; ++w) v += RW[w].gW2[i];
+            for (int q = 0; q < A::NQ; ++q) {
+                float* p = &T.zb[((warp / A::SUB) * J + c) * H * H + sk * H + sn + 8 * q + 2 * (lane & 3)];
+                *reinterpret_cast<float2*>(p) = make_float2(sacc[c][q][0], sacc[c][q][1]);
+                *reinterpret_cast<float2*>(p + 8 * H) = make_float2(sacc[c][q][2], sacc[c][q][3]);
+            }
+        next = pr.item_ctr ? s_item : it + (int)gridDim.x;
+        __syncthreads();
+        float s[PT][J];
+#pragma unroll
+        for (int e = 0; e < PT; ++e) {
+            const int i = tid + e * A::T, n = i % H;
+#pragma unroll
+            for (int c = 0; c < J; ++c) {
+                float v = 0.f;
+#pragma unroll
+                for (int g = 0; g < A::PG; ++g) v += T.zb[(g * J + c) * H * H + i];
+                s[e][c] = c > XD ? -2.0f * v : v;
+            }
+            float v = s[e][0];
+#pragma unroll
+            for (int d = 0; d < XD; ++d) v = fmaf(S.cw[n * XD + d], s[e][1 + d], v);
+#pragma unroll
+            for (int q = 0; q < NS; ++q) v = fmaf(S.c2[n * NS + q], s[e][1 + XD + q], v);
             dst[C::oW2 + i] = v;
         }
-        for (int i = tid; i < H2; i += blockDim.x) {
-            float v = 0.f, v3 = 0.f;
+        __syncthreads();
+        // the tangent part of W1-bar: [d][k] rows of W2[k][n] (S_{1+d} + 2 cw_d sum_s S_s), summed over k
 #pragma unroll
-            for (int w = 0; w < NW; ++w) {
-                v += RW[w].gb2[i];
-                v3 += RW[w].gW3[i];
+        for (int e = 0; e < PT; ++e) {
+            const int i = tid + e * A::T, n = i % H, k = i / H;
+            const float wkn = w2g[i];
+#pragma unroll
+            for (int d = 0; d < XD; ++d) {
+                float v = 0.f;
+#pragma unroll
+                for (int q = 0; q < NS; ++q)
+                    if ((C::slot_dims(q) >> d) & 1) v += s[e][1 + XD + q];
+                v = fmaf(2.0f * S.cw[n * XD + d], v, s[e][1 + d]);
+                T.zb[(d * H + n) * (H + 1) + k] = wkn * v;
             }
-            dst[C::ob2 + i] = v;
-            dst[C::oW3 + i] = v3;
         }
-        if (tid == 0) {
-            float v = 0.f;
+        __syncthreads();
+        for (int o = warp; o < H * XD; o += A::NW) {  // one warp per (n, d)
+            const int n = o / XD, d = o - n * XD;
+            float v = lane < H ? T.zb[(d * H + n) * (H + 1) + lane] : 0.f;
 #pragma unroll
-            for (int w = 0; w < NW; ++w) v += RW[w].gb3;
-            dst[C::ob3] = v;
+            for (int q = 16; q > 0; q >>= 1) v += __shfl_xor_sync(0xffffffffu, v, q);
+            if (lane == 0) {
+                const int q = n & 7, w0 = (n >> 3) * 4, at = d == 0 ? 24 + q : 32 + 8 * (d - 1) + q;
+                float u = 0.f;
+#pragma unroll
+                for (int w = 0; w < 4; ++w) u += T.red[w0 + w][at];
+                dst[C::oW1 + n * XD + d] = fmaf(v, S.inv_sd[d], u);
+            }
         }
+        for (int i = tid; i < 3 * H; i += A::T) {
+            const int g = i / H, n = i - g * H, w0 = (n >> 3) * 4, at = g * 8 + (n & 7);
+            float u = 0.f;
+#pragma unroll
+            for (int w = 0; w < 4; ++w) u += T.red[w0 + w][at];
+            dst[(g == 0 ? C::oW3 : (g == 1 ? C::ob2 : C::ob1)) + n] = u;
+        }
+        if (tid == 0) dst[C::ob3] = (T.red3[0] + T.red3[1]) + (T.red3[2] + T.red3[3]);
     }
-    if (failed) mbar_wait_bounded(mbar, phase, wait_ns);  // let the timed-out MMAs finish
+    if (failed) {
+        if (tid == 0) atomicOr(status, FBP_STATUS_TC_TIMEOUT);
+        // let the timed-out MMAs finish (phase is the same for both barriers or one behind)
+        mbar_wait_bounded(mbar1, phase, wait_ns);
+        mbar_wait_bounded(mbar2, phase, wait_ns);
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TcAdjSmem<C>::COLS)
-                     : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(A::COLS) : "memory");
 }
+#undef FBP_TC_ISSUE
 
 }  // namespace fbp

@@ -1,0 +1,119 @@
+// tcgen05 building blocks shared by the tensor-core jet kernels that keep the
+// pair-dependent operand in tensor memory: 8-column TMEM loads and stores, an
+// MMA with A in TMEM, the TF32 split and the K-major layout of the B operands.
+#pragma once
+
+#include "jet_tc.cuh"
+
+namespace fbp {
+
+// The network's compile-time shape without W2 in SParams: the kernels below
+// keep it only as B operands.
+template <class B>
+struct TcCfg : B {
+    static constexpr bool W2S = false;
+};
+
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr),
+                 "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
+                 "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
+                 "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
+                 : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// Waits (bounded) for the phase with one polling lane per warp; false on a time-out.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t mbar, uint32_t parity, uint64_t limit_ns, int lane) {
+    int ok = 1;
+    if (lane == 0) ok = mbar_wait_bounded(mbar, parity, limit_ns);
+    return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// D (TMEM) (+)= A (TMEM, one 32-bit column per K element, row = lane) B^T (shared memory)
+__device__ __forceinline__ void umma_tf32_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                             uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// v = hi + lo with hi = v rounded to TF32's 10 mantissa bits (ties away), so
+// |lo| <= 2^-12 |v|; the MMA reads the top 10 bits of lo, an error of at most
+// 2^-22 |v|, of either sign.  (Truncating v instead doubles lo and the error.)
+__device__ __forceinline__ void split_tf32_rn(float v, float& hi, float& lo) {
+    hi = __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xFFFFE000u);
+    lo = v - hi;
+}
+
+__device__ __forceinline__ void split2_tf32_rn(float2 v, float2& hi, float2& lo) {
+    hi = make_float2(__uint_as_float((__float_as_uint(v.x) + 0x1000u) & 0xFFFFE000u),
+                     __uint_as_float((__float_as_uint(v.y) + 0x1000u) & 0xFFFFE000u));
+    lo = fma2(hi, dup2(-1.0f), v);
+}
+
+// Splits 8 values and stores them as columns [col, col+8) (hi) and
+// [col + lo_off, ...) (lo) of this thread's TMEM lane.
+__device__ __forceinline__ void tmem_st_split8(uint32_t col, uint32_t lo_off, const float (&v)[8]) {
+    float hi[8], lo[8];
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+        float2 a, b;
+        split2_tf32_rn(make_float2(v[i], v[i + 1]), a, b);
+        hi[i] = a.x, hi[i + 1] = a.y;
+        lo[i] = b.x, lo[i + 1] = b.y;
+    }
+    tmem_st8(col, hi);
+    tmem_st8(col + lo_off, lo);
+}
+
+// One warp's 16 x 8 x 8 product with TF32 operands and FP32 sums: D = A B
+// (ZERO) or D += A B.  Lane (g, t) = (lane / 4, lane % 4) holds A (g, t),
+// (g + 8, t), (g, t + 4), (g + 8, t + 4), B (t, g), (t + 4, g) and D (g, 2t),
+// (g, 2t + 1), (g + 8, 2t), (g + 8, 2t + 1).
+template <bool ZERO = false>
+__device__ __forceinline__ void mma_tf32(float (&d)[4], const float (&a)[4], const float (&b)[2]) {
+    if constexpr (ZERO)
+        asm volatile(
+            "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+            : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+            : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])),
+              "r"(__float_as_uint(a[3])), "r"(__float_as_uint(b[0])), "r"(__float_as_uint(b[1])), "f"(0.f));
+    else
+        asm volatile(
+            "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+            : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])),
+              "r"(__float_as_uint(a[3])), "r"(__float_as_uint(b[0])), "r"(__float_as_uint(b[1])));
+}
+
+// B operand with H K-elements per row in the no-swizzle K-major layout: core
+// matrices of 8 rows x 4 floats, 128 bytes apart along K, 32 H bytes along the rows.
+template <int H>
+struct KMajor {
+    static constexpr uint32_t LBO = 128, SBO = 32 * H;
+    // float offset of (row, k), and the (row, k) of offset o: a loop over
+    // offsets fills the operand without bank conflicts
+    __device__ __forceinline__ static int off(int row, int k) {
+        return (row >> 3) * 8 * H + (k >> 2) * 32 + (row & 7) * 4 + (k & 3);
+    }
+    __device__ __forceinline__ static void at(int o, int& row, int& k) {
+        row = (o / (8 * H)) * 8 + ((o >> 2) & 7);
+        k = ((o % (8 * H)) >> 5) * 4 + (o & 3);
+    }
+};
+
+}  // namespace fbp

@@ -276,8 +276,9 @@ def t_status(ps):
 
 
 def tc_supported(xd, h1, h2, d2mask=3 | _lib.D2_LAPLACIAN, act=_lib.ACT_TANH):
-    """True where the tensor-core forward kernel is compiled (xd = 2, two
-    16-wide hidden layers; the jet masks and activations of fbp_has_tc_shape)."""
+    """True where a tensor-core forward kernel is compiled (xd = 2 and two
+    16-wide hidden layers, or tanh and two 32-wide ones; the jet masks and
+    activations of fbp_has_tc_shape)."""
     return bool(_lib.load().fbp_has_tc_shape(xd, h1, h2, d2mask, act))
 
 
@@ -348,25 +349,27 @@ class FBPINNEngine:
         tc_ok = tc_supported(self.xd, self.h1, self.h2, self.d2mask, self.act)
         if tensor_cores and not tc_ok:
             raise _lib.FBPLibraryError(f"no tensor-core forward kernel for layer sizes {ls} ({activation}, "
-                                       f"d2mask {self.d2mask}); compiled: 2-16-16-1 networks")
+                                       f"d2mask {self.d2mask}); compiled: 2-16-16-1 networks and xd-32-32-1 tanh networks")
         self.tensor_cores = (tc_ok and self.act == _lib.ACT_TANH) if tensor_cores is None else bool(tensor_cores)
-        # adjoint with the layer-2 recompute on the tensor cores (fbp_adjoint_pairs_tc):
-        # None = off unless requested; True = required; False = off
+        # adjoint with its layer-2 recompute and W2^T products on the tensor cores
+        # (fbp_adjoint_pairs_tc): None = where it is compiled and the caller does not
+        # ask for stored z-jets; True = required; False = the FMA kernel
         tca_ok = bool(_lib.load().fbp_has_tc_adjoint_shape(self.xd, self.h1, self.h2, self.d2mask, self.act))
         if tc_adjoint and not tca_ok:
             raise _lib.FBPLibraryError(f"no tensor-core adjoint kernel for layer sizes {ls} ({activation}, "
-                                       f"d2mask {self.d2mask}); compiled: xd-16-16-1 tanh networks")
-        self.tc_adjoint = bool(tc_adjoint) and tca_ok
+                                       f"d2mask {self.d2mask}); compiled: xd-16-16-1 and xd-32-32-1 tanh networks")
+        self.tc_adjoint = tca_ok and (not store_z2 if tc_adjoint is None else bool(tc_adjoint))
         # store_z2: the forward of a training step stores the layer-2 z-jets of
         # every pair (J * h2 floats) and the FMA adjoint reads them instead of
         # recomputing layer 2 (h1 multiply-adds per stored value); a point set
         # keeps the buffer while it takes at most z2_limit bytes (an eighth of
-        # the device memory), else the adjoint recomputes.  None: where the first
-        # hidden layer is at least 32 wide (measured: 3-32-32-1 gains, 2-16-16-1
-        # loses -- its stores cost the forward more than the reads save in the
-        # latency-bound adjoint)
+        # the device memory), else the adjoint recomputes.  None: where the FMA
+        # adjoint runs and the first hidden layer is at least 32 wide (measured:
+        # the recompute is h1 multiply-adds per stored value, and at 16 the stores
+        # cost the forward more than the reads save; the tensor-core adjoint
+        # recomputes at no such cost)
         if store_z2 is None:
-            store_z2 = self.h1 >= 32
+            store_z2 = self.h1 >= 32 and not self.tc_adjoint
         self.z2_rows = self.J * self.h2 if (store_z2 and self.h2 > 0 and not self.tc_adjoint) else 0
         self.z2_limit = torch.cuda.get_device_properties(self.device).total_memory // 8
         # sample(): uniform batches in the order of a Morton cell grid (locality of
