@@ -1,19 +1,20 @@
-// C ABI of the tensor-core forward jet kernel (tcgen05, 3xTF32) for networks
-// with two 16-wide hidden layers: the plain tanh FCN here, the other
-// activations in jet_tc_act.cu.
-#include "jet_tc_launch.cuh"
+// C ABI of the tensor-core forward jet kernels (tcgen05, 3xTF32): tanh networks
+// with two 16- or 32-wide hidden layers (jet_tc_fwd.cu) and 16-wide ones with
+// the other activations (jet_tc_act.cu).
+#include "common.cuh"
 
 namespace fbp {
 int tc_group_act(int mode, const fbp_net* net, const float* x, const fbp_pairs* pr, float* pair_out,
                  int32_t* status, int grid, cudaStream_t st);
 
+int tc_group_tanh(int mode, const fbp_net* net, const float* x, const fbp_pairs* pr, float* pair_out, int32_t* status,
+                int grid, cudaStream_t st);
+
 static int tc_dispatch(int mode, const fbp_net* net, const float* x, const fbp_pairs* pr, float* pair_out,
                        int32_t* status, int grid, cudaStream_t st) {
-    if (net->ud != 1 || net->h1 != 16 || net->h2 != 16) return 1;
-    FBP_TC_TRY(2, 3 | FBP_D2_LAPLACIAN, FBP_ACT_TANH)
-    FBP_TC_TRY(2, 3, FBP_ACT_TANH)
-    FBP_TC_TRY(2, 1, FBP_ACT_TANH)
-    FBP_TC_TRY(2, 0, FBP_ACT_TANH)
+    if (net->ud != 1 || net->h1 != net->h2) return 1;
+    if (net->act == FBP_ACT_TANH) return tc_group_tanh(mode, net, x, pr, pair_out, status, grid, st);
+    if (net->h1 != 16) return 1;
     return tc_group_act(mode, net, x, pr, pair_out, status, grid, st);
 }
 }  // namespace fbp
@@ -25,9 +26,9 @@ extern "C" int fbp_forward_pairs_tc(const fbp_net* net, const float* x, const fb
                 "fbp_forward_pairs_tc: null network pointer");
     FBP_REQUIRE(pairs->sd_rec && pairs->items && pairs->n_items, FBP_ERR_INVALID,
                 "fbp_forward_pairs_tc: null pair pointer");
-    FBP_REQUIRE(net->ud == 1 && net->h1 == 16 && net->h2 == 16, FBP_ERR_UNSUPPORTED,
-                "fbp_forward_pairs_tc: only the xd-16-16-1 networks are compiled (got h1=%d h2=%d ud=%d)", net->h1,
-                net->h2, net->ud);
+    FBP_REQUIRE(net->ud == 1 && net->h1 == net->h2 && (net->h1 == 16 || net->h1 == 32), FBP_ERR_UNSUPPORTED,
+                "fbp_forward_pairs_tc: only the xd-16-16-1 and xd-32-32-1 networks are compiled (got h1=%d h2=%d ud=%d)",
+                net->h1, net->h2, net->ud);
     const int r = fbp::tc_dispatch(1, net, x, pairs, pair_out, status, grid, fbp::as_stream(stream));
     if (r != 1) return r;
     fbp::set_error("fbp_forward_pairs_tc: no compiled kernel for xd=%d d2mask=%d act=%d", net->xd, net->d2mask,

@@ -1,5 +1,6 @@
 // Tensor-core (tcgen05, 3xTF32) variant of the per-pair forward jet kernel for
-// networks with two 16-wide hidden layers.
+// networks with two 16-wide hidden layers and activations other than the plain
+// tanh (whose kernel is in jet_tc_fwd.cuh).
 //
 // Layer 2 of the jet, z_c[k] = sum_n W2[k][n] v_c[n] (+ b2[k] for c = 0), is
 // J small GEMMs per tile of 128 pairs (M = 128 pairs, N = 16, K = 16).  The
@@ -149,7 +150,7 @@ __host__ __device__ constexpr int tc_a_of(int c) {
 // tp = 1 - a^2, tpp = -2 a tp.
 template <class C>
 __device__ __forceinline__ void tanh_jet_pair(const float2 (&z)[C::J], float2 (&g)[C::J]) {
-    const float2 a = make_float2(tanh_fast(z[0].x), tanh_fast(z[0].y));
+    const float2 a = tanh_fast2(z[0]);
     const float2 tp = fma2(make_float2(-a.x, -a.y), a, dup2(1.0f));
     const float2 tpp = mul2(mul2(dup2(-2.0f), a), tp);
     g[0] = a;
@@ -197,7 +198,7 @@ __device__ __forceinline__ void tc_epilogue(const SParams<C>& S, uint32_t taddr,
                 __stcs(zs + (size_t)(c * H2 + k + 1) * zs_cap, z[c].y);
             }
         }
-        if constexpr (C::ACT == FBP_ACT_TANH || C::ACT == FBP_ACT_FOURIER) {
+        if constexpr (C::ACT == FBP_ACT_FOURIER) {
             tanh_jet_pair<C>(z, g);  // layer 2 is a plain tanh
         } else {
             float zs[2][J], gs[2][J];
@@ -332,23 +333,15 @@ __global__ void __launch_bounds__(TC_TILE) forward_pairs_tc_kernel(fbp_net net, 
 #pragma unroll
                         for (int d = 0; d < XD; ++d)
                             z = fma2(make_float2(S.W1[n * XD + d], S.W1[(n + 1) * XD + d]), dup2(xn[d]), z);
-                        if constexpr (C::ACT == FBP_ACT_TANH) {
-                            const float2 a = make_float2(tanh_fast(z.x), tanh_fast(z.y));
-                            const float2 tp = fma2(make_float2(-a.x, -a.y), a, dup2(1.0f));
-                            av[0][q] = a;
-                            av[1][q] = tp;
-                            if constexpr (NA > 2) av[NA - 1][q] = mul2(mul2(dup2(-2.0f), a), tp);
-                        } else {
-                            // sigma, sigma', sigma'' of the layer-1 activation c f(o z)
-                            float a0, t0, tt0, ttt0, a1, t1, tt1, ttt1;
-                            const float c0 = act_c<C, false>(S, n), o0 = act_o<C, false>(S, n);
-                            const float c1 = act_c<C, false>(S, n + 1), o1 = act_o<C, false>(S, n + 1);
-                            C::AF1::derivs(C::AF1::stored(z.x, o0), c0, o0, a0, t0, tt0, ttt0);
-                            C::AF1::derivs(C::AF1::stored(z.y, o1), c1, o1, a1, t1, tt1, ttt1);
-                            av[0][q] = make_float2(a0, a1);
-                            av[1][q] = make_float2(t0, t1);
-                            if constexpr (NA > 2) av[NA - 1][q] = make_float2(tt0, tt1);
-                        }
+                        // sigma, sigma', sigma'' of the layer-1 activation c f(o z)
+                        float a0, t0, tt0, ttt0, a1, t1, tt1, ttt1;
+                        const float c0 = act_c<C, false>(S, n), o0 = act_o<C, false>(S, n);
+                        const float c1 = act_c<C, false>(S, n + 1), o1 = act_o<C, false>(S, n + 1);
+                        C::AF1::derivs(C::AF1::stored(z.x, o0), c0, o0, a0, t0, tt0, ttt0);
+                        C::AF1::derivs(C::AF1::stored(z.y, o1), c1, o1, a1, t1, tt1, ttt1);
+                        av[0][q] = make_float2(a0, a1);
+                        av[1][q] = make_float2(t0, t1);
+                        if constexpr (NA > 2) av[NA - 1][q] = make_float2(tt0, tt1);
                     }
                     const uint32_t off = kmajor16_off(tid, n4) >> 2;
 #pragma unroll

@@ -234,3 +234,47 @@ def test_tensor_core_adjoint_timeout_path_reports_and_recovers(cuda):
     a, b = ref[:n_items], ps.grad_part[:n_items]
     assert torch.isfinite(b).all()
     assert (a - b).abs().max().item() <= TC_TOL * a.abs().max().item()
+
+
+@pytest.mark.parametrize("xd,h,d2", [(2, 16, 3 | 8), (2, 16, 0), (1, 32, 1), (2, 32, 3 | 8), (2, 32, 3),
+                                     (3, 32, 7 | _lib.D2_GROUP(3)), (3, 32, 7)])
+@pytest.mark.parametrize("n", [1, 127, 129, 2000])
+def test_tensor_memory_kernels_match_fma(cuda, xd, h, d2, n):
+    """The kernels with their operands in tensor memory against the FMA
+    kernels at the edges of their 128-pair tiles: two boxes that hold every
+    point (items of one pair, of one pair less and more than a tile, and of
+    many tiles with a rest) and one that holds some.  Records to TC_TOL of
+    each component's largest over 2000 points, gradients (of the same seeds)
+    to TC_TOL of each network's largest."""
+    from helpers import boxes_static
+    xmin = np.array([[0.0] * xd, [-0.5] * xd, [0.3] * xd], dtype=np.float32)
+    xmax = np.array([[1.0] * xd, [1.2] * xd, [0.9] * xd], dtype=np.float32)
+    static = boxes_static(xmin, xmax)
+    layers = random_layers([xd, h, h, 1], 3, seed=h)
+    x = torch.rand((2000, xd), generator=torch.Generator().manual_seed(h))
+    seeds = torch.randn((4096, 16), generator=torch.Generator().manual_seed(1)).cuda()
+
+    def both(tc, x):
+        eng = FBPINNEngine(static, [xd, h, h, 1], d2, chunk=1024, tensor_cores=tc, tc_adjoint=False, store_z2=False)
+        if tc:
+            eng.tc_adjoint = bool(_lib.load().fbp_has_tc_adjoint_shape(xd, h, h, d2, _lib.ACT_TANH))
+            assert eng.tc_adjoint == (eng.J <= 6)
+        eng.set_theta(pack_layers([(w.float(), b.float()) for w, b in layers]))
+        ps = eng.points(x)
+        ps.pair_out.fill_(float("nan"))
+        eng.forward_pairs(ps)
+        rec = ps.pair_out[:ps.s].clone()
+        ps.slot_out.copy_(seeds[:ps.slot_out.shape[0], :ps.slot_out.shape[1]])
+        ps.grad_part.fill_(float("nan"))
+        grad = eng.adjoint(ps).clone()
+        torch.cuda.synchronize()
+        ps.check_status()
+        return rec, grad, eng.J
+
+    scale = both(False, x)[0].abs().max(0).values
+    (r0, g0, J), (r1, g1, _) = both(False, x[:n]), both(True, x[:n])
+    assert torch.isfinite(r1[:, :2 * J]).all() and torch.isfinite(g1).all()
+    err = ((r1 - r0).abs().max(0).values / scale.clamp(min=1e-30))[:2 * J]
+    assert err.max().item() <= TC_TOL, err.tolist()
+    err = (g1 - g0).abs().max(1).values / g0.abs().max(1).values.clamp(min=1e-30)
+    assert err.max().item() <= TC_TOL, err.tolist()
