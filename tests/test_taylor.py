@@ -1,0 +1,85 @@
+"""The Taylor rules of constrained_jets against its nested-jvp route (float64,
+CPU): the jets and their gradient, for the built-in constraints and for
+functions that use every rule, other shapes, or a call without a rule."""
+
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from fbpinns_gb300 import engine, problems as PR, taylor
+
+
+def _static(p):
+    return {"static": {"problem": {k: v.double() if torch.is_tensor(v) else v for k, v in p.items()}}}
+
+
+WAVE = np.array([[0.1, -0.2, 0.3, 1.0], [0.4, 0.3, 0.2, -0.7]])
+W = torch.linspace(-1, 1, 6, dtype=torch.float64).reshape(2, 3)
+
+
+def _rules(p, x, u):
+    """Every rule, with scalars, constants and jets on either side."""
+    a, b = x[:, 0:1], x[..., 1:2]
+    c = torch.tanh(2 * a + 1) - torch.exp(-b) / 3 + 1 / (2 + a * a)
+    c = c + torch.sin(b) * torch.cos(a) - torch.neg(b) ** 3 + (3 - a) / (b + 4)
+    c = torch.sub(c, 0.5) + torch.square(a).mul(0.1) + 2.0 - torch.reciprocal(a + 5) * torch.full_like(p, 1.5)
+    return c * u + (u * u - torch.add(a, b)) ** 1
+
+
+def _broadcast(p, x, u):
+    """(k, n, 2) intermediates, sums over one and two dims, None and int indices."""
+    d = x[None] - W[:, None, :x.shape[1]]
+    s = torch.exp(-(d ** 2).sum(2, keepdim=True)).sum(0)
+    t = (d * x).sum((0, -1))[:, None]
+    return s * u + t + x[:, 0].mul(2)[:, None]
+
+
+CASES = {
+    "ho": (1, 1, PR.HarmonicOscillator1DHardBC.constraining_fn, _static({"sd": 0.1})),
+    "burgers": (2, 1, PR.BurgersEquation2D.constraining_fn, _static({"sd": 0.1})),
+    "poisson": (2, 3, PR.Poisson2D.constraining_fn, _static({"sd": 0.1})),
+    "wave": (3, 7, PR.WaveEquationGaussianVelocity3D.constraining_fn,
+             _static({"c0": 1.0, "source": torch.as_tensor(WAVE)})),
+    "rules": (2, 3, _rules, torch.zeros((17, 1), dtype=torch.float64)),
+    "rules_1d_second": (2, 2, _rules, torch.zeros((17, 1), dtype=torch.float64)),
+    "broadcast": (3, 5, _broadcast, None),
+    "all_points": (2, 3, lambda p, x, u: u * x[:, 0:1] + (u * u).sum(0, keepdim=True), None),
+    "no_u": (2, 3, lambda p, x, u: torch.sin(x[:, 1:2]), None),
+    "constant": (2, 3, lambda p, x, u: torch.ones_like(u), None),
+    "scaled": (2, 3, lambda p, x, u: u * 2, None),
+    "no_rule": (2, 3, lambda p, x, u: torch.atan(x[:, 0:1]) * u + torch.where(x[:, 1:2] > 0.5, u, 2 * u), None),
+    "power": (2, 3, lambda p, x, u: (x[:, 0:1] + 2) ** 0.5 * u, None),
+    "in_place": (2, 3, lambda p, x, u: (x[:, 0:1] * u).add_(u), None),
+}
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_taylor_rules_match_nested_jvp(name, monkeypatch):
+    xd, d2, fn, p = CASES[name]
+    J = engine.jet_size(xd, d2)
+    g = torch.Generator().manual_seed(3)
+    x = torch.rand((17, xd), generator=g, dtype=torch.float64)
+    U = torch.randn((17, J), generator=g, dtype=torch.float64, requires_grad=True)
+    seed = torch.randn((17, J), generator=g, dtype=torch.float64)
+    for need in (None, [1], [J - 1]):
+        got = engine.constrained_jets(fn, p, x, U, xd, d2, need)
+        with monkeypatch.context() as m:
+            m.setattr(taylor, "RULES", {})
+            m.setattr(taylor, "PLAIN", set())
+            ref = engine.constrained_jets(fn, p, x, U, xd, d2, need)
+        torch.testing.assert_close(got, ref, rtol=1e-11, atol=1e-11 * ref.abs().max().item())
+        assert got.requires_grad == ref.requires_grad
+        if ref.requires_grad:
+            dg, dr = (torch.autograd.grad((v * seed).sum(), U)[0] for v in (got, ref))
+            torch.testing.assert_close(dg, dr, rtol=1e-11, atol=1e-11 * dr.abs().max().item())
+
+
+def test_every_builtin_constraint_has_rules():
+    for name in ("ho", "burgers", "poisson", "wave"):
+        xd, d2, fn, p = CASES[name]
+        x = torch.rand((5, xd), dtype=torch.float64)
+        z = torch.zeros((xd, 5, 1), dtype=torch.float64)
+        _, d, dd = taylor.jets(lambda a, b: fn(p, a, b), x, list(range(xd)), x[:, 0:1] * 1, z + 1, z)
+        assert d.shape == dd.shape == (xd, 5, 1) and torch.isfinite(d).all() and math.isfinite(dd.sum().item())
