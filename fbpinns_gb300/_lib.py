@@ -83,6 +83,9 @@ _SIG = {
     "fbp_scan_i32_noalloc": (C.c_int, [_P, _P, _I64, _P]),
     "fbp_inside_count": (C.c_int, [_P, _I64, C.POINTER(Boxes), _P, _P, _P, _P, _P, _P, _P]),
     "fbp_inside_fill": (C.c_int, [_P, _I64, C.POINTER(Boxes), _P, _P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _P, _P]),
+    "fbp_inside_lists_scratch_bytes": (C.c_size_t, [_I64]),
+    "fbp_inside_lists": (C.c_int, [_P, _I64, C.POINTER(Boxes), _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _P, _P,
+                                   C.c_size_t, _P]),
     "fbp_gather_i32": (C.c_int, [_P, _I64, _P, _P, _P, _P]),
     "fbp_compact_scratch_bytes": (C.c_size_t, [_I64]),
     "fbp_compact_flags": (C.c_int, [_P, _I64, _P, _P, _P, C.c_size_t, _P]),
@@ -103,6 +106,8 @@ _SIG = {
     "fbp_adjoint_pairs_tc": (C.c_int, [C.POINTER(Net), _P, C.POINTER(Pairs), _P, _P, _P, _I32, _P]),
     "fbp_has_tc_adjoint_shape": (C.c_int, [_I32, _I32, _I32, _I32, _I32]),
     "fbp_grad_reduce": (C.c_int, [_P, _P, _I64, _I32, _P, _P]),
+    "fbp_step_tail": (C.c_int, [_P, _I32, C.c_double, _P, _P, _P, _P, _P, _P, _P, _P, _I64, _I32, C.c_float, C.c_float,
+                                C.c_float, C.c_float, C.c_float, _P, _P, _P]),
     "fbp_adam": (C.c_int, [_P, _P, _P, _P, _P, _I64, _I32, C.c_float, C.c_float, C.c_float, C.c_float, C.c_float,
                            _P, _P]),
     "fbp_sample_uniform": (C.c_int, [_P, _I64, _I32, C.POINTER(C.c_double), C.POINTER(C.c_double), C.c_uint64,

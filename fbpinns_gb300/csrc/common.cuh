@@ -124,6 +124,19 @@ __device__ __forceinline__ float tanh_fast(float x) {
     return copysignf((1.0f - e) * rcp_ftz(1.0f + e), x);
 }
 
+// One parameter's Adam step (optax.adam: moments, bias corrections bc1 = 1 - b1^t,
+// bc2 = 1 - b2^t, scale(-lr)).
+__device__ __forceinline__ void adam_element(float& theta, float& m1, float& m2, float g, float lr, float b1, float b2,
+                                             float eps, float eps_root, float bc1, float bc2) {
+    const float mu = (1.0f - b1) * g + b1 * m1;
+    const float nu = (1.0f - b2) * g * g + b2 * m2;
+    m1 = mu;
+    m2 = nu;
+    const float mh = mu / bc1;
+    const float nh = nu / bc2;
+    theta = theta + (-lr) * (mh / (sqrtf(nh + eps_root) + eps));
+}
+
 inline int jet_size_rt(int xd, int d2) { return 1 + xd + d2_slots(d2); }
 
 }  // namespace fbp

@@ -54,14 +54,7 @@ __global__ void adam_kernel(float* __restrict__ theta, float* __restrict__ m1, f
          i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t row = i / P;
         if (state[row] != 1) continue;
-        const float g = grad[i];
-        const float mu = (1.0f - b1) * g + b1 * m1[i];
-        const float nu = (1.0f - b2) * g * g + b2 * m2[i];
-        m1[i] = mu;
-        m2[i] = nu;
-        const float mh = mu / bc1;
-        const float nh = nu / bc2;
-        theta[i] = theta[i] + (-lr) * (mh / (sqrtf(nh + eps_root) + eps));
+        adam_element(theta[i], m1[i], m2[i], grad[i], lr, b1, b2, eps, eps_root, bc1, bc2);
     }
 }
 

@@ -50,24 +50,34 @@ __device__ __forceinline__ bool inside_box(const float* xp, const float* __restr
 constexpr int64_t COUNT_MAX_M = 12288;
 constexpr int COUNT_CTAS = 2, COUNT_T = 512;
 
+// Points per chunk of the list build: the count pass leaves the pairs and
+// slots of each chunk (the CTA's points), and the fill pass, which works on the
+// same chunks, adds those of the chunks before its own and scans within the
+// chunk -- two launches for the lists, where separate scans take four more
+// (with the work queues in one launch each and the sort's starts in its scatter,
+// 16381 points in 85 boxes redrawn every step: 161 -> 150.5 us a step).
+constexpr int LIST_CHUNK = 256;
+
 // SHIST: model_count through the CTA's table in shared memory (m words).
+// sums (nullable; !SHIST, CTAs of LIST_CHUNK threads): per chunk its pairs and slots.
 template <int XD, bool SHIST>
 __global__ void inside_count_kernel(const float* __restrict__ x, int64_t n, fbp_boxes b,
                                     int32_t* __restrict__ pt_count, int32_t* __restrict__ pt_nlvl,
                                     uint64_t* __restrict__ pt_lvl, int32_t* __restrict__ model_count,
-                                    uint64_t* __restrict__ pt_hit, int32_t* __restrict__ pt_cand) {
+                                    uint64_t* __restrict__ pt_hit, int32_t* __restrict__ pt_cand,
+                                    int2* __restrict__ sums) {
     extern __shared__ int32_t box_count[];
     if constexpr (SHIST) {
         for (int64_t j = threadIdx.x; j < b.m; j += blockDim.x) box_count[j] = 0;
         __syncthreads();
     }
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
-         p += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t p0 = blockIdx.x * (int64_t)blockDim.x; p0 < n; p0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t p = p0 + threadIdx.x;
         float xp[XD];
 #pragma unroll
-        for (int d = 0; d < XD; ++d) xp[d] = x[p * XD + d];
+        for (int d = 0; d < XD; ++d) xp[d] = p < n ? x[p * XD + d] : 0.f;
         const int c = cell_of<XD>(xp, b);
-        const int e0 = b.cell_start[c], e1 = b.cell_start[c + 1];
+        const int e0 = b.cell_start[c], e1 = p < n ? b.cell_start[c + 1] : e0;
         int cnt = 0;
         uint64_t lvl = 0, hit = 0;
         for (int e = e0; e < e1; ++e) {
@@ -83,12 +93,29 @@ __global__ void inside_count_kernel(const float* __restrict__ x, int64_t n, fbp_
                     atomicAdd(&model_count[j], 1);
             }
         }
-        pt_count[p] = cnt;
-        if (pt_nlvl) pt_nlvl[p] = __popcll(lvl);
-        if (pt_lvl) pt_lvl[p] = lvl;
-        // hits as a mask over the cell's candidate list (cells of <= 64 candidates)
-        if (pt_hit) pt_hit[p] = hit;
-        if (pt_cand) pt_cand[p] = e1 - e0 <= 64 ? e0 : -1;
+        if (p < n) {
+            pt_count[p] = cnt;
+            if (pt_nlvl) pt_nlvl[p] = __popcll(lvl);
+            if (pt_lvl) pt_lvl[p] = lvl;
+            // hits as a mask over the cell's candidate list (cells of <= 64 candidates)
+            if (pt_hit) pt_hit[p] = hit;
+            if (pt_cand) pt_cand[p] = e1 - e0 <= 64 ? e0 : -1;
+        }
+        if constexpr (!SHIST) {
+            if (sums) {
+                __shared__ int2 warp_sums[LIST_CHUNK / 32];
+                const int ws = __reduce_add_sync(0xffffffffu, cnt), wu = __reduce_add_sync(0xffffffffu, __popcll(lvl));
+                if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = make_int2(ws, wu);
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    int2 t = make_int2(0, 0);
+#pragma unroll
+                    for (int w = 0; w < LIST_CHUNK / 32; ++w) t = make_int2(t.x + warp_sums[w].x, t.y + warp_sums[w].y);
+                    sums[p0 / LIST_CHUNK] = t;
+                }
+                __syncthreads();
+            }
+        }
     }
     if constexpr (SHIST) {
         __syncthreads();
@@ -110,33 +137,78 @@ constexpr int FILL_WARPS = 8;     // warps per CTA
 constexpr int FILL_STAGE = 1280;  // staged pairs per warp
 constexpr int64_t FILL_MAX_M = int64_t(1) << 21;
 
-template <int XD>
+// OFFS: pt_off and np_off are made here, from pt_count, the levels and the
+// count pass's chunk sums; else they are read.
+template <int XD, bool OFFS>
 __global__ void __launch_bounds__(FILL_WARPS * 32)
-    inside_fill_kernel(const float* __restrict__ x, int64_t n, fbp_boxes b, const int32_t* __restrict__ pt_off,
-                       const int32_t* __restrict__ np_off, const uint64_t* __restrict__ pt_lvl,
+    inside_fill_kernel(const float* __restrict__ x, int64_t n, fbp_boxes b, int32_t* __restrict__ pt_off,
+                       int32_t* __restrict__ np_off, const int32_t* __restrict__ pt_count,
+                       const int2* __restrict__ sums, const uint64_t* __restrict__ pt_lvl,
                        const uint64_t* __restrict__ pt_hit, const int32_t* __restrict__ pt_cand,
                        int32_t* __restrict__ n_take, int32_t* __restrict__ m_take, int32_t* __restrict__ p_take,
                        int32_t* __restrict__ np_take, int64_t s_cap, int64_t u_cap, int32_t* __restrict__ status) {
     __shared__ int32_t stage[FILL_WARPS][FILL_STAGE];
     __shared__ uint64_t s_lvl[FILL_WARPS][32];
     __shared__ int32_t s_ubase[FILL_WARPS][32];
+    __shared__ int2 s_part[FILL_WARPS], s_pre[FILL_WARPS];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t nwarps = (int64_t)gridDim.x * FILL_WARPS;
-    for (int64_t p0 = ((int64_t)blockIdx.x * FILL_WARPS + w) * 32; p0 < n; p0 += nwarps * 32) {
+    static_assert(FILL_WARPS * 32 == LIST_CHUNK, "a CTA fills a chunk at a time");
+    int64_t done = 0;               // chunks whose sums are in pre
+    int2 pre = make_int2(0, 0);     // this thread's part of the sums of the chunks before
+    const int64_t nchunk = (n + LIST_CHUNK - 1) / LIST_CHUNK;
+    for (int64_t chunk = blockIdx.x; chunk < nchunk; chunk += gridDim.x) {
+        const int64_t p0 = chunk * LIST_CHUNK + w * 32;
         const int64_t p = p0 + lane;
         const bool valid = p < n;
-        const int np = (int)min((int64_t)32, n - p0);
-        const int64_t wb = pt_off[p0], we = pt_off[p0 + np];
-        const int64_t total = we - wb;
-        const bool staged = total <= FILL_STAGE && b.m <= FILL_MAX_M;
-        int64_t base = 0;
+        const int np = (int)max((int64_t)0, min((int64_t)32, n - p0));
+        int64_t base = 0, wb = 0, we = 0;
         int32_t ubase = 0;
         uint64_t lvl = 0;
-        if (valid) {
-            base = pt_off[p];
-            ubase = np_off[p];
-            lvl = pt_lvl[p];
+        if (valid) lvl = pt_lvl[p];
+        if constexpr (OFFS) {
+            for (int64_t c = done + threadIdx.x; c < chunk; c += LIST_CHUNK) {
+                const int2 t = sums[c];
+                pre.x += t.x;
+                pre.y += t.y;
+            }
+            done = chunk;
+            const int cnt = valid ? pt_count[p] : 0, nl = __popcll(lvl);
+            int a = cnt, u = nl;  // inclusive scans over the warp
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int ta = __shfl_up_sync(0xffffffffu, a, o), tu = __shfl_up_sync(0xffffffffu, u, o);
+                if (lane >= o) a += ta, u += tu;
+            }
+            const int wa = __shfl_sync(0xffffffffu, a, 31), wu = __shfl_sync(0xffffffffu, u, 31);
+            const int pa = __reduce_add_sync(0xffffffffu, pre.x), pu = __reduce_add_sync(0xffffffffu, pre.y);
+            __syncthreads();  // the previous chunk's s_part and s_pre have been read
+            if (lane == 0) s_part[w] = make_int2(wa, wu), s_pre[w] = make_int2(pa, pu);
+            __syncthreads();
+            int2 o = make_int2(0, 0);
+#pragma unroll
+            for (int v = 0; v < FILL_WARPS; ++v) {
+                o.x += s_pre[v].x + (v < w ? s_part[v].x : 0);
+                o.y += s_pre[v].y + (v < w ? s_part[v].y : 0);
+            }
+            base = o.x + a - cnt;
+            ubase = o.y + u - nl;
+            wb = o.x;
+            we = o.x + wa;
+            if (valid) {
+                pt_off[p] = (int32_t)base;
+                np_off[p] = ubase;
+                if (p == n - 1) pt_off[n] = (int32_t)base + cnt, np_off[n] = ubase + nl;
+            }
+        } else if (np > 0) {
+            wb = pt_off[p0];
+            we = pt_off[p0 + np];
+            if (valid) {
+                base = pt_off[p];
+                ubase = np_off[p];
+            }
         }
+        const int64_t total = we - wb;
+        const bool staged = total <= FILL_STAGE && b.m <= FILL_MAX_M;
         s_lvl[w][lane] = lvl;
         s_ubase[w][lane] = ubase;
         if (valid) {
@@ -466,8 +538,12 @@ __global__ void __launch_bounds__(SCATTER_W * 32)
     sort_scatter_kernel(const int32_t* __restrict__ key, const int32_t* __restrict__ n_take,
                         const int32_t* __restrict__ p_take, const uint8_t* __restrict__ pt_keep,
                         const int32_t* __restrict__ s_dev, int64_t s_cap, int64_t m, int64_t nchunks,
-                        int64_t chn, const int32_t* __restrict__ hoff, int4* __restrict__ sd_rec) {
+                        int64_t chn, const int32_t* __restrict__ hoff, int4* __restrict__ sd_rec,
+                        int32_t* __restrict__ sd_start) {
     extern __shared__ int run[];  // [W][m]: per-warp counts, then running offsets
+    // sd_start[j] = hoff[j * nchunks] (start of bucket j), sd_start[m] = s
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j <= m; j += (int64_t)gridDim.x * blockDim.x)
+        sd_start[j] = hoff[j * nchunks];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
     int* myrun = run + (int64_t)w * m;
     const int64_t s = min((int64_t)*s_dev, s_cap);
@@ -548,52 +624,53 @@ __global__ void __launch_bounds__(SCATTER_W * 32)
     }
 }
 
-// sd_start[j] = hoff[j * nchunks] (start of bucket j), sd_start[m] = s
-__global__ void sort_starts_kernel(const int32_t* __restrict__ hoff, int64_t m, int64_t nchunks,
-                                   int32_t* __restrict__ sd_start) {
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j <= m;
-         j += (int64_t)gridDim.x * blockDim.x)
-        sd_start[j] = hoff[j * nchunks];
-}
-
 // ---------------------------------------------------------------------------
 // work queue
 // ---------------------------------------------------------------------------
-__global__ void work_count_kernel(const int32_t* __restrict__ sd_start, int64_t m, const uint8_t* __restrict__ sel,
-                                  int chunk, int32_t* __restrict__ nit) {
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < m;
-         j += (int64_t)gridDim.x * blockDim.x) {
-        const int c = sd_start[j + 1] - sd_start[j];
-        nit[j] = (sel && !sel[j]) ? 0 : (c + chunk - 1) / chunk;
-    }
-}
+// A CTA makes the items of WORK_T subdomains: it adds the item counts of the
+// subdomains before its own (m reads, from L2), scans its own, and its warps
+// write the items of one subdomain after the other (a subdomain holding all
+// points has hundreds of them).  One launch; count, scan and fill apart take four.
+constexpr int WORK_T = 256;
 
-// one warp per subdomain: the lanes write its items (a subdomain holding all
-// points has hundreds of them)
-__global__ void work_fill_kernel(const int32_t* __restrict__ sd_start, int64_t m, const int32_t* __restrict__ ioff,
-                                 int chunk, int32_t* __restrict__ items, int32_t* __restrict__ item_start,
-                                 int32_t* __restrict__ n_items, int64_t cap, int32_t* __restrict__ status) {
-    const int lane = threadIdx.x & 31;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t j = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; j < m; j += nw) {
-        const int i0 = ioff[j], i1 = ioff[j + 1];
-        const int b = sd_start[j], e = sd_start[j + 1];
-        for (int it = i0 + lane; it < i1; it += 32) {
-            if (it >= cap) {
+__global__ void __launch_bounds__(WORK_T) work_kernel(const int32_t* __restrict__ sd_start, int64_t m,
+                                                      const uint8_t* __restrict__ sel, int chunk,
+                                                      int32_t* __restrict__ items, int32_t* __restrict__ item_start,
+                                                      int32_t* __restrict__ n_items, int64_t cap,
+                                                      int32_t* __restrict__ status) {
+    __shared__ int sw[33];
+    __shared__ int2 s_item[WORK_T];  // first item and number of items of the CTA's subdomains
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t j0 = (int64_t)blockIdx.x * WORK_T;
+    auto count = [&](int64_t j) {
+        return (sel && !sel[j]) ? 0 : (sd_start[j + 1] - sd_start[j] + chunk - 1) / chunk;
+    };
+    int before = 0, prefix, total;
+    for (int64_t j = threadIdx.x; j < j0; j += WORK_T) before += count(j);
+    block_exclusive_scan(before, sw, prefix);  // prefix = the sum over the CTA
+    const int64_t j = j0 + threadIdx.x;
+    const int c = j < m ? count(j) : 0;
+    const int i0 = prefix + block_exclusive_scan(c, sw, total);
+    s_item[threadIdx.x] = make_int2(i0, c);
+    if (j < m) item_start[j] = (int32_t)min((int64_t)i0, cap);
+    if (j == m - 1) {
+        item_start[m] = (int32_t)min((int64_t)(i0 + c), cap);
+        *n_items = (int32_t)min((int64_t)(i0 + c), cap);
+    }
+    __syncthreads();
+    for (int q = w; q < WORK_T && j0 + q < m; q += WORK_T / 32) {
+        const int2 it = s_item[q];
+        const int b = sd_start[j0 + q], e = sd_start[j0 + q + 1];
+        for (int k = lane; k < it.y; k += 32) {
+            const int64_t i = (int64_t)it.x + k;
+            if (i >= cap) {
                 atomicOr(status, FBP_STATUS_ITEM_OVERFLOW);
                 break;
             }
-            const int beg = b + (it - i0) * chunk;
-            items[3 * (int64_t)it + 0] = (int32_t)j;
-            items[3 * (int64_t)it + 1] = beg;
-            items[3 * (int64_t)it + 2] = min(chunk, e - beg);
-        }
-        if (lane == 0) {
-            item_start[j] = min((int64_t)i0, cap);
-            if (j == m - 1) {
-                item_start[m] = min((int64_t)i1, cap);
-                *n_items = (int32_t)min((int64_t)i1, cap);
-            }
+            const int beg = b + k * chunk;
+            items[3 * i + 0] = (int32_t)(j0 + q);
+            items[3 * i + 1] = beg;
+            items[3 * i + 2] = min(chunk, e - beg);
         }
     }
 }
@@ -667,6 +744,51 @@ extern "C" int fbp_scan_i32(const int32_t* in, int32_t* out, int64_t n, void* sc
     return scan_launch(in, out, n, (int32_t*)scratch, as_stream(stream));
 }
 
+// sums: see inside_count_kernel (excludes model_count in shared memory)
+static int launch_count(const float* x, int64_t n, const fbp_boxes* boxes, int32_t* pt_count, int32_t* pt_nlvl,
+                        uint64_t* pt_lvl, int32_t* model_count, uint64_t* pt_hit, int32_t* pt_cand, int2* sums,
+                        cudaStream_t st) {
+    const bool shist = model_count && boxes->m <= COUNT_MAX_M;
+    const int t = shist ? COUNT_T : LIST_CHUNK;
+    const int g = shist ? grid_for(n, t, COUNT_CTAS) : grid_for(n, t);
+    const size_t shm = shist ? (size_t)boxes->m * sizeof(int32_t) : 0;
+#define X(D)                                                                                                         \
+    if (boxes->xd == D) {                                                                                            \
+        if (shist)                                                                                                   \
+            inside_count_kernel<D, true><<<g, t, shm, st>>>(x, n, *boxes, pt_count, pt_nlvl, pt_lvl, model_count,    \
+                                                            pt_hit, pt_cand, nullptr);                               \
+        else                                                                                                         \
+            inside_count_kernel<D, false><<<g, t, 0, st>>>(x, n, *boxes, pt_count, pt_nlvl, pt_lvl, model_count,     \
+                                                           pt_hit, pt_cand, sums);                                   \
+    }
+    X(1) X(2) X(3)
+#undef X
+    FBP_LAUNCH_CHECK();
+    return FBP_OK;
+}
+
+static int launch_fill(const float* x, int64_t n, const fbp_boxes* boxes, int32_t* pt_off, int32_t* np_off,
+                       const int32_t* pt_count, const int2* sums, const uint64_t* pt_lvl, const uint64_t* pt_hit,
+                       const int32_t* pt_cand, int32_t* n_take, int32_t* m_take, int32_t* p_take, int32_t* np_take,
+                       int64_t s_cap, int64_t u_cap, int32_t* status, cudaStream_t st) {
+    const int g = grid_for(n, FILL_WARPS * 32, 8);  // 32 points per warp
+#define X(D)                                                                                                        \
+    if (boxes->xd == D) {                                                                                           \
+        if (sums)                                                                                                   \
+            inside_fill_kernel<D, true><<<g, FILL_WARPS * 32, 0, st>>>(                                             \
+                x, n, *boxes, pt_off, np_off, pt_count, sums, pt_lvl, pt_hit, pt_cand, n_take, m_take, p_take,      \
+                np_take, s_cap, u_cap, status);                                                                     \
+        else                                                                                                        \
+            inside_fill_kernel<D, false><<<g, FILL_WARPS * 32, 0, st>>>(                                            \
+                x, n, *boxes, pt_off, np_off, nullptr, nullptr, pt_lvl, pt_hit, pt_cand, n_take, m_take, p_take,    \
+                np_take, s_cap, u_cap, status);                                                                     \
+    }
+    X(1) X(2) X(3)
+#undef X
+    FBP_LAUNCH_CHECK();
+    return FBP_OK;
+}
+
 extern "C" int fbp_inside_count(const float* x, int64_t n, const fbp_boxes* boxes, int32_t* pt_count,
                                 int32_t* pt_nlvl, uint64_t* pt_lvl, int32_t* model_count, uint64_t* pt_hit,
                                 int32_t* pt_cand, void* stream) {
@@ -674,24 +796,8 @@ extern "C" int fbp_inside_count(const float* x, int64_t n, const fbp_boxes* boxe
     if (rc) return rc;
     FBP_REQUIRE(pt_count && (x || n == 0), FBP_ERR_INVALID, "fbp_inside_count: null pointer");
     if (n == 0) return FBP_OK;
-    const bool shist = model_count && boxes->m <= COUNT_MAX_M;
-    const int t = shist ? COUNT_T : 256;
-    const int g = shist ? grid_for(n, t, COUNT_CTAS) : grid_for(n, t);
-    const size_t shm = shist ? (size_t)boxes->m * sizeof(int32_t) : 0;
-    cudaStream_t st = as_stream(stream);
-#define X(D)                                                                                                      \
-    if (boxes->xd == D) {                                                                                        \
-        if (shist)                                                                                                \
-            inside_count_kernel<D, true><<<g, t, shm, st>>>(x, n, *boxes, pt_count, pt_nlvl, pt_lvl, model_count, \
-                                                             pt_hit, pt_cand);                                    \
-        else                                                                                                      \
-            inside_count_kernel<D, false><<<g, t, 0, st>>>(x, n, *boxes, pt_count, pt_nlvl, pt_lvl, model_count, \
-                                                            pt_hit, pt_cand);                                     \
-    }
-    X(1) X(2) X(3)
-#undef X
-    FBP_LAUNCH_CHECK();
-    return FBP_OK;
+    return launch_count(x, n, boxes, pt_count, pt_nlvl, pt_lvl, model_count, pt_hit, pt_cand, nullptr,
+                        as_stream(stream));
 }
 
 extern "C" int fbp_inside_fill(const float* x, int64_t n, const fbp_boxes* boxes, const int32_t* pt_off,
@@ -706,15 +812,41 @@ extern "C" int fbp_inside_fill(const float* x, int64_t n, const fbp_boxes* boxes
     FBP_REQUIRE((n_take && m_take && p_take) || s_cap == 0, FBP_ERR_INVALID, "fbp_inside_fill: null take");
     FBP_REQUIRE(np_take || u_cap == 0, FBP_ERR_INVALID, "fbp_inside_fill: null np_take");
     if (n == 0) return FBP_OK;
-    const int g = grid_for(n, FILL_WARPS * 32, 8);  // 32 points per warp
+    return launch_fill(x, n, boxes, const_cast<int32_t*>(pt_off), const_cast<int32_t*>(np_off), nullptr, nullptr,
+                       pt_lvl, pt_hit, pt_cand, n_take, m_take, p_take, np_take, s_cap, u_cap, status,
+                       as_stream(stream));
+}
+
+extern "C" size_t fbp_inside_lists_scratch_bytes(int64_t n) {
+    return (size_t)((n + LIST_CHUNK - 1) / LIST_CHUNK + 1) * sizeof(int2);
+}
+
+extern "C" int fbp_inside_lists(const float* x, int64_t n, const fbp_boxes* boxes, int32_t* pt_count,
+                                uint64_t* pt_lvl, uint64_t* pt_hit, int32_t* pt_cand, int32_t* pt_off,
+                                int32_t* np_off, int32_t* n_take, int32_t* m_take, int32_t* p_take, int32_t* np_take,
+                                int64_t s_cap, int64_t u_cap, int32_t* status, void* scratch, size_t scratch_bytes,
+                                void* stream) {
+    int rc = check_boxes(boxes);
+    if (rc) return rc;
+    FBP_REQUIRE(pt_off && np_off && status, FBP_ERR_INVALID, "fbp_inside_lists: null pointer");
+    FBP_REQUIRE(n == 0 || (x && pt_count && pt_lvl), FBP_ERR_INVALID, "fbp_inside_lists: null pointer");
+    FBP_REQUIRE(!pt_hit == !pt_cand, FBP_ERR_INVALID, "fbp_inside_lists: pt_hit and pt_cand go together");
+    FBP_REQUIRE((n_take && m_take && p_take) || s_cap == 0, FBP_ERR_INVALID, "fbp_inside_lists: null take");
+    FBP_REQUIRE(np_take || u_cap == 0, FBP_ERR_INVALID, "fbp_inside_lists: null np_take");
+    FBP_REQUIRE(n >= 0 && n < (int64_t)1 << 31, FBP_ERR_INVALID, "fbp_inside_lists: n=%lld", (long long)n);
+    FBP_REQUIRE(scratch && ((uintptr_t)scratch & 7) == 0 && scratch_bytes >= fbp_inside_lists_scratch_bytes(n),
+                FBP_ERR_CAPACITY, "fbp_inside_lists: scratch too small");
     cudaStream_t st = as_stream(stream);
-    switch (boxes->xd) {
-        case 1: inside_fill_kernel<1><<<g, FILL_WARPS * 32, 0, st>>>(x, n, *boxes, pt_off, np_off, pt_lvl, pt_hit, pt_cand, n_take, m_take, p_take, np_take, s_cap, u_cap, status); break;
-        case 2: inside_fill_kernel<2><<<g, FILL_WARPS * 32, 0, st>>>(x, n, *boxes, pt_off, np_off, pt_lvl, pt_hit, pt_cand, n_take, m_take, p_take, np_take, s_cap, u_cap, status); break;
-        case 3: inside_fill_kernel<3><<<g, FILL_WARPS * 32, 0, st>>>(x, n, *boxes, pt_off, np_off, pt_lvl, pt_hit, pt_cand, n_take, m_take, p_take, np_take, s_cap, u_cap, status); break;
+    if (n == 0) {
+        FBP_CUDA_CHECK(cudaMemsetAsync(pt_off, 0, sizeof(int32_t), st));
+        FBP_CUDA_CHECK(cudaMemsetAsync(np_off, 0, sizeof(int32_t), st));
+        return FBP_OK;
     }
-    FBP_LAUNCH_CHECK();
-    return FBP_OK;
+    int2* sums = static_cast<int2*>(scratch);
+    rc = launch_count(x, n, boxes, pt_count, nullptr, pt_lvl, nullptr, pt_hit, pt_cand, sums, st);
+    if (rc) return rc;
+    return launch_fill(x, n, boxes, pt_off, np_off, pt_count, sums, pt_lvl, pt_hit, pt_cand, n_take, m_take, p_take,
+                       np_take, s_cap, u_cap, status, st);
 }
 
 extern "C" int fbp_gather_i32(const int32_t* in, int64_t n, const int32_t* count_dev, const int32_t* inv,
@@ -795,9 +927,7 @@ static int sort_pairs(const int32_t* m_take, const int32_t* n_take, const int32_
     if (nch > 0) {
         const int g = (int)std::min<int64_t>(nch, (int64_t)sm_count() * 32 / sw);
         sort_scatter_kernel<<<g, 32 * sw, shm * sw, st>>>(m_take, n_take, p_take, pt_keep, s_dev, s_cap, m, nch,
-                                                          chn, hoff, reinterpret_cast<int4*>(sd_rec));
-        FBP_LAUNCH_CHECK();
-        sort_starts_kernel<<<grid_for(m + 1, 256), 256, 0, st>>>(hoff, m, nch, sd_start);
+                                                          chn, hoff, reinterpret_cast<int4*>(sd_rec), sd_start);
         FBP_LAUNCH_CHECK();
     } else {
         FBP_CUDA_CHECK(cudaMemsetAsync(sd_start, 0, (size_t)(m + 1) * sizeof(int32_t), st));
@@ -849,15 +979,8 @@ extern "C" int fbp_build_work(const int32_t* sd_start, int64_t m, const uint8_t*
     FBP_REQUIRE(scratch && scratch_bytes >= fbp_work_scratch_bytes(m), FBP_ERR_CAPACITY,
                 "fbp_build_work: scratch too small");
     cudaStream_t st = as_stream(stream);
-    int32_t* nit = (int32_t*)scratch;
-    int32_t* ioff = nit + (m + 1);
-    int32_t* sums = ioff + (m + 1);
-    work_count_kernel<<<grid_for(m, 256), 256, 0, st>>>(sd_start, m, select, chunk, nit);
-    FBP_LAUNCH_CHECK();
-    int rc = scan_launch(nit, ioff, m, sums, st);
-    if (rc) return rc;
-    work_fill_kernel<<<grid_for(m * 32, 256), 256, 0, st>>>(sd_start, m, ioff, chunk, items, item_start, n_items,
-                                                        items_cap, status);
+    work_kernel<<<(unsigned)((m + WORK_T - 1) / WORK_T), WORK_T, 0, st>>>(sd_start, m, select, chunk, items, item_start,
+                                                                        n_items, items_cap, status);
     FBP_LAUNCH_CHECK();
     return FBP_OK;
 }

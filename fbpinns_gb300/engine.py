@@ -11,11 +11,11 @@ Step (fused path, built-in problems), all stream-ordered, no host sync:
     forward_pairs   per-pair jets of u*w and w            (K-fwd)
     pou_loss        POU combination, hard constraint, PDE residual,
                     FP64 loss partials, per-slot seeds    (K-seg + K-loss)
-    loss_finalize   deterministic FP64 sum
     adjoint_pairs   per-pair recompute + adjoint, one gradient partial per
                     work item                             (K-adj)
-    grad_reduce     partials -> grad (m, P) in item order
-    adam            masked Adam with the shared count     (K-adam)
+    step_tail       deterministic FP64 sum of the loss, partials ->
+                    grad (m, P) in item order, masked Adam with the
+                    shared count                          (K-adam)
 
 With ``resample=True`` a step also draws new uniform points (Philox) and
 rebuilds the interaction lists on the device into fixed-capacity buffers, so
@@ -394,6 +394,7 @@ class FBPINNEngine:
         nparts = 8 * torch.cuda.get_device_properties(dev).multi_processor_count + 1
         self.loss_part = torch.zeros(nparts, dtype=torch.float64, device=dev)
         self.loss = torch.zeros(1, dtype=torch.float64, device=dev)
+        self._ticket = torch.zeros(1, dtype=torch.int32, device=dev)  # fbp_step_tail's, zero between steps
         self.npou = self.grid.npou
         self._problem = None
 
@@ -486,7 +487,7 @@ class FBPINNEngine:
                                         _lib.stream_ptr(stream)),
                    "fbp_pou_backward")
 
-    def pou_loss(self, ps, U_out=None, stream=None):
+    def pou_loss(self, ps, U_out=None, stream=None, finalize=True):
         if self._problem is None:
             raise RuntimeError("set_problem() first: the fused loss needs a built-in problem")
         lib = _lib.load()
@@ -499,11 +500,16 @@ class FBPINNEngine:
                                     _lib.ptr(ps.slot_out), _lib.ptr(U_out), ps.pair_out.shape[0], ps.slot_out.shape[0],
                                     _lib.ptr(self.loss_part),
                                     self.loss_part.numel(), _lib.ptr(t.status), st), "fbp_pou_loss")
-        # a scheduled point set's partials are already divided by its training-point count
-        _lib.check(lib.fbp_loss_finalize(_lib.ptr(self.loss_part), self.loss_part.numel(),
-                                         1.0 if ps.scheduled else 1.0 / ps.n, _lib.ptr(self.loss), st),
-                   "fbp_loss_finalize")
+        if finalize:
+            _lib.check(lib.fbp_loss_finalize(_lib.ptr(self.loss_part), self.loss_part.numel(), self._loss_scale(ps),
+                                             _lib.ptr(self.loss), st), "fbp_loss_finalize")
         return self.loss
+
+    @staticmethod
+    def _loss_scale(ps):
+        """The loss is the mean over the points; a scheduled point set's partials
+        are already divided by its training-point count."""
+        return 1.0 if ps.scheduled else 1.0 / ps.n
 
     def adjoint(self, ps, theta=None, out=None, stream=None, reduce=True, z2=True):
         """Gradient partials of the loss seeds in ps.slot_out; z2: read the
@@ -543,10 +549,18 @@ class FBPINNEngine:
     def fused_step(self, ps, lr, stream=None, **adam_kw):
         """One training step on point set ps; returns the device loss (float64, 1 elem)."""
         self.forward_pairs(ps, stream=stream)
-        loss = self.pou_loss(ps, stream=stream)
-        self.adjoint(ps, stream=stream)
-        self.adam(lr, stream=stream, **adam_kw)
-        return loss
+        self.pou_loss(ps, stream=stream, finalize=False)
+        self.adjoint(ps, stream=stream, reduce=False)
+        self._tail(ps, lr, stream=stream, **adam_kw)
+        return self.loss
+
+    def _tail(self, ps, lr, b1=0.9, b2=0.999, eps=1e-8, eps_root=0.0, stream=None):
+        """The loss, the gradient from the items' partials and its Adam step, one launch."""
+        _lib.check(_lib.load().fbp_step_tail(
+            _lib.ptr(self.loss_part), self.loss_part.numel(), self._loss_scale(ps), _lib.ptr(self.loss),
+            _lib.ptr(ps.grad_part), _lib.ptr(ps.item_start_act), _lib.ptr(self.grad), _lib.ptr(self.theta),
+            _lib.ptr(self.m1), _lib.ptr(self.m2), _lib.ptr(self.state), self.m, self.P, lr, b1, b2, eps, eps_root,
+            _lib.ptr(self.count), _lib.ptr(self._ticket), _lib.stream_ptr(stream)), "fbp_step_tail")
 
     def sample(self, x_out, seed, offset, xmin, xmax, counter=None, stream=None, order=None):
         """Uniform points into x_out; the stream offset is offset + *counter.

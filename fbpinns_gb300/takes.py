@@ -99,6 +99,8 @@ class PointTakes:
         lib = _lib.load()
         self._scan_scratch = torch.empty(int(lib.fbp_scan_scratch_bytes(self.n)) // 4 + 1, dtype=torch.int32,
                                          device=dev)
+        self._list_scratch = torch.empty(int(lib.fbp_inside_lists_scratch_bytes(self.n)) // 4, dtype=torch.int32,
+                                         device=dev)
         self.s_cap = s_cap
         self.u_cap = u_cap
         self._alloc(s_cap or 0, u_cap or 0)
@@ -126,6 +128,17 @@ class PointTakes:
         assert x.is_cuda and x.dtype == torch.float32 and x.shape == (self.n, self.grid.xd)
         x = x.contiguous()
         # the status word is sticky: cleared only by reset_status()
+        if self.s_cap is not None and not count_models:  # nothing to read back: two launches
+            _lib.check(lib.fbp_inside_lists(_lib.ptr(x), self.n, C.byref(b), _lib.ptr(self.pt_count),
+                                            _lib.ptr(self.pt_lvl), _lib.ptr(self.pt_hit) if self.use_hit_masks else None,
+                                            _lib.ptr(self.pt_cand) if self.use_hit_masks else None,
+                                            _lib.ptr(self.pt_off), _lib.ptr(self.np_off), _lib.ptr(self.n_take),
+                                            _lib.ptr(self.m_take), _lib.ptr(self.p_take), _lib.ptr(self.np_take),
+                                            self.n_take.numel(), self.np_take.numel(), _lib.ptr(self.status),
+                                            _lib.ptr(self._list_scratch), self._list_scratch.numel() * 4, st),
+                       "fbp_inside_lists")
+            self._sizes = None
+            return None
         if count_models:
             self.model_count.zero_()
         _lib.check(lib.fbp_inside_count(_lib.ptr(x), self.n, C.byref(b), _lib.ptr(self.pt_count),

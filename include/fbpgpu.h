@@ -280,6 +280,16 @@ int fbp_inside_fill(const float* x, int64_t n, const fbp_boxes* boxes,
                     int32_t* n_take, int32_t* m_take, int32_t* p_take, int32_t* np_take,
                     int64_t s_cap, int64_t u_cap, int32_t* status, void* stream);
 
+/* fbp_inside_count, the two exclusive scans and fbp_inside_fill in two
+ * launches, with the same results (pt_count and pt_lvl are working arrays,
+ * pt_hit / pt_cand optional ones); scratch 8-byte aligned. */
+size_t fbp_inside_lists_scratch_bytes(int64_t n);
+int fbp_inside_lists(const float* x, int64_t n, const fbp_boxes* boxes, int32_t* pt_count,
+                     uint64_t* pt_lvl, uint64_t* pt_hit, int32_t* pt_cand,
+                     int32_t* pt_off, int32_t* np_off, int32_t* n_take, int32_t* m_take,
+                     int32_t* p_take, int32_t* np_take, int64_t s_cap, int64_t u_cap,
+                     int32_t* status, void* scratch, size_t scratch_bytes, void* stream);
+
 /* out[i] = inv[in[i]] for i < *count_dev (or < n when count_dev is NULL):
  * the re-index of m_take to positions in all_ims = [active; fixed]
  * (fbpinns/trainers.py:367-372). */
@@ -405,6 +415,15 @@ int fbp_has_tc_adjoint_shape(int32_t xd, int32_t h1, int32_t h2, int32_t d2mask,
 /* grad[j] = sum of the partials of subdomain j's items, in item order. */
 int fbp_grad_reduce(const float* grad_part, const int32_t* item_start, int64_t m,
                     int32_t nparam, float* grad, void* stream);
+
+/* fbp_loss_finalize, fbp_grad_reduce and fbp_adam in one launch, with the same
+ * results.  ticket: one int32, zero before the first call and left at zero;
+ * calls that share it must not overlap. */
+int fbp_step_tail(const double* loss_part, int32_t n_part, double scale, double* loss,
+                  const float* grad_part, const int32_t* item_start, float* grad,
+                  float* theta, float* m1, float* m2, const uint8_t* state, int64_t m,
+                  int32_t nparam, float lr, float b1, float b2, float eps, float eps_root,
+                  int32_t* count_dev, int32_t* ticket, void* stream);
 
 /* Adam (optax.adam defaults and ordering, the shared step count) applied to
  * rows j with state[j] == 1 only; other rows untouched.  count_dev is the

@@ -892,3 +892,37 @@ def test_host_point_order_follows_probe_extent(cuda):
     torch.cuda.synchronize()
     st.check()
     assert np.isfinite(float(st.loss_host.item()))
+
+
+@pytest.mark.parametrize("n", [1, 500])
+def test_fused_step_tail_matches_separate_launches(cuda, n):
+    """fbp_step_tail (loss, gradient, Adam, step count in one launch) bitwise
+    against loss_finalize + grad_reduce + adam, over three steps with an
+    inactive network and one whose items are many (chunks of 64 pairs)."""
+    static = decomposition("multilevel")
+    m = static["m"]
+    layers = random_layers([2, 16, 16, 1], m, seed=2)
+    spec = PR.Poisson2D.fused_spec({"static": {"problem": PR.Poisson2D.init_params(n_freq=3, sd=0.1)[0]}})
+    x = torch.rand((n, 2), generator=torch.Generator().manual_seed(5))
+    state = np.ones(m, dtype=int)
+    state[1] = 2
+    out = []
+    for fused in (True, False):
+        eng = _engine(static, layers, 3 | _lib.D2_LAPLACIAN, chunk=64)
+        eng.set_problem(spec)
+        eng.set_state(state)
+        ps = eng.points(x)
+        losses = []
+        for _ in range(3):
+            if fused:
+                loss = eng.fused_step(ps, 1e-3)
+            else:
+                eng.forward_pairs(ps)
+                loss = eng.pou_loss(ps)
+                eng.adjoint(ps)
+                eng.adam(1e-3)
+            losses.append(loss.item())
+        out.append((losses, [t.clone() for t in (eng.grad, eng.theta, eng.m1, eng.m2, eng.count)]))
+    assert out[0][0] == out[1][0]
+    for a, b in zip(out[0][1], out[1][1]):
+        assert torch.equal(a, b)

@@ -209,3 +209,55 @@ def test_points_per_box_counts(cuda, m, n):
     t.build(torch.from_numpy(x).cuda())
     ref = np.array([((x >= lo[j]) & (x <= hi[j])).sum() for j in range(m)])
     np.testing.assert_array_equal(_np(t.model_count), ref)
+
+
+@pytest.mark.parametrize("hits", [True, False])
+@pytest.mark.parametrize("n", [1, 255, 257, 4097, 400_001])
+def test_lists_in_two_launches_match_separate_scans(cuda, n, hits):
+    """fbp_inside_lists (capacities given: count, then fill with the offsets)
+    against count, scans and fill: one chunk of 256 points, a rest, and more
+    chunks than the fill pass has CTAs; points outside every box included."""
+    g = T.grid_of(decomposition("multilevel"))
+    x = (torch.rand((n, 2), generator=torch.Generator().manual_seed(n)) * 3 - 1).cuda()
+    ref = T.PointTakes(g, n)
+    ref.use_hit_masks = hits
+    s, u = ref.build(x)
+    t = T.PointTakes(g, n, s_cap=s, u_cap=u)
+    t.use_hit_masks = hits
+    t.n_take.fill_(-1)
+    assert t.build(x, count_models=False) is None
+    t.check_status()
+    for k in ("pt_off", "np_off"):
+        assert torch.equal(getattr(t, k), getattr(ref, k)), k
+    for k, c in (("n_take", s), ("m_take", s), ("p_take", s), ("np_take", u)):
+        assert torch.equal(getattr(t, k)[:c], getattr(ref, k)[:c]), k
+
+
+@pytest.mark.parametrize("m", [1, 255, 256, 257, 1000])
+def test_work_queue_of_many_subdomains(cuda, m):
+    """fbp_build_work against numpy at the edges of its CTAs' 256 subdomains:
+    empty, unselected, one-item and many-item subdomains."""
+    from fbpinns_gb300 import _lib
+    lib = _lib.load()
+    rng = np.random.default_rng(m)
+    c = rng.choice([0, 1, 63, 64, 65, 700], m)
+    c[0] = 5000
+    sel = (rng.uniform(size=m) < 0.8).astype(np.uint8)
+    start = np.concatenate([[0], np.cumsum(c)]).astype(np.int32)
+    ref = [(j, b, min(64, start[j + 1] - b)) for j in range(m) if sel[j] for b in range(start[j], start[j + 1], 64)]
+    cap = len(ref) + 1
+    items = torch.full((3 * cap,), -1, dtype=torch.int32, device="cuda")
+    istart = torch.zeros(m + 1, dtype=torch.int32, device="cuda")
+    cnt, status = (torch.zeros(1, dtype=torch.int32, device="cuda") for _ in range(2))
+    nb = int(lib.fbp_work_scratch_bytes(m))
+    scratch = torch.empty(nb // 4 + 1, dtype=torch.int32, device="cuda")
+    sd, se = torch.from_numpy(start).cuda(), torch.from_numpy(sel).cuda()
+    for limit in (cap, max(len(ref) // 2, 1)):
+        status.zero_()
+        _lib.check(lib.fbp_build_work(_lib.ptr(sd), m, _lib.ptr(se), 64, _lib.ptr(items), _lib.ptr(istart), _lib.ptr(cnt),
+                                      limit, _lib.ptr(status), _lib.ptr(scratch), nb, _lib.stream_ptr()), "fbp_build_work")
+        k = min(len(ref), limit)
+        assert int(cnt.item()) == k and int(status.item()) == (4 if limit < len(ref) else 0)
+        np.testing.assert_array_equal(_np(items)[:3 * k].reshape(-1, 3), np.array(ref, dtype=np.int64).reshape(-1, 3)[:k])
+        first = np.concatenate([[0], np.cumsum([sum(1 for r in ref if r[0] == j) for j in range(m)])])
+        np.testing.assert_array_equal(_np(istart), np.minimum(first, limit))
