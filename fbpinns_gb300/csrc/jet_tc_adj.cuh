@@ -1,5 +1,6 @@
-// Tensor-core (tcgen05, 3xTF32) per-pair adjoint for tanh networks with two
-// hidden layers of equal width H = 16 or 32.
+// Tensor-core (tcgen05, 3xTF32) per-pair adjoint for networks with two hidden
+// layers of equal width H = 16 or 32 and tanh, sin or adaptive activations
+// (TcAct; written for tanh below).
 //
 // Of the adjoint's three layer-2 contractions, two have the pairs as rows and
 // run on the tensor cores with the pair-dependent operand in tensor memory
@@ -35,7 +36,10 @@
 // Measured on a GB300, against the FMA adjoint (jet.cuh): 2.34e6 pairs of
 // 2-16-16-1 networks, J = 4, 0.466 -> 0.337 ms; a training step of 4096
 // networks 2-32-32-1 on 2.1e6 points 17.0 -> 11.9 ms, of 900 networks 3-32-32-1
-// (J = 6) on 58^3 points 6.44 -> 4.40 ms with the same forward.
+// (J = 6) on 58^3 points 6.44 -> 4.40 ms with the same forward; of 341 SIRENs
+// 2-16-16-1 on 65537 points 815 -> 582 us, of as many AdaptiveFCNs 840 -> 530 us
+// (the parameters of adaptive activations need no sums over pairs of their own:
+// their gradients follow from the weights', at the item's end).
 //
 // Waits on the MMA-completion mbarriers are bounded: on a time-out the kernel
 // records FBP_STATUS_TC_TIMEOUT, stops, waits once more and frees its TMEM.
@@ -47,9 +51,9 @@ namespace fbp {
 
 template <class C>
 struct TcAdj {
-    static_assert(C::TWO && C::H1 == C::H2 && (C::H1 == 16 || C::H1 == 32) && C::EXTRA == 0 && C::J <= 6,
-                  "tensor-core adjoint shape");
-    static constexpr int H = C::H1, J = C::J, XD = C::XD, NS = C::NS;
+    static_assert(C::TWO && C::H1 == C::H2 && (C::H1 == 16 || C::H1 == 32) && C::J <= 6, "tensor-core adjoint shape");
+    static constexpr int H = C::H1, J = C::J, XD = C::XD, NS = C::NS, E = C::EXTRA;
+    static constexpr bool SINL = TcAct<C>::template SIN<false>;
     static constexpr int NPT = H / 8;      // threads per pair
     static constexpr int T = 128 * NPT;    // threads per CTA
     static constexpr int NW = T / 32;
@@ -75,11 +79,14 @@ struct TcAdj {
     // the tile's pairs
     static constexpr int NQ = J > 4 ? 1 : 2;
     static constexpr int KB = H / 16, SUB = KB * (H / (8 * NQ)), PG = NW / SUB, PPG = 128 / PG;
-    // per-thread sums of b1 and W1's value part, kept in shared memory between
-    // tiles (as float4, conflict-free) where it has the room
-    static constexpr int NST = 2 * (1 + XD);
-    static constexpr int BASE = 4 * (4 * J * H * H + 128 * (ZS + AS) + 2 * (XD + J) * 128 + 4 * NPT * 48);
-    static constexpr bool STASH = BASE + NST * T * 16 <= (H == 16 ? 110 : 222) * 1024;
+    // per-thread sums over the item's pairs of 8 neurons: W3, b2, b1, W1's value part
+    static constexpr int iW3 = 0, iB2 = 1, iB1 = 2, iW1 = 3, NSUM = 3 + XD;
+    // those from iB1 on are kept in shared memory between tiles where it has
+    // the room (as float4, conflict-free), else in registers
+    static constexpr int NST = 2 * (NSUM - iB1);
+    static constexpr int BASE = 4 * (4 * J * H * H + 128 * (ZS + AS * (SINL ? 2 : 1)) + 2 * (XD + J) * 128 +
+                                     4 * NPT * 8 * NSUM);
+    static constexpr bool STASH = BASE + NST * T * 16 <= (H == 16 ? 111 : 222) * 1024;
 };
 
 template <class C>
@@ -89,10 +96,12 @@ struct TcAdjSmem {
     float b2[2][A::J * A::H * A::H];  // GEMM 2 B: component c's H x H matrix, rows n, K = k
     float zb[128 * A::ZS];            // z2bar rows; at the item's end the S_c of the pair groups
     float a1[128 * A::AS];            // layer-1 activations
+    float tp1[A::SINL ? 128 * A::AS : 4];  // and their first derivatives where those do not follow from them
     float xo[2][A::XD + A::J][128];   // per pair of this and the next tile: normalised point, o-bar jet
-    float red[4 * A::NPT][48];        // per warp: the item's sums over its lanes
+    float red[4 * A::NPT][8 * A::NSUM];  // per warp: the item's sums over its lanes
     float4 stash[A::STASH ? A::NST : 1][A::STASH ? A::T : 1];
     float red3[4];
+    float redx[2][A::H];  // sums of W2 W2-bar over k and over n (adaptive activations)
     uint64_t mbar[2];
     uint32_t tmem_base;
 };
@@ -105,7 +114,7 @@ __device__ __forceinline__ void tc_adj_issue1(uint32_t tmem, uint32_t b_hi, uint
     using A = TcAdj<C>;
     constexpr int H = A::H, c0 = O == 0 ? 0 : (O == 1 ? 1 : 1 + A::XD), nc = O == 0 ? 1 : (O == 1 ? A::XD : A::NS);
     constexpr uint32_t idesc = umma_idesc_tf32(128, nc * H), rows = (uint32_t)(c0 * (H / 8)) * KMajor<H>::SBO;
-    const uint32_t d = tmem + A::cZ + c0 * H, a = tmem + O * A::OP;
+    const uint32_t d = tmem + A::cZ + c0 * H, a = tmem + (A::SINL && O == 2 ? 0 : O) * A::OP;
 #pragma unroll
     for (int p = 0; p < 3; ++p)
 #pragma unroll
@@ -152,8 +161,9 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
                                                                                     float* __restrict__ grad_part,
                                                                                     int32_t* __restrict__ status) {
     using A = TcAdj<C>;
-    constexpr int J = C::J, XD = C::XD, NS = C::NS, H = A::H, RS = rec_stride(J), NPT = A::NPT, NA = A::NA;
-    static_assert(A::PG * J * H * H <= 128 * A::ZS && J * H * (H + 1) <= 128 * A::ZS, "S_c fit the z2bar rows");
+    using F = TcAct<C>;
+    constexpr int J = C::J, XD = C::XD, NS = C::NS, E = A::E, H = A::H, RS = rec_stride(J), NPT = A::NPT, NA = A::NA;
+    static_assert(A::PG * J * H * H <= 128 * A::ZS && (XD + 2) * H * (H + 1) <= 128 * A::ZS, "S_c fit the z2bar rows");
     __shared__ SParams<C> S;
     __shared__ int s_item;
     extern __shared__ float4 dyn_smem[];
@@ -251,21 +261,19 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
 #pragma unroll
             for (int c = 0; c < J; ++c) {
                 const float f = c == 0 ? 1.0f : (c <= XD ? S.cw[n * XD + (c - 1)] : S.c2[n * NS + (c - 1 - XD)]);
-                float hi, lo;
-                split_tf32_rn(w2[e] * f, hi, lo);
-                // the factor -2 of tpp = -2 a tp: with the second-derivative
-                // operands of GEMM 1, with the tangents of GEMM 2 (T_1 tpp)
-                const float s1 = c > XD ? -2.0f : 1.0f, s2 = c >= 1 && c <= XD ? -2.0f : 1.0f;
-                T.b1[0][c * H * H + o] = s1 * hi;  // rows k, K = n
-                T.b1[1][c * H * H + o] = s1 * lo;
-                T.b2[0][c * H * H + ot] = s2 * hi;  // rows n, K = k
-                T.b2[1][c * H * H + ot] = s2 * lo;
+                // k2 = tpp / m2 goes with the second-derivative operands of GEMM 1
+                // and the tangents of GEMM 2 (T_1 tpp), o^2 with its second
+                // derivatives (T_2 tppp)
+                const float o1 = act_o<C, false>(S, n), k2 = F::template k2<false>(o1), v = w2[e] * f;
+                const float v1 = c > XD ? v * k2 : v, v2 = c == 0 ? v : (c <= XD ? v * k2 : v * (o1 * o1));
+                split_tf32_rn(v1, T.b1[0][c * H * H + o], T.b1[1][c * H * H + o]);    // rows k, K = n
+                split_tf32_rn(v2, T.b2[0][c * H * H + ot], T.b2[1][c * H * H + ot]);  // rows n, K = k
             }
         }
         if (h == 1 && 128 + r < cnt) rec = pair_rec(pr, beg + 128 + r);  // the second tile's pairs
         fence_async_smem();
-        float sacc[J][A::NQ][4];  // S_c, 16 k x 8 NQ n as MMA accumulators (c > XD: over tpp / -2)
-        float2 g3[4], gb2[4], gb1[4], gw1[XD][4];
+        float sacc[J][A::NQ][4];  // S_c, 16 k x 8 NQ n as MMA accumulators (c > XD: over m2 = tpp / k2)
+        float2 sum[A::NSUM][4];  // see TcAdj
         float g3b = 0.f;
 #pragma unroll
         for (int c = 0; c < J; ++c)
@@ -274,22 +282,22 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
 #pragma unroll
                 for (int i = 0; i < 4; ++i) sacc[c][q][i] = 0.f;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            g3[q] = gb2[q] = gb1[q] = dup2(0.f);
+        for (int i = 0; i < A::NSUM; ++i)
 #pragma unroll
-            for (int d = 0; d < XD; ++d) gw1[d][q] = dup2(0.f);
-        }
-        auto stash = [&](bool load) {  // gb1 and gw1 from / to shared memory
+            for (int q = 0; q < 4; ++q) sum[i][q] = dup2(0.f);
+        auto stash = [&](bool load) {  // the sums from iB1 on, from / to shared memory
 #pragma unroll
-            for (int i = 0; i < A::NST; ++i) {
-                float2(&v)[4] = i < 2 ? gb1 : gw1[i < 2 ? 0 : i / 2 - 1];
-                if (load) {
-                    const float4 w = T.stash[A::STASH ? i : 0][A::STASH ? tid : 0];
-                    v[2 * (i & 1)] = make_float2(w.x, w.y);
-                    v[2 * (i & 1) + 1] = make_float2(w.z, w.w);
-                } else {
-                    T.stash[A::STASH ? i : 0][A::STASH ? tid : 0] =
-                        make_float4(v[2 * (i & 1)].x, v[2 * (i & 1)].y, v[2 * (i & 1) + 1].x, v[2 * (i & 1) + 1].y);
+            for (int i = A::iB1; i < A::NSUM; ++i) {
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    float4& w = T.stash[A::STASH ? 2 * (i - A::iB1) + b : 0][A::STASH ? tid : 0];
+                    if (load) {
+                        const float4 v = w;
+                        sum[i][2 * b] = make_float2(v.x, v.y);
+                        sum[i][2 * b + 1] = make_float2(v.z, v.w);
+                    } else {
+                        w = make_float4(sum[i][2 * b].x, sum[i][2 * b].y, sum[i][2 * b + 1].x, sum[i][2 * b + 1].y);
+                    }
                 }
             }
         };
@@ -317,20 +325,25 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
 #pragma unroll
                     for (int d = 0; d < XD; ++d)
                         z = fma2(make_float2(S.W1[n * XD + d], S.W1[(n + 1) * XD + d]), dup2(xn[d]), z);
-                    const float2 av = tanh_fast2(z);
-                    const float2 t1 = fma2(make_float2(-av.x, -av.y), av, dup2(1.0f));
+                    float2 av, t1;
+                    F::template first<false>(S, n, z, av, t1);
                     a[q] = av.x, a[q + 1] = av.y;
                     tp[q] = t1.x, tp[q + 1] = t1.y;
-                    if constexpr (NS > 0) {
-                        const float2 t2 = mul2(av, t1);  // tpp / -2; the factor is in B
+                    if constexpr (NS > 0 && !A::SINL) {
+                        const float2 t2 = F::template m2<false>(av, t1);
                         tpp[q] = t2.x, tpp[q + 1] = t2.y;
                     }
                 }
                 *reinterpret_cast<float4*>(arow) = make_float4(a[0], a[1], a[2], a[3]);
                 *reinterpret_cast<float4*>(arow + 4) = make_float4(a[4], a[5], a[6], a[7]);
+                if constexpr (A::SINL) {
+                    float* trow = &T.tp1[r * A::AS + n0];
+                    *reinterpret_cast<float4*>(trow) = make_float4(tp[0], tp[1], tp[2], tp[3]);
+                    *reinterpret_cast<float4*>(trow + 4) = make_float4(tp[4], tp[5], tp[6], tp[7]);
+                }
                 tmem_st_split8(mine, H, a);
                 tmem_st_split8(mine + A::OP, H, tp);
-                if constexpr (NS > 0) tmem_st_split8(mine + 2 * A::OP, H, tpp);
+                if constexpr (NS > 0 && !A::SINL) tmem_st_split8(mine + 2 * A::OP, H, tpp);
             }
             tmem_wait_st();
             tc_fence_before();
@@ -364,16 +377,16 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
 #pragma unroll
                     for (int c = 0; c < J; ++c) z[c] = make_float2(acc[c][2 * q], acc[c][2 * q + 1]);
                     z[0] = add2(z[0], *reinterpret_cast<const float2*>(&S.b2[k]));
-                    const float2 a = tanh_fast2(z[0]);
-                    const float2 tp = fma2(make_float2(-a.x, -a.y), a, dup2(1.0f));
-                    const float2 m2 = mul2(a, tp), tpp = mul2(dup2(-2.0f), m2);
-                    const float2 tppp = mul2(tp, fma2(dup2(-6.0f), tp, dup2(4.0f)));  // tp (6 a^2 - 2), a^2 = 1 - tp
+                    float2 a, tp;
+                    F::template first<true>(S, k, z[0], a, tp);
+                    const float2 tpp = F::template second<true>(S, k, F::template m2<true>(a, tp));
+                    const float2 tppp = F::template third<true>(S, k, tp);
                     // the sensitivities of sigma' and sigma'' over W3: P = sum_d ob_d z_d +
                     // sum_s ob_s z_s, Q = sum_s ob_s sum_d z_d^2; then W3-bar += ob_0 a +
                     // tp P + tpp Q, z2bar_0 = W3 (ob_0 tp + tpp P + tppp Q), z2bar_d =
                     // W3 (ob_d tp + 2 ob_s tpp z_d), z2bar_s = W3 ob_s tp
                     const float2 w3 = *reinterpret_cast<const float2*>(&S.W3[k]);
-                    const float2 wtp = mul2(w3, tp), w4 = mul2(dup2(-4.0f), mul2(w3, m2));  // 2 W3 tpp
+                    const float2 wtp = mul2(w3, tp), w4 = mul2(dup2(2.0f), mul2(w3, tpp));
                     float2 P = mul2(dup2(ob[1]), z[1]), Q = dup2(0.f), zb[J];
 #pragma unroll
                     for (int d = 1; d < XD; ++d) P = fma2(dup2(ob[1 + d]), z[1 + d], P);
@@ -395,15 +408,15 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
                         Q = s == 0 ? mul2(os, q2) : fma2(os, q2, Q);
                         zb[1 + XD + s] = mul2(os, wtp);
                     }
-                    float2 s3 = fma2(tp, P, fma2(dup2(ob[0]), a, g3[q]));
+                    float2 s3 = fma2(tp, P, fma2(dup2(ob[0]), a, sum[A::iW3][q]));
                     float2 z0 = fma2(tpp, P, mul2(dup2(ob[0]), tp));
                     if constexpr (NS > 0) {
                         s3 = fma2(tpp, Q, s3);
                         z0 = fma2(tppp, Q, z0);
                     }
                     zb[0] = mul2(w3, z0);
-                    g3[q] = s3;
-                    gb2[q] = add2(gb2[q], zb[0]);
+                    sum[A::iW3][q] = s3;
+                    sum[A::iB2][q] = add2(sum[A::iB2][q], zb[0]);
 #pragma unroll
                     for (int c = 0; c < J; ++c) acc[c][2 * q] = zb[c].x, acc[c][2 * q + 1] = zb[c].y;
                 }
@@ -436,20 +449,28 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
                 const int p2 = sp + 2 * (lane & 3);
                 const float* zr = &T.zb[p2 * A::ZS + sk];
                 const float* ar = &T.a1[p2 * A::AS + sn + (lane >> 2)];
+                const float* tr = A::SINL ? &T.tp1[p2 * A::AS + sn + (lane >> 2)] : nullptr;
 #pragma unroll 1
-                for (int p = 0; p < np; p += 8, zr += 8 * A::ZS, ar += 8 * A::AS) {
+                for (int p = 0; p < np; p += 8, zr += 8 * A::ZS, ar += 8 * A::AS, tr += 8 * A::AS) {
                     float bh[NA][A::NQ][2], bl[NA][A::NQ][2];
 #pragma unroll
                     for (int q = 0; q < A::NQ; ++q) {
                         const float2 a = make_float2(ar[8 * q], ar[A::AS + 8 * q]);
-                        const float2 tp = fma2(make_float2(-a.x, -a.y), a, dup2(1.0f));
+                        float2 tp;
+                        if constexpr (A::SINL) {
+                            tp = make_float2(tr[8 * q], tr[A::AS + 8 * q]);
+                        } else {
+                            float2 t = a;
+                            if constexpr (E > 0) t = mul2(a, dup2(act_o<C, false>(S, sn + (lane >> 2) + 8 * q)));
+                            tp = fma2(make_float2(-t.x, -t.y), t, dup2(1.0f));
+                        }
                         split(a, bh[0][q], bl[0][q]);
                         split(tp, bh[1][q], bl[1][q]);
-                        if constexpr (NS > 0) split(mul2(a, tp), bh[NA - 1][q], bl[NA - 1][q]);  // tpp / -2
+                        if constexpr (NS > 0 && !A::SINL) split(F::template m2<false>(a, tp), bh[NA - 1][q], bl[NA - 1][q]);
                     }
 #pragma unroll
                     for (int c = 0; c < J; ++c) {
-                        const int o = c == 0 ? 0 : (c <= XD ? 1 : NA - 1);
+                        const int o = c == 0 ? 0 : (c <= XD ? 1 : (A::SINL ? 0 : NA - 1));
                         float ah[4], al[4];
                         split(make_float2(zr[c * H], zr[c * H + 8]), ah, al);
                         split(make_float2(zr[A::ZS + c * H], zr[A::ZS + c * H + 8]), ah + 2, al + 2);
@@ -485,18 +506,31 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
                 tmem_wait_ld();
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
+                    const int n = n0 + 2 * q;
                     const float2 a = *reinterpret_cast<const float2*>(arow + 2 * q);
-                    const float2 tp = fma2(make_float2(-a.x, -a.y), a, dup2(1.0f));
-                    // z1bar = tp (T_0 + a T_1 + (6 a^2 - 2) T_2), T_1 over B times -2
-                    float2 z1 = fma2(a, make_float2(tb[1][2 * q], tb[1][2 * q + 1]),
-                                     make_float2(tb[0][2 * q], tb[0][2 * q + 1]));
-                    if constexpr (NS > 0)
-                        z1 = fma2(fma2(dup2(-6.0f), tp, dup2(4.0f)),
-                                  make_float2(tb[NA - 1][2 * q], tb[NA - 1][2 * q + 1]), z1);
-                    z1 = mul2(z1, tp);
-                    gb1[q] = add2(gb1[q], z1);
+                    const float2 t0 = make_float2(tb[0][2 * q], tb[0][2 * q + 1]);
+                    const float2 t1 = make_float2(tb[1][2 * q], tb[1][2 * q + 1]);
+                    const float2 t2 = NS > 0 ? make_float2(tb[NA - 1][2 * q], tb[NA - 1][2 * q + 1]) : dup2(0.f);
+                    float2 tp, z1;
+                    if constexpr (A::SINL) {
+                        tp = *reinterpret_cast<const float2*>(&T.tp1[r * A::AS + n]);
+                    } else {
+                        float2 t = a;
+                        if constexpr (E > 0) t = mul2(a, make_float2(act_o<C, false>(S, n), act_o<C, false>(S, n + 1)));
+                        tp = fma2(make_float2(-t.x, -t.y), t, dup2(1.0f));
+                    }
+                    if constexpr (A::SINL) {
+                        // z1bar = tp (T_0 - T_2) + a T_1, with the factors in B
+                        z1 = fma2(a, t1, mul2(tp, add2(t0, make_float2(-t2.x, -t2.y))));
+                    } else {
+                        // z1bar = tp (T_0 + a T_1 + (4 - 6 tp) T_2)
+                        z1 = fma2(a, t1, t0);
+                        if constexpr (NS > 0) z1 = fma2(fma2(dup2(-6.0f), tp, dup2(4.0f)), t2, z1);
+                        z1 = mul2(z1, tp);
+                    }
+                    sum[A::iB1][q] = add2(sum[A::iB1][q], z1);
 #pragma unroll
-                    for (int d = 0; d < XD; ++d) gw1[d][q] = fma2(z1, dup2(xn[d]), gw1[d][q]);
+                    for (int d = 0; d < XD; ++d) sum[A::iW1 + d][q] = fma2(z1, dup2(xn[d]), sum[A::iW1 + d][q]);
                 }
                 if constexpr (A::STASH) stash(false);
             }
@@ -506,25 +540,32 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
         float* dst = grad_part + (size_t)it * C::P;
         if constexpr (A::STASH) stash(true);
         {
-            float v[32];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                v[2 * q] = g3[q].x, v[2 * q + 1] = g3[q].y;
-                v[8 + 2 * q] = gb2[q].x, v[8 + 2 * q + 1] = gb2[q].y;
-                v[16 + 2 * q] = gb1[q].x, v[16 + 2 * q + 1] = gb1[q].y;
-                v[24 + 2 * q] = gw1[0][q].x, v[24 + 2 * q + 1] = gw1[0][q].y;
-            }
-            warp_reduce_scatter<32>(v, lane);
-            T.red[warp][lane] = v[0];
-            if constexpr (XD > 1) {
-                float u[16];
+            for (int i0 = 0; i0 < A::NSUM; i0 += 4) {
+                constexpr int NS4 = A::NSUM;
+                if (NS4 - i0 > 2) {
+                    float v[32];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    u[2 * q] = gw1[1][q].x, u[2 * q + 1] = gw1[1][q].y;
-                    u[8 + 2 * q] = XD > 2 ? gw1[XD - 1][q].x : 0.f, u[8 + 2 * q + 1] = XD > 2 ? gw1[XD - 1][q].y : 0.f;
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const float2 w = i0 + i < NS4 ? sum[i0 + i < NS4 ? i0 + i : 0][q] : dup2(0.f);
+                            v[8 * i + 2 * q] = w.x, v[8 * i + 2 * q + 1] = w.y;
+                        }
+                    warp_reduce_scatter<32>(v, lane);
+                    if (8 * i0 + lane < 8 * NS4) T.red[warp][8 * i0 + lane] = v[0];
+                } else {
+                    float v[16];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const float2 w = i0 + i < NS4 ? sum[i0 + i < NS4 ? i0 + i : 0][q] : dup2(0.f);
+                            v[8 * i + 2 * q] = w.x, v[8 * i + 2 * q + 1] = w.y;
+                        }
+                    warp_reduce_scatter<16>(v, lane);
+                    if (!(lane & 1) && 8 * i0 + (lane >> 1) < 8 * NS4) T.red[warp][8 * i0 + (lane >> 1)] = v[0];
                 }
-                warp_reduce_scatter<16>(u, lane);
-                if (!(lane & 1)) T.red[warp][32 + (lane >> 1)] = u[0];
             }
             if (h == 0) {
 #pragma unroll
@@ -543,7 +584,7 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
             }
         next = pr.item_ctr ? s_item : it + (int)gridDim.x;
         __syncthreads();
-        float s[PT][J];
+        float s[PT][J], w2bar[PT];
 #pragma unroll
         for (int e = 0; e < PT; ++e) {
             const int i = tid + e * A::T, n = i % H;
@@ -552,7 +593,7 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
                 float v = 0.f;
 #pragma unroll
                 for (int g = 0; g < A::PG; ++g) v += T.zb[(g * J + c) * H * H + i];
-                s[e][c] = c > XD ? -2.0f * v : v;
+                s[e][c] = c > XD ? F::template k2<false>(act_o<C, false>(S, n)) * v : v;
             }
             float v = s[e][0];
 #pragma unroll
@@ -560,6 +601,7 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
 #pragma unroll
             for (int q = 0; q < NS; ++q) v = fmaf(S.c2[n * NS + q], s[e][1 + XD + q], v);
             dst[C::oW2 + i] = v;
+            w2bar[e] = v;
         }
         __syncthreads();
         // the tangent part of W1-bar: [d][k] rows of W2[k][n] (S_{1+d} + 2 cw_d sum_s S_s), summed over k
@@ -576,15 +618,21 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
                 v = fmaf(2.0f * S.cw[n * XD + d], v, s[e][1 + d]);
                 T.zb[(d * H + n) * (H + 1) + k] = wkn * v;
             }
+            if constexpr (E > 0) {  // W2 * W2-bar, for the sums over k and over n
+                T.zb[(XD * H + n) * (H + 1) + k] = wkn * w2bar[e];
+                T.zb[((XD + 1) * H + k) * (H + 1) + n] = wkn * w2bar[e];
+            }
         }
         __syncthreads();
-        for (int o = warp; o < H * XD; o += A::NW) {  // one warp per (n, d)
-            const int n = o / XD, d = o - n * XD;
+        for (int o = warp; o < H * (XD + (E > 0 ? 2 : 0)); o += A::NW) {  // one warp per (d, n)
+            const int d = o / H, n = o - d * H;
             float v = lane < H ? T.zb[(d * H + n) * (H + 1) + lane] : 0.f;
 #pragma unroll
             for (int q = 16; q > 0; q >>= 1) v += __shfl_xor_sync(0xffffffffu, v, q);
-            if (lane == 0) {
-                const int q = n & 7, w0 = (n >> 3) * 4, at = d == 0 ? 24 + q : 32 + 8 * (d - 1) + q;
+            if (E > 0 && d >= XD) {
+                if (lane == 0) T.redx[d - XD][n] = v;
+            } else if (lane == 0) {
+                const int w0 = (n >> 3) * 4, at = 8 * (A::iW1 + d) + (n & 7);
                 float u = 0.f;
 #pragma unroll
                 for (int w = 0; w < 4; ++w) u += T.red[w0 + w][at];
@@ -592,11 +640,45 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
             }
         }
         for (int i = tid; i < 3 * H; i += A::T) {
-            const int g = i / H, n = i - g * H, w0 = (n >> 3) * 4, at = g * 8 + (n & 7);
+            const int g = i / H, n = i - g * H, w0 = (n >> 3) * 4;
             float u = 0.f;
 #pragma unroll
-            for (int w = 0; w < 4; ++w) u += T.red[w0 + w][at];
-            dst[(g == 0 ? C::oW3 : (g == 1 ? C::ob2 : C::ob1)) + n] = u;
+            for (int w = 0; w < 4; ++w) u += T.red[w0 + w][8 * g + (n & 7)];
+            dst[(g == A::iW3 ? C::oW3 : (g == A::iB2 ? C::ob2 : C::ob1)) + n] = u;
+        }
+        if constexpr (E > 0) {
+            // Activation parameters of sigma(z) = c f(o z): o scales the weights into
+            // the neuron and c those out of it, so
+            //   dL/do = (sum of W Wbar + b bbar of its layer) / o,
+            //   dL/dc = (sum of W Wbar of the next layer) / c
+            // AdaptiveFCN (c = a, o = 1/a): dL/da = dL/dc - o^2 dL/do.
+            __syncthreads();  // the entries read back below are written
+            if (tid < 2 * H) {
+                const bool l2 = tid >= H;
+                const int n = l2 ? tid - H : tid;
+                float go, gc;
+                if (l2) {
+                    go = T.redx[1][n] + S.b2[n] * dst[C::ob2 + n];
+                    gc = S.W3[n] * dst[C::oW3 + n];
+                } else {
+                    go = S.b1[n] * dst[C::ob1 + n];
+#pragma unroll
+                    for (int d = 0; d < XD; ++d) go = fmaf(S.W1[n * XD + d], dst[C::oW1 + n * XD + d], go);
+                    gc = T.redx[0][n];
+                }
+                const float c = l2 ? act_c<C, true>(S, n) : act_c<C, false>(S, n);
+                const float o = l2 ? act_o<C, true>(S, n) : act_o<C, false>(S, n);
+                go /= o;
+                gc /= c;
+                float* gx = dst + (l2 ? C::oX2 : C::oX1) + n;
+                if constexpr (C::ACT == FBP_ACT_ADAPTIVE_TANH) {
+                    gx[0] = gc - o * o * go;
+                } else {
+                    gx[0] = gc;
+                    gx[H] = go;
+                }
+            }
+            if (tid < E) dst[C::oX3 + tid] = 0.f;  // the output layer's parameters are unused
         }
         if (tid == 0) dst[C::ob3] = (T.red3[0] + T.red3[1]) + (T.red3[2] + T.red3[3]);
     }

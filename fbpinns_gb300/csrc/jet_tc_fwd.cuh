@@ -1,9 +1,13 @@
-// Tensor-core (tcgen05, 3xTF32) per-pair forward jets for tanh networks with
-// two hidden layers of H = 16 or 32 neurons.
+// Tensor-core (tcgen05, 3xTF32) per-pair forward jets for networks with two
+// hidden layers of H = 16 or 32 neurons.
 //
-// As in forward_pairs_tc_kernel (the other activations), layer 2 is J GEMMs per
-// tile of 128 pairs with the pair-dependent operands a, tp, tpp and the
-// per-neuron scales in B_c = W2 diag(f_c).  In shared memory the operands of a
+// Layer 2 of the jet, z_c[k] = sum_n W2[k][n] v_c[n] (+ b2[k] for c = 0), is J
+// GEMMs per tile of 128 pairs.  The layer-1 jet components factor as v_0 = a,
+// v_{1+d} = tp cw[:, d] and v_{1+xd+s} = tpp c2_s (a, tp, tpp = the activation
+// and its first two derivatives at the neuron's pre-activation; cw = W1 / sd,
+// c2_s the sum of cw[:, d]^2 over the dims of second-derivative slot s), so
+// the pair-dependent operands are only a, tp and tpp / k2 (TcAct), and the
+// per-neuron scales are in B_c = W2 diag(f_c).  In shared memory the operands of a
 // tile take 48 or 96 KB and an MMA at least 40 cycles to read them; here they
 // live in tensor memory, written by the threads of the pair (H / 8 per pair,
 // eight neurons each; two CTAs of 256 threads or one of 512 per SM), where an
@@ -18,9 +22,13 @@
 // and the tile's two barriers.  Measured on a GB300: 2.34e6 pairs of 2-16-16-1
 // networks, J = 4, 0.161 -> 0.137 ms (operands in shared memory, one thread per
 // pair); a training step of 4096 networks 2-32-32-1 on 2.1e6 points 11.9 ->
-// 10.0 ms, of 900 networks 3-32-32-1 (J = 6) on 58^3 points 4.40 -> 3.47 ms
-// (FMA kernel before).
+// 10.0 ms, of 900 networks 3-32-32-1 (J = 6) on 58^3 points 4.40 -> 3.47 ms, of
+// 341 SIRENs or AdaptiveFCNs 2-16-16-1 on 65537 points 582 -> 570 and 530 -> 509
+// us (FMA kernel before).
 #pragma once
+
+#include <algorithm>
+#include <atomic>
 
 #include "tc_ops.cuh"
 
@@ -28,8 +36,8 @@ namespace fbp {
 
 template <class C>
 struct TcFwd {
-    static_assert(C::TWO && C::H1 == C::H2 && (C::H1 == 16 || C::H1 == 32) && C::EXTRA == 0,
-                  "tensor-core forward shape");
+    static_assert(C::TWO && C::H1 == C::H2 && (C::H1 == 16 || C::H1 == 32), "tensor-core forward shape");
+    static constexpr bool SINL = TcAct<C>::template SIN<false>;  // the tpp operand is a
     static constexpr int H = C::H1, J = C::J, XD = C::XD, NS = C::NS;
     static constexpr int NPT = H / 8, T = 128 * NPT;
     static constexpr int NA = NS > 0 ? 3 : 2, OP = 2 * H;
@@ -60,7 +68,7 @@ __device__ __forceinline__ void tc_fwd_issue(uint32_t tmem, uint32_t zcol, uint3
     using A = TcFwd<C>;
     constexpr int H = A::H, c0 = O == 0 ? 0 : (O == 1 ? 1 : 1 + A::XD), nc = O == 0 ? 1 : (O == 1 ? A::XD : A::NS);
     constexpr uint32_t idesc = umma_idesc_tf32(128, nc * H), rows = (uint32_t)(c0 * (H / 8)) * KMajor<H>::SBO;
-    const uint32_t d = tmem + zcol + c0 * H, a = tmem + O * A::OP;
+    const uint32_t d = tmem + zcol + c0 * H, a = tmem + (A::SINL && O == 2 ? 0 : O) * A::OP;
 #pragma unroll
     for (int p = 0; p < 3; ++p)
 #pragma unroll
@@ -75,6 +83,7 @@ __global__ void __launch_bounds__(TcFwd<C>::T) __maxnreg__(TcFwd<C>::REGS) forwa
                                                                            fbp_pairs pr, float* __restrict__ pair_out,
                                                                            int32_t* __restrict__ status) {
     using A = TcFwd<C>;
+    using F = TcAct<C>;
     constexpr int J = C::J, XD = C::XD, NS = C::NS, H = A::H, RS = rec_stride(J), NPT = A::NPT, NA = A::NA;
     __shared__ SParams<C> S;
     __shared__ int s_item;
@@ -145,7 +154,8 @@ __global__ void __launch_bounds__(TcFwd<C>::T) __maxnreg__(TcFwd<C>::REGS) forwa
 #pragma unroll
             for (int c = 0; c < J; ++c) {
                 const float f = c == 0 ? 1.0f : (c <= XD ? S.cw[n * XD + (c - 1)] : S.c2[n * NS + (c - 1 - XD)]);
-                split_tf32_rn(w2[e] * f, T.b[0][c * H * H + o], T.b[1][c * H * H + o]);
+                const float v = c > XD ? w2[e] * f * F::template k2<false>(act_o<C, false>(S, n)) : w2[e] * f;
+                split_tf32_rn(v, T.b[0][c * H * H + o], T.b[1][c * H * H + o]);
             }
         }
         fence_async_smem();
@@ -177,7 +187,25 @@ __global__ void __launch_bounds__(TcFwd<C>::T) __maxnreg__(TcFwd<C>::REGS) forwa
                         __stcs(zs + (size_t)(c * H + k + 1) * pr.zs_cap, z[c].y);
                     }
                 }
-                tanh_jet_pair<C>(z, g);
+                float2 tp;
+                F::template first<true>(S, k, z[0], g[0], tp);
+#pragma unroll
+                for (int d = 0; d < XD; ++d) g[1 + d] = mul2(tp, z[1 + d]);
+                if constexpr (NS > 0) {
+                    const float2 tpp = F::template second<true>(S, k, F::template m2<true>(g[0], tp));
+#pragma unroll
+                    for (int s = 0; s < NS; ++s) {
+                        float2 q2 = dup2(0.f);  // sum of z_d^2 over the slot's dims
+                        bool first = true;
+#pragma unroll
+                        for (int d = 0; d < XD; ++d)
+                            if ((C::slot_dims(s) >> d) & 1) {
+                                q2 = first ? mul2(z[1 + d], z[1 + d]) : fma2(z[1 + d], z[1 + d], q2);
+                                first = false;
+                            }
+                        g[1 + XD + s] = fma2(tp, z[1 + XD + s], mul2(tpp, q2));
+                    }
+                }
                 const float2 w3 = *reinterpret_cast<const float2*>(&S.W3[k]);
 #pragma unroll
                 for (int c = 0; c < J; ++c) o2[c] = fma2(w3, g[c], o2[c]);
@@ -245,18 +273,18 @@ __global__ void __launch_bounds__(TcFwd<C>::T) __maxnreg__(TcFwd<C>::REGS) forwa
 #pragma unroll
                     for (int d = 0; d < XD; ++d)
                         z = fma2(make_float2(S.W1[n * XD + d], S.W1[(n + 1) * XD + d]), dup2(xn[d]), z);
-                    const float2 av = tanh_fast2(z);
-                    const float2 t1 = fma2(make_float2(-av.x, -av.y), av, dup2(1.0f));
+                    float2 av, t1;
+                    F::template first<false>(S, n, z, av, t1);
                     a[q] = av.x, a[q + 1] = av.y;
                     tp[q] = t1.x, tp[q + 1] = t1.y;
-                    if constexpr (NS > 0) {
-                        const float2 t2 = mul2(mul2(dup2(-2.0f), av), t1);
+                    if constexpr (NS > 0 && !A::SINL) {
+                        const float2 t2 = F::template m2<false>(av, t1);
                         tpp[q] = t2.x, tpp[q + 1] = t2.y;
                     }
                 }
                 tmem_st_split8(mine, H, a);
                 tmem_st_split8(mine + A::OP, H, tp);
-                if constexpr (NS > 0) tmem_st_split8(mine + 2 * A::OP, H, tpp);
+                if constexpr (NS > 0 && !A::SINL) tmem_st_split8(mine + 2 * A::OP, H, tpp);
             }
             tmem_wait_st();
             tc_fence_before();
@@ -309,10 +337,10 @@ __global__ void __launch_bounds__(TcFwd<C>::T) __maxnreg__(TcFwd<C>::REGS) forwa
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(A::COLS) : "memory");
 }
 
-template <int XD, int H, int D2>
+template <int XD, int H, int D2, int ACT>
 int launch_forward_tm(const fbp_net& net, const float* x, const fbp_pairs& pr, float* pair_out, int32_t* status,
                       int grid, cudaStream_t st) {
-    using C = TcCfg<Cfg<XD, H, H, D2, FBP_ACT_TANH>>;
+    using C = TcCfg<Cfg<XD, H, H, D2, ACT>>;
     FBP_REQUIRE(net.nparam == C::P, FBP_ERR_INVALID, "forward_tc: nparam %d != %d for this shape", net.nparam, C::P);
     // 512 / COLS CTAs per SM share its tensor memory (a further one would wait
     // in tcgen05.alloc); enough shared memory is asked for that no more fit
@@ -332,12 +360,18 @@ int launch_forward_tm(const fbp_net& net, const float* x, const fbp_pairs& pr, f
     return FBP_OK;
 }
 
-template <int XD, int H, int D2>
+template <int XD, int H, int D2, int ACT>
 int tm_try(int mode, const fbp_net& net, const float* x, const fbp_pairs& pr, float* pair_out, int32_t* status,
            int grid, cudaStream_t st) {
-    if (net.xd != XD || net.h1 != H || net.h2 != H || net.d2mask != D2 || net.act != FBP_ACT_TANH) return 1;
+    if (net.xd != XD || net.h1 != H || net.h2 != H || net.d2mask != D2 || net.act != ACT) return 1;
     if (mode == 2) return FBP_OK;
-    return launch_forward_tm<XD, H, D2>(net, x, pr, pair_out, status, grid, st);
+    return launch_forward_tm<XD, H, D2, ACT>(net, x, pr, pair_out, status, grid, st);
 }
 
 }  // namespace fbp
+
+#define FBP_TM_TRY(XD, H, D2, ACT)                                                             \
+    {                                                                                          \
+        int r_ = fbp::tm_try<XD, H, D2, ACT>(mode, *net, x, *pr, pair_out, status, grid, st);   \
+        if (r_ != 1) return r_;                                                                \
+    }

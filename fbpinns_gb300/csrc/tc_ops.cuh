@@ -3,7 +3,7 @@
 // MMA with A in TMEM, the TF32 split and the K-major layout of the B operands.
 #pragma once
 
-#include "jet_tc.cuh"
+#include "jet.cuh"
 
 namespace fbp {
 
@@ -13,6 +13,65 @@ template <class B>
 struct TcCfg : B {
     static constexpr bool W2S = false;
 };
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+// Shared-memory matrix descriptor: start, leading (K) and stride (M/N) byte
+// offsets between core matrices, descriptor version 1, no swizzle.
+__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
+    d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
+    d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
+    d |= (uint64_t)1 << 46;
+    return d;
+}
+
+// Instruction descriptor of kind::tf32: FP32 accumulator, TF32 A and B, both
+// K-major, N >> 3 at bit 17, M >> 4 at bit 24.
+__host__ __device__ constexpr uint32_t umma_idesc_tf32(int M, int N) {
+    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+
+__device__ __forceinline__ void umma_commit(uint32_t mbar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
+                 : "memory");
+}
+
+__device__ __forceinline__ bool mbar_try_wait(uint32_t mbar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
+__device__ __forceinline__ uint64_t global_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Bounded wait: true when the phase completed, false once limit_ns of wall
+// time has passed without it.
+__device__ __forceinline__ bool mbar_wait_bounded(uint32_t mbar, uint32_t parity, uint64_t limit_ns) {
+    const uint64_t t0 = global_ns();
+    while (!mbar_try_wait(mbar, parity))
+        if (global_ns() - t0 > limit_ns) return false;
+    return true;
+}
+
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+constexpr uint64_t TC_WAIT_NS = 200000000ull;  // 0.2 s: an MMA group takes microseconds
+constexpr uint64_t TC_TEST_WAIT_NS = 1000000ull;  // 1 ms, with FBP_STATUS_TC_TEST_NO_MMA
 
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const float (&v)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr),
@@ -113,6 +172,60 @@ struct KMajor {
     __device__ __forceinline__ static void at(int o, int& row, int& k) {
         row = (o / (8 * H)) * 8 + ((o >> 2) & 7);
         k = ((o % (8 * H)) >> 5) * 4 + (o & 3);
+    }
+};
+
+// Activations of the tensor-core kernels: from a = sigma and tp = sigma' the
+// second and third derivatives are products with the neuron's o (c f(o z)),
+//   tanh, adaptive tanh (c o = 1):  tp = 1 - (o a)^2, tpp = -2 o^2 a tp, tppp = o^2 tp (4 - 6 tp)
+//   sin, adaptive sin:              tpp = -o^2 a,     tppp = -o^2 tp
+// so the tpp operand of an MMA is m2 = a tp (tanh) or a itself (sin), with
+// k2 = tpp / m2 in the other operand.
+template <class C>
+struct TcAct {
+    // L2: layer 2 (else layer 1)
+    template <bool L2>
+    static constexpr int ACT = L2 ? act_layer2(C::ACT) : act_layer1(C::ACT);
+    template <bool L2>
+    static constexpr bool SIN = ACT<L2> == FBP_ACT_SIN || ACT<L2> == FBP_ACT_ADAPTIVE_SIN;
+    // k2 and o^2 of a neuron with activation parameter o
+    template <bool L2>
+    __device__ __forceinline__ static float k2(float o) {
+        return (SIN<L2> ? -1.0f : -2.0f) * (C::EXTRA > 0 ? o * o : 1.0f);
+    }
+    // neurons n, n + 1 at the pre-activations z: value and first derivative
+    template <bool L2>
+    __device__ __forceinline__ static void first(const SParams<C>& S, int n, float2 z, float2& a, float2& tp) {
+        if constexpr (ACT<L2> == FBP_ACT_TANH) {
+            a = tanh_fast2(z);
+            tp = fma2(make_float2(-a.x, -a.y), a, dup2(1.0f));
+        } else {
+            using A = Act<ACT<L2>>;
+            float d2, d3;
+            A::derivs(A::stored(z.x, act_o<C, L2>(S, n)), act_c<C, L2>(S, n), act_o<C, L2>(S, n), a.x, tp.x, d2, d3);
+            A::derivs(A::stored(z.y, act_o<C, L2>(S, n + 1)), act_c<C, L2>(S, n + 1), act_o<C, L2>(S, n + 1), a.y, tp.y,
+                      d2, d3);
+        }
+    }
+    template <bool L2>
+    __device__ __forceinline__ static float2 m2(float2 a, float2 tp) {
+        return SIN<L2> ? a : mul2(a, tp);
+    }
+    template <bool L2>
+    __device__ __forceinline__ static float2 oo(const SParams<C>& S, int n) {
+        const float2 o = make_float2(act_o<C, L2>(S, n), act_o<C, L2>(S, n + 1));
+        return mul2(o, o);
+    }
+    // the second derivative from m2 of neurons n, n + 1, the third from tp
+    template <bool L2>
+    __device__ __forceinline__ static float2 second(const SParams<C>& S, int n, float2 m2) {
+        const float2 t = mul2(dup2(SIN<L2> ? -1.0f : -2.0f), m2);
+        return C::EXTRA > 0 ? mul2(oo<L2>(S, n), t) : t;
+    }
+    template <bool L2>
+    __device__ __forceinline__ static float2 third(const SParams<C>& S, int n, float2 tp) {
+        const float2 t = SIN<L2> ? make_float2(-tp.x, -tp.y) : mul2(tp, fma2(dup2(-6.0f), tp, dup2(4.0f)));
+        return C::EXTRA > 0 ? mul2(oo<L2>(S, n), t) : t;
     }
 };
 

@@ -344,21 +344,20 @@ class FBPINNEngine:
         self.adaptive_items = bool(adaptive_items)
         self.sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
         # forward jets on the tensor cores (3xTF32) where that kernel is compiled:
-        # None = for the plain tanh FCN wherever available (for the other
-        # activations, whose sin/cos/tanh calls dominate, the FMA kernel is as
-        # fast), True = required, False = CUDA-core FMA kernel
+        # None = wherever available (but for FourierFCN, whose adjoint is the FMA
+        # kernel), True = required, False = CUDA-core FMA kernel
         tc_ok = tc_supported(self.xd, self.h1, self.h2, self.d2mask, self.act)
         if tensor_cores and not tc_ok:
             raise _lib.FBPLibraryError(f"no tensor-core forward kernel for layer sizes {ls} ({activation}, "
                                        f"d2mask {self.d2mask}); compiled: 2-16-16-1 networks and xd-32-32-1 tanh networks")
-        self.tensor_cores = (tc_ok and self.act == _lib.ACT_TANH) if tensor_cores is None else bool(tensor_cores)
+        self.tensor_cores = (tc_ok and self.act != _lib.ACT_FOURIER) if tensor_cores is None else bool(tensor_cores)
         # adjoint with its layer-2 recompute and W2^T products on the tensor cores
         # (fbp_adjoint_pairs_tc): None = where it is compiled and the caller does not
         # ask for stored z-jets; True = required; False = the FMA kernel
         tca_ok = bool(_lib.load().fbp_has_tc_adjoint_shape(self.xd, self.h1, self.h2, self.d2mask, self.act))
         if tc_adjoint and not tca_ok:
             raise _lib.FBPLibraryError(f"no tensor-core adjoint kernel for layer sizes {ls} ({activation}, "
-                                       f"d2mask {self.d2mask}); compiled: xd-16-16-1 and xd-32-32-1 tanh networks")
+                                       f"d2mask {self.d2mask}); compiled: xd-16-16-1 and xd-32-32-1 networks")
         self.tc_adjoint = tca_ok and (not store_z2 if tc_adjoint is None else bool(tc_adjoint))
         # store_z2: the forward of a training step stores the layer-2 z-jets of
         # every pair (J * h2 floats) and the FMA adjoint reads them instead of

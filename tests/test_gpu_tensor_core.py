@@ -278,3 +278,35 @@ def test_tensor_memory_kernels_match_fma(cuda, xd, h, d2, n):
     assert err.max().item() <= TC_TOL, err.tolist()
     err = (g1 - g0).abs().max(1).values / g0.abs().max(1).values.clamp(min=1e-30)
     assert err.max().item() <= TC_TOL, err.tolist()
+
+
+@pytest.mark.parametrize("act,d2", [("sin", 3 | 8), ("sin", 1), ("adaptive_tanh", 3 | 8), ("adaptive_tanh", 1),
+                                    ("adaptive_sin", 3 | 8), ("adaptive_sin", 1)])
+@pytest.mark.parametrize("n", [1, 127, 129, 2000])
+def test_tensor_core_adjoint_other_activations(cuda, act, d2, n):
+    """Adjoint of SIREN and the adaptive networks (activation parameters
+    included, which follow from the weights' gradients) against the FMA
+    adjoint for the same seeds, at the edges of the 128-pair tiles; TC_TOL of
+    each network's largest gradient."""
+    from helpers import boxes_static
+    xmin = np.array([[0.0, 0.0], [-0.5, -0.5], [0.3, 0.3]], dtype=np.float32)
+    xmax = np.array([[1.0, 1.0], [1.2, 1.2], [0.9, 0.9]], dtype=np.float32)
+    static = boxes_static(xmin, xmax)
+    layers = _net_layers(act, 3, seed=21)
+    x = torch.rand((n, 2), generator=torch.Generator().manual_seed(n))
+    seeds = torch.randn((4096, 16), generator=torch.Generator().manual_seed(1)).cuda()
+    grads = []
+    for tc in (False, True):
+        eng = FBPINNEngine(static, [2, 16, 16, 1], d2, chunk=1024, activation=act, tensor_cores=False, tc_adjoint=tc)
+        assert eng.tc_adjoint == tc
+        eng.set_theta(pack_layers(layers))
+        ps = eng.points(x)
+        eng.forward_pairs(ps)
+        ps.slot_out.copy_(seeds[:ps.slot_out.shape[0], :ps.slot_out.shape[1]])
+        ps.grad_part.fill_(float("nan"))
+        grads.append(eng.adjoint(ps).clone())
+        torch.cuda.synchronize()
+        ps.check_status()
+    assert torch.isfinite(grads[1]).all()
+    err = (grads[1] - grads[0]).abs().max(1).values / grads[0].abs().max(1).values.clamp(min=1e-30)
+    assert err.max().item() <= TC_TOL, err.tolist()
