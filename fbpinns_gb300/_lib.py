@@ -84,8 +84,9 @@ _SIG = {
     "fbp_inside_count": (C.c_int, [_P, _I64, C.POINTER(Boxes), _P, _P, _P, _P, _P, _P, _P]),
     "fbp_inside_fill": (C.c_int, [_P, _I64, C.POINTER(Boxes), _P, _P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _P, _P]),
     "fbp_inside_lists_scratch_bytes": (C.c_size_t, [_I64]),
-    "fbp_inside_lists": (C.c_int, [_P, _I64, C.POINTER(Boxes), _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _P, _P,
-                                   C.c_size_t, _P]),
+    "fbp_inside_count_chunks": (C.c_int, [_P, _I64, C.POINTER(Boxes), _P, _P, _P, _P, _P, _P, C.c_size_t, _P]),
+    "fbp_inside_fill_chunks": (C.c_int, [_P, _I64, C.POINTER(Boxes), _P, _P, _P, _P, _P, C.c_size_t, _P, _P, _P, _P, _P,
+                                         _P, _I64, _I64, _P, _P]),
     "fbp_gather_i32": (C.c_int, [_P, _I64, _P, _P, _P, _P]),
     "fbp_compact_scratch_bytes": (C.c_size_t, [_I64]),
     "fbp_compact_flags": (C.c_int, [_P, _I64, _P, _P, _P, C.c_size_t, _P]),
@@ -98,6 +99,7 @@ _SIG = {
     "fbp_forward_pairs": (C.c_int, [C.POINTER(Net), _P, C.POINTER(Pairs), _P, _I32, _P]),
     "fbp_forward_pairs_tc": (C.c_int, [C.POINTER(Net), _P, C.POINTER(Pairs), _P, _P, _I32, _P]),
     "fbp_pou_forward": (C.c_int, [_I32, _I32, _I64, _I32, _P, _P, _P, _P, _P, _I64, _I64, _P, _P]),
+    "fbp_pou_solution": (C.c_int, [_I32, _I32, C.POINTER(Problem), _I64, _I32, _P, _P, _P, _P, _P, _I64, _P, _P]),
     "fbp_pou_backward": (C.c_int, [_I32, _I32, _I64, _I32, _P, _P, _P, _I64, _P]),
     "fbp_pou_loss": (C.c_int, [_I32, _I32, C.POINTER(Problem), _I64, _I32, _P, _P, _P, _P, _P, _P, _P, _I64, _I64,
                                _P, _I32, _P, _P]),

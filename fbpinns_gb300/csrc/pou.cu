@@ -424,6 +424,56 @@ __global__ void __launch_bounds__(POU_T) pou_forward_kernel(int64_t n, int npou,
     }
 }
 
+// The constrained solution at the points: POU sum of the pairs' values, then
+// the built-in ansatz A + B u.  One thread per point; only the value and the
+// window of each record are read (one 32-byte sector), eight pairs at a time.
+template <int XD, int D2>
+__global__ void __launch_bounds__(POU_T) pou_solution_kernel(fbp_problem P, int64_t n, int npou,
+                                                              const float* __restrict__ x,
+                                                              const int32_t* __restrict__ pt_off,
+                                                              const int32_t* __restrict__ p_take,
+                                                              const float* __restrict__ pair_out,
+                                                              float* __restrict__ out, int64_t s_cap,
+                                                              int32_t* status) {
+    constexpr int J = JL<XD, D2>::J, RS = rec_stride(J), PU = 8;
+    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
+        const int e0 = (int)min((int64_t)pt_off[p], s_cap), e1 = (int)min((int64_t)pt_off[p + 1], s_cap);
+        float xp[XD];
+#pragma unroll
+        for (int d = 0; d < XD; ++d) xp[d] = x[p * XD + d];
+        float u = 0.f, N = 0.f, W = 0.f;
+        int cur = -1;
+        for (int eb = e0; eb < e1; eb += PU) {
+            int r[PU];
+            float a[PU], b[PU];
+#pragma unroll
+            for (int q = 0; q < PU; ++q) {
+                const bool in = eb + q < e1;
+                r[q] = in ? p_take[eb + q] : -2;
+                a[q] = in ? pair_out[(size_t)(eb + q) * RS] : 0.f;
+                b[q] = in ? pair_out[(size_t)(eb + q) * RS + J] : 0.f;
+            }
+#pragma unroll
+            for (int q = 0; q < PU; ++q) {
+                if (eb + q >= e1) break;
+                if (r[q] != cur) {
+                    if (cur >= 0) u += N * (1.0f / W);
+                    if (r[q] < cur) atomicOr(status, FBP_STATUS_LEVEL_ORDER);
+                    cur = r[q];
+                    N = W = 0.f;
+                }
+                N += a[q];
+                W += b[q];
+            }
+        }
+        if (cur >= 0) u += N * (1.0f / W);
+        u *= 1.0f / (float)npou;
+        float A[J], B[J];
+        ansatz<XD, D2>(P, xp, A, B);
+        out[p] = A[0] + B[0] * u;
+    }
+}
+
 template <int XD, int D2>
 __global__ void __launch_bounds__(POU_T) pou_backward_kernel(int64_t n, int npou, const int32_t* __restrict__ np_off,
                                                               const float* __restrict__ Ubar,
@@ -819,6 +869,28 @@ extern "C" int fbp_pou_forward(int32_t xd, int32_t d2mask, int64_t n, int32_t np
     FBP_XD_D2_CASES(X)
 #undef X
     set_error("fbp_pou_forward: unsupported xd=%d d2mask=%d", xd, d2mask);
+    return FBP_ERR_UNSUPPORTED;
+}
+
+extern "C" int fbp_pou_solution(int32_t xd, int32_t d2mask, const fbp_problem* prob, int64_t n, int32_t npou,
+                                const float* x, const int32_t* pt_off, const int32_t* p_take, const float* pair_out,
+                                float* out, int64_t s_cap, int32_t* status, void* stream) {
+    FBP_REQUIRE(prob && pt_off && out && status && npou > 0 && (x || n == 0), FBP_ERR_INVALID,
+                "fbp_pou_solution: bad args");
+    FBP_REQUIRE(prob->ng == 0 || prob->gauss, FBP_ERR_INVALID, "fbp_pou_solution: null gaussians");
+    if (n == 0) return FBP_OK;
+    cudaStream_t st = as_stream(stream);
+    // 64 threads per CTA: the 10^4 points of a test grid reach every SM
+    const int g = (int)std::min<int64_t>((n + 63) / 64, (int64_t)sm_count() * 32);
+#define X(a, b)                                                                                                     \
+    if (xd == a && d2mask == b) {                                                                                   \
+        pou_solution_kernel<a, b><<<g, 64, 0, st>>>(*prob, n, npou, x, pt_off, p_take, pair_out, out, s_cap, status); \
+        FBP_LAUNCH_CHECK();                                                                                         \
+        return FBP_OK;                                                                                              \
+    }
+    FBP_XD_D2_CASES(X)
+#undef X
+    set_error("fbp_pou_solution: unsupported xd=%d d2mask=%d", xd, d2mask);
     return FBP_ERR_UNSUPPORTED;
 }
 

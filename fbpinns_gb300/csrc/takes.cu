@@ -59,7 +59,8 @@ constexpr int COUNT_CTAS = 2, COUNT_T = 512;
 constexpr int LIST_CHUNK = 256;
 
 // SHIST: model_count through the CTA's table in shared memory (m words).
-// sums (nullable; !SHIST, CTAs of LIST_CHUNK threads): per chunk its pairs and slots.
+// sums (nullable): per chunk its pairs and slots; with SHIST added by the warps
+// (sums zeroed before), else written by CTAs of LIST_CHUNK threads.
 template <int XD, bool SHIST>
 __global__ void inside_count_kernel(const float* __restrict__ x, int64_t n, fbp_boxes b,
                                     int32_t* __restrict__ pt_count, int32_t* __restrict__ pt_nlvl,
@@ -101,10 +102,16 @@ __global__ void inside_count_kernel(const float* __restrict__ x, int64_t n, fbp_
             if (pt_hit) pt_hit[p] = hit;
             if (pt_cand) pt_cand[p] = e1 - e0 <= 64 ? e0 : -1;
         }
-        if constexpr (!SHIST) {
-            if (sums) {
+        if (sums) {
+            const int ws = __reduce_add_sync(0xffffffffu, cnt), wu = __reduce_add_sync(0xffffffffu, __popcll(lvl));
+            if constexpr (SHIST) {
+                int2* t = &sums[(p0 + threadIdx.x) / LIST_CHUNK];
+                if ((threadIdx.x & 31) == 0 && ws) {
+                    atomicAdd(&t->x, ws);
+                    atomicAdd(&t->y, wu);
+                }
+            } else {
                 __shared__ int2 warp_sums[LIST_CHUNK / 32];
-                const int ws = __reduce_add_sync(0xffffffffu, cnt), wu = __reduce_add_sync(0xffffffffu, __popcll(lvl));
                 if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = make_int2(ws, wu);
                 __syncthreads();
                 if (threadIdx.x == 0) {
@@ -744,7 +751,7 @@ extern "C" int fbp_scan_i32(const int32_t* in, int32_t* out, int64_t n, void* sc
     return scan_launch(in, out, n, (int32_t*)scratch, as_stream(stream));
 }
 
-// sums: see inside_count_kernel (excludes model_count in shared memory)
+// sums: see inside_count_kernel
 static int launch_count(const float* x, int64_t n, const fbp_boxes* boxes, int32_t* pt_count, int32_t* pt_nlvl,
                         uint64_t* pt_lvl, int32_t* model_count, uint64_t* pt_hit, int32_t* pt_cand, int2* sums,
                         cudaStream_t st) {
@@ -756,7 +763,7 @@ static int launch_count(const float* x, int64_t n, const fbp_boxes* boxes, int32
     if (boxes->xd == D) {                                                                                            \
         if (shist)                                                                                                   \
             inside_count_kernel<D, true><<<g, t, shm, st>>>(x, n, *boxes, pt_count, pt_nlvl, pt_lvl, model_count,    \
-                                                            pt_hit, pt_cand, nullptr);                               \
+                                                            pt_hit, pt_cand, sums);                                  \
         else                                                                                                         \
             inside_count_kernel<D, false><<<g, t, 0, st>>>(x, n, *boxes, pt_count, pt_nlvl, pt_lvl, model_count,     \
                                                            pt_hit, pt_cand, sums);                                   \
@@ -821,32 +828,49 @@ extern "C" size_t fbp_inside_lists_scratch_bytes(int64_t n) {
     return (size_t)((n + LIST_CHUNK - 1) / LIST_CHUNK + 1) * sizeof(int2);
 }
 
-extern "C" int fbp_inside_lists(const float* x, int64_t n, const fbp_boxes* boxes, int32_t* pt_count,
-                                uint64_t* pt_lvl, uint64_t* pt_hit, int32_t* pt_cand, int32_t* pt_off,
-                                int32_t* np_off, int32_t* n_take, int32_t* m_take, int32_t* p_take, int32_t* np_take,
-                                int64_t s_cap, int64_t u_cap, int32_t* status, void* scratch, size_t scratch_bytes,
-                                void* stream) {
+static int check_chunks(int64_t n, const void* sums, size_t sums_bytes) {
+    FBP_REQUIRE(n >= 0 && n < (int64_t)1 << 31, FBP_ERR_INVALID, "inside lists: n=%lld", (long long)n);
+    FBP_REQUIRE(sums && ((uintptr_t)sums & 7) == 0 && sums_bytes >= fbp_inside_lists_scratch_bytes(n),
+                FBP_ERR_CAPACITY, "inside lists: chunk sums too small");
+    return FBP_OK;
+}
+
+extern "C" int fbp_inside_count_chunks(const float* x, int64_t n, const fbp_boxes* boxes, int32_t* pt_count,
+                                       uint64_t* pt_lvl, int32_t* model_count, uint64_t* pt_hit, int32_t* pt_cand,
+                                       void* sums, size_t sums_bytes, void* stream) {
     int rc = check_boxes(boxes);
     if (rc) return rc;
-    FBP_REQUIRE(pt_off && np_off && status, FBP_ERR_INVALID, "fbp_inside_lists: null pointer");
-    FBP_REQUIRE(n == 0 || (x && pt_count && pt_lvl), FBP_ERR_INVALID, "fbp_inside_lists: null pointer");
-    FBP_REQUIRE(!pt_hit == !pt_cand, FBP_ERR_INVALID, "fbp_inside_lists: pt_hit and pt_cand go together");
-    FBP_REQUIRE((n_take && m_take && p_take) || s_cap == 0, FBP_ERR_INVALID, "fbp_inside_lists: null take");
-    FBP_REQUIRE(np_take || u_cap == 0, FBP_ERR_INVALID, "fbp_inside_lists: null np_take");
-    FBP_REQUIRE(n >= 0 && n < (int64_t)1 << 31, FBP_ERR_INVALID, "fbp_inside_lists: n=%lld", (long long)n);
-    FBP_REQUIRE(scratch && ((uintptr_t)scratch & 7) == 0 && scratch_bytes >= fbp_inside_lists_scratch_bytes(n),
-                FBP_ERR_CAPACITY, "fbp_inside_lists: scratch too small");
+    rc = check_chunks(n, sums, sums_bytes);
+    if (rc) return rc;
+    FBP_REQUIRE(n == 0 || (x && pt_count && pt_lvl), FBP_ERR_INVALID, "fbp_inside_count_chunks: null pointer");
+    FBP_REQUIRE(!pt_hit == !pt_cand, FBP_ERR_INVALID, "fbp_inside_count_chunks: pt_hit and pt_cand go together");
+    if (n == 0) return FBP_OK;
+    return launch_count(x, n, boxes, pt_count, nullptr, pt_lvl, model_count, pt_hit, pt_cand, static_cast<int2*>(sums),
+                        as_stream(stream));
+}
+
+extern "C" int fbp_inside_fill_chunks(const float* x, int64_t n, const fbp_boxes* boxes, const int32_t* pt_count,
+                                      const uint64_t* pt_lvl, const uint64_t* pt_hit, const int32_t* pt_cand,
+                                      const void* sums, size_t sums_bytes, int32_t* pt_off, int32_t* np_off,
+                                      int32_t* n_take, int32_t* m_take, int32_t* p_take, int32_t* np_take,
+                                      int64_t s_cap, int64_t u_cap, int32_t* status, void* stream) {
+    int rc = check_boxes(boxes);
+    if (rc) return rc;
+    rc = check_chunks(n, sums, sums_bytes);
+    if (rc) return rc;
+    FBP_REQUIRE(pt_off && np_off && status, FBP_ERR_INVALID, "fbp_inside_fill_chunks: null pointer");
+    FBP_REQUIRE(n == 0 || (x && pt_count && pt_lvl), FBP_ERR_INVALID, "fbp_inside_fill_chunks: null pointer");
+    FBP_REQUIRE(!pt_hit == !pt_cand, FBP_ERR_INVALID, "fbp_inside_fill_chunks: pt_hit and pt_cand go together");
+    FBP_REQUIRE((n_take && m_take && p_take) || s_cap == 0, FBP_ERR_INVALID, "fbp_inside_fill_chunks: null take");
+    FBP_REQUIRE(np_take || u_cap == 0, FBP_ERR_INVALID, "fbp_inside_fill_chunks: null np_take");
     cudaStream_t st = as_stream(stream);
     if (n == 0) {
         FBP_CUDA_CHECK(cudaMemsetAsync(pt_off, 0, sizeof(int32_t), st));
         FBP_CUDA_CHECK(cudaMemsetAsync(np_off, 0, sizeof(int32_t), st));
         return FBP_OK;
     }
-    int2* sums = static_cast<int2*>(scratch);
-    rc = launch_count(x, n, boxes, pt_count, nullptr, pt_lvl, nullptr, pt_hit, pt_cand, sums, st);
-    if (rc) return rc;
-    return launch_fill(x, n, boxes, pt_off, np_off, pt_count, sums, pt_lvl, pt_hit, pt_cand, n_take, m_take, p_take,
-                       np_take, s_cap, u_cap, status, st);
+    return launch_fill(x, n, boxes, pt_off, np_off, pt_count, static_cast<const int2*>(sums), pt_lvl, pt_hit, pt_cand,
+                       n_take, m_take, p_take, np_take, s_cap, u_cap, status, st);
 }
 
 extern "C" int fbp_gather_i32(const int32_t* in, int64_t n, const int32_t* count_dev, const int32_t* inv,

@@ -67,12 +67,6 @@ def grid_of(static, device="cuda"):
     return g
 
 
-def _scan(lib, src, dst, n, stream):
-    scratch = torch.empty(int(lib.fbp_scan_scratch_bytes(n)) // 4 + 1, dtype=torch.int32, device=src.device)
-    _lib.check(lib.fbp_scan_i32(_lib.ptr(src), _lib.ptr(dst), n, _lib.ptr(scratch), scratch.numel() * 4, stream),
-               "fbp_scan_i32")
-
-
 class PointTakes:
     """Interaction lists of one point set, built by count -> scan -> fill.
 
@@ -85,22 +79,22 @@ class PointTakes:
     def __init__(self, grid, n, s_cap=None, u_cap=None):
         self.grid, self.n = grid, int(n)
         dev = grid.device
-        self.pt_count = torch.zeros(self.n, dtype=torch.int32, device=dev)
-        self.pt_nlvl = torch.zeros(self.n, dtype=torch.int32, device=dev)
-        self.pt_lvl = torch.zeros(self.n, dtype=torch.int64, device=dev)
+        # (every one written by the passes before it is read)
+        self.pt_count = torch.empty(self.n, dtype=torch.int32, device=dev)
+        self.pt_lvl = torch.empty(self.n, dtype=torch.int64, device=dev)
         # hits of the count pass as candidate-list masks, read by the fill pass
-        self.pt_hit = torch.zeros(self.n, dtype=torch.int64, device=dev)
-        self.pt_cand = torch.zeros(self.n, dtype=torch.int32, device=dev)
+        self.pt_hit = torch.empty(self.n, dtype=torch.int64, device=dev)
+        self.pt_cand = torch.empty(self.n, dtype=torch.int32, device=dev)
         self.use_hit_masks = True
-        self.pt_off = torch.zeros(self.n + 1, dtype=torch.int32, device=dev)
-        self.np_off = torch.zeros(self.n + 1, dtype=torch.int32, device=dev)
-        self.model_count = torch.zeros(grid.m, dtype=torch.int32, device=dev)
-        self.status = torch.zeros(1, dtype=torch.int32, device=dev)
-        lib = _lib.load()
-        self._scan_scratch = torch.empty(int(lib.fbp_scan_scratch_bytes(self.n)) // 4 + 1, dtype=torch.int32,
-                                         device=dev)
-        self._list_scratch = torch.empty(int(lib.fbp_inside_lists_scratch_bytes(self.n)) // 4, dtype=torch.int32,
-                                         device=dev)
+        self.pt_off = torch.empty(self.n + 1, dtype=torch.int32, device=dev)
+        self.np_off = torch.empty(self.n + 1, dtype=torch.int32, device=dev)
+        # points per box, pairs and slots per chunk of points, and the status word
+        # (read back together where the sizes are)
+        pad = (grid.m + 3) // 4 * 4
+        nsum = int(_lib.load().fbp_inside_lists_scratch_bytes(self.n)) // 4
+        self._counts = torch.zeros(pad + nsum + 1, dtype=torch.int32, device=dev)
+        self.model_count, self._sums = self._counts[:grid.m], self._counts[pad:pad + nsum]
+        self.status = self._counts[pad + nsum:]
         self.s_cap = s_cap
         self.u_cap = u_cap
         self._alloc(s_cap or 0, u_cap or 0)
@@ -128,45 +122,32 @@ class PointTakes:
         assert x.is_cuda and x.dtype == torch.float32 and x.shape == (self.n, self.grid.xd)
         x = x.contiguous()
         # the status word is sticky: cleared only by reset_status()
-        if self.s_cap is not None and not count_models:  # nothing to read back: two launches
-            _lib.check(lib.fbp_inside_lists(_lib.ptr(x), self.n, C.byref(b), _lib.ptr(self.pt_count),
-                                            _lib.ptr(self.pt_lvl), _lib.ptr(self.pt_hit) if self.use_hit_masks else None,
-                                            _lib.ptr(self.pt_cand) if self.use_hit_masks else None,
-                                            _lib.ptr(self.pt_off), _lib.ptr(self.np_off), _lib.ptr(self.n_take),
-                                            _lib.ptr(self.m_take), _lib.ptr(self.p_take), _lib.ptr(self.np_take),
-                                            self.n_take.numel(), self.np_take.numel(), _lib.ptr(self.status),
-                                            _lib.ptr(self._list_scratch), self._list_scratch.numel() * 4, st),
-                       "fbp_inside_lists")
-            self._sizes = None
-            return None
         if count_models:
-            self.model_count.zero_()
-        _lib.check(lib.fbp_inside_count(_lib.ptr(x), self.n, C.byref(b), _lib.ptr(self.pt_count),
-                                        _lib.ptr(self.pt_nlvl), _lib.ptr(self.pt_lvl),
-                                        _lib.ptr(self.model_count) if count_models else None,
-                                        _lib.ptr(self.pt_hit), _lib.ptr(self.pt_cand), st),
-                   "fbp_inside_count")
-        sb = self._scan_scratch.numel() * 4
-        _lib.check(lib.fbp_scan_i32(_lib.ptr(self.pt_count), _lib.ptr(self.pt_off), self.n,
-                                    _lib.ptr(self._scan_scratch), sb, st), "fbp_scan_i32")
-        _lib.check(lib.fbp_scan_i32(_lib.ptr(self.pt_nlvl), _lib.ptr(self.np_off), self.n,
-                                    _lib.ptr(self._scan_scratch), sb, st), "fbp_scan_i32")
+            self._counts[:-1].zero_()
+        hit, cand = (_lib.ptr(self.pt_hit), _lib.ptr(self.pt_cand)) if self.use_hit_masks else (None, None)
+        sums, nb = _lib.ptr(self._sums), self._sums.numel() * 4
+        _lib.check(lib.fbp_inside_count_chunks(_lib.ptr(x), self.n, C.byref(b), _lib.ptr(self.pt_count),
+                                               _lib.ptr(self.pt_lvl), _lib.ptr(self.model_count) if count_models else None,
+                                               hit, cand, sums, nb, st), "fbp_inside_count_chunks")
         sizes = None
         if self.s_cap is None:
-            s = int(self.pt_off[self.n].item())
-            u = int(self.np_off[self.n].item())
+            # one read of the counts (model_counts: with the box counts)
+            if stream is not None:
+                torch.cuda.current_stream().wait_stream(stream)
+            h = self._counts.cpu().numpy() if count_models else None
+            tot = (h[-1 - nb // 4:-1] if count_models else self._sums.cpu().numpy()).reshape(-1, 2)[:-1]
+            self.model_counts = h[:self.grid.m] if count_models else None
+            s, u = int(tot[:, 0].sum(dtype=np.int64)), int(tot[:, 1].sum(dtype=np.int64))
             self._alloc(s, u)
             s_cap, u_cap = s, u
             sizes = (s, u)
         else:
             s_cap, u_cap = self.n_take.numel(), self.np_take.numel()
-        _lib.check(lib.fbp_inside_fill(_lib.ptr(x), self.n, C.byref(b), _lib.ptr(self.pt_off), _lib.ptr(self.np_off),
-                                       _lib.ptr(self.pt_lvl),
-                                       _lib.ptr(self.pt_hit) if self.use_hit_masks else None,
-                                       _lib.ptr(self.pt_cand) if self.use_hit_masks else None,
-                                       _lib.ptr(self.n_take), _lib.ptr(self.m_take),
-                                       _lib.ptr(self.p_take), _lib.ptr(self.np_take), s_cap, u_cap,
-                                       _lib.ptr(self.status), st), "fbp_inside_fill")
+        _lib.check(lib.fbp_inside_fill_chunks(_lib.ptr(x), self.n, C.byref(b), _lib.ptr(self.pt_count),
+                                              _lib.ptr(self.pt_lvl), hit, cand, sums, nb, _lib.ptr(self.pt_off),
+                                              _lib.ptr(self.np_off), _lib.ptr(self.n_take), _lib.ptr(self.m_take),
+                                              _lib.ptr(self.p_take), _lib.ptr(self.np_take), s_cap, u_cap,
+                                              _lib.ptr(self.status), st), "fbp_inside_fill_chunks")
         self._sizes = sizes
         return sizes
 
@@ -249,23 +230,26 @@ def get_inputs(x_batch, active, all_params, decomposition=None):
     g = grid_of(static)
     m = g.m
     active = np.array(active).copy()
-    assert np.isin(active, np.array([0, 1, 2])).all()
+    assert ((active == 0) | (active == 1) | (active == 2)).all()
     assert active.shape == (m,)
     x = _x_dev(x_batch, g.device)
     t = PointTakes(g, x.shape[0])
     s, u = t.build(x)
-    t.check_status()
-    training = (t.model_count > 0).cpu().numpy()
+    training = t.model_counts > 0
     active[active == 0] = 1
     active = active * training.astype(active.dtype)
     ims_ = np.arange(m)
     active_ims, fixed_ims = ims_[active == 1], ims_[active == 2]
     all_ims = np.concatenate([active_ims, fixed_ims])
-    inv = np.zeros(m, dtype=np.int32)
-    inv[all_ims] = np.arange(len(all_ims), dtype=np.int32)
-    m_take = gather_i32(t.m_take[:s].contiguous(), torch.as_tensor(inv, device=g.device))
-    takes = (m_take, t.n_take[:s].clone(), t.p_take[:s].clone(), t.np_take[:u].clone(), g.npou)
-    return takes, torch.as_tensor(all_ims, dtype=torch.int32, device=g.device), (active, active_ims, fixed_ims)
+    # positions in all_ims, and all_ims itself, in one copy to the device
+    up = np.zeros(m + len(all_ims), dtype=np.int32)
+    up[all_ims] = np.arange(len(all_ims), dtype=np.int32)
+    up[m:] = all_ims
+    t.check_status()  # (the host's part above ran while the lists were filled)
+    up = torch.as_tensor(up).to(g.device)
+    m_take = gather_i32(t.m_take[:s], up[:m])
+    takes = (m_take, t.n_take[:s], t.p_take[:s], t.np_take[:u], g.npou)
+    return takes, up[m:], (active, active_ims, fixed_ims)
 
 
 def split_takes(takes, offsets, n_points):

@@ -281,14 +281,19 @@ int fbp_inside_fill(const float* x, int64_t n, const fbp_boxes* boxes,
                     int64_t s_cap, int64_t u_cap, int32_t* status, void* stream);
 
 /* fbp_inside_count, the two exclusive scans and fbp_inside_fill in two
- * launches, with the same results (pt_count and pt_lvl are working arrays,
- * pt_hit / pt_cand optional ones); scratch 8-byte aligned. */
+ * launches, with the same results.  sums holds (pairs, slots) as two int32 per
+ * chunk of 256 points (8-byte aligned, fbp_inside_lists_scratch_bytes), so
+ * their totals are the list sizes; with model_count (nullable, added to) sums
+ * must be zero before the count.  pt_hit / pt_cand as above, optional. */
 size_t fbp_inside_lists_scratch_bytes(int64_t n);
-int fbp_inside_lists(const float* x, int64_t n, const fbp_boxes* boxes, int32_t* pt_count,
-                     uint64_t* pt_lvl, uint64_t* pt_hit, int32_t* pt_cand,
-                     int32_t* pt_off, int32_t* np_off, int32_t* n_take, int32_t* m_take,
-                     int32_t* p_take, int32_t* np_take, int64_t s_cap, int64_t u_cap,
-                     int32_t* status, void* scratch, size_t scratch_bytes, void* stream);
+int fbp_inside_count_chunks(const float* x, int64_t n, const fbp_boxes* boxes, int32_t* pt_count,
+                            uint64_t* pt_lvl, int32_t* model_count, uint64_t* pt_hit, int32_t* pt_cand,
+                            void* sums, size_t sums_bytes, void* stream);
+int fbp_inside_fill_chunks(const float* x, int64_t n, const fbp_boxes* boxes, const int32_t* pt_count,
+                           const uint64_t* pt_lvl, const uint64_t* pt_hit, const int32_t* pt_cand,
+                           const void* sums, size_t sums_bytes, int32_t* pt_off, int32_t* np_off,
+                           int32_t* n_take, int32_t* m_take, int32_t* p_take, int32_t* np_take,
+                           int64_t s_cap, int64_t u_cap, int32_t* status, void* stream);
 
 /* out[i] = inv[in[i]] for i < *count_dev (or < n when count_dev is NULL):
  * the re-index of m_take to positions in all_ims = [active; fixed]
@@ -384,6 +389,13 @@ int fbp_pou_loss(int32_t xd, int32_t d2mask, const fbp_problem* prob,
                  const float* pair_out, float* slot_out, float* U_out,
                  int64_t s_cap, int64_t u_cap,
                  double* loss_part, int32_t n_part, int32_t* status, void* stream);
+
+/* The constrained solution out (n,) = A(x) + B(x) u(x) of a built-in problem's
+ * ansatz at the points: the values only of fbp_pou_forward followed by the
+ * problem's constraining_fn. */
+int fbp_pou_solution(int32_t xd, int32_t d2mask, const fbp_problem* prob, int64_t n, int32_t npou,
+                     const float* x, const int32_t* pt_off, const int32_t* p_take,
+                     const float* pair_out, float* out, int64_t s_cap, int32_t* status, void* stream);
 
 /* Deterministic sum of the n_part FP64 partials, times scale. */
 int fbp_loss_finalize(const double* loss_part, int32_t n_part, double scale,
