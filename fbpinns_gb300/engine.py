@@ -430,11 +430,8 @@ class FBPINNEngine:
         n.window, n.wmins, n.wmaxs = g.window, _lib.ptr(g.wmins), _lib.ptr(g.wmaxs)
         return n
 
-    def set_problem(self, spec):
-        """Fused residual of a built-in problem (problems.Problem.fused_spec)."""
-        if spec is None:
-            self._problem = None
-            return
+    def _problem_struct(self, spec):
+        """(fbp_problem of a fused_spec, its Gaussians on the device or None)."""
         pr = _lib.Problem()
         pr.kind = int(spec["kind"])
         pr.n_int = int(spec.get("n_int", 0))
@@ -442,22 +439,29 @@ class FBPINNEngine:
             pr.p[i] = float(v)
         gauss = spec.get("gauss")
         if gauss is not None:
-            self._gauss = torch.as_tensor(gauss, dtype=torch.float32).to(self.device).contiguous()
-            pr.gauss, pr.ng = _lib.ptr(self._gauss), int(self._gauss.shape[0])
+            gauss = torch.as_tensor(gauss, dtype=torch.float32).to(self.device).contiguous()
+            pr.gauss, pr.ng = _lib.ptr(gauss), int(gauss.shape[0])
         else:
-            self._gauss = None
             pr.gauss, pr.ng = None, 0
-        self._problem = pr
+        return pr, gauss
+
+    def set_problem(self, spec):
+        """Fused residual of a built-in problem (problems.Problem.fused_spec)."""
+        if spec is None:
+            self._problem = None
+            return
+        self._problem, self._gauss = self._problem_struct(spec)
 
     # -- kernels -------------------------------------------------------------
     def points(self, x, select=None, caps=None, chunk=None, scheduled=False):
         return PointSet(self, x, select=select, caps=caps, chunk=chunk, scheduled=scheduled)
 
-    def forward_pairs(self, ps, theta=None, stream=None, z2=True):
+    def forward_pairs(self, ps, theta=None, stream=None, z2=True, d2mask=None):
         """Per-pair jets into ps.pair_out; z2: also store the layer-2 z-jets
-        for an adjoint that follows (False for jets that are not differentiated)."""
+        for an adjoint that follows (False for jets that are not differentiated);
+        d2mask: another compiled jet mask of at most the engine's jet size."""
         lib = _lib.load()
-        net = self.net_struct(theta)
+        net = self.net_struct(theta, d2mask)
         pr = ps.pairs_struct(False, z2)
         grid = ps.forward_items_cap if self.fwd_schedule() == "per_item" else \
             (self.launch_grid if self.forward_grid is None else self.forward_grid)
@@ -468,6 +472,22 @@ class FBPINNEngine:
             return
         _lib.check(lib.fbp_forward_pairs(C.byref(net), _lib.ptr(ps.x), C.byref(pr), _lib.ptr(ps.pair_out),
                                          grid, _lib.stream_ptr(stream)), "fbp_forward_pairs")
+
+    def solution(self, ps, spec):
+        """The constrained solution (n, 1) at ps's points, spec: fused_spec of the
+        problem whose ansatz it takes.  The jets carry no second derivatives
+        where such a kernel is compiled (in the form that the engine uses)."""
+        lib = _lib.load()
+        t = ps.takes
+        pr, _gauss = self._problem_struct(spec)
+        has = lib.fbp_has_tc_shape if self.tensor_cores else lib.fbp_has_shape
+        mask = 0 if has(self.xd, self.h1, self.h2, 0, self.act) else self.d2mask
+        self.forward_pairs(ps, z2=False, d2mask=mask)
+        out = torch.empty((ps.n, 1), dtype=torch.float32, device=self.device)
+        _lib.check(lib.fbp_pou_solution(self.xd, mask, C.byref(pr), ps.n, self.npou, _lib.ptr(ps.x), _lib.ptr(t.pt_off),
+                                        _lib.ptr(t.p_take), _lib.ptr(ps.pair_out), _lib.ptr(out), ps.pair_out.shape[0],
+                                        _lib.ptr(t.status), _lib.stream_ptr()), "fbp_pou_solution")
+        return out
 
     def pou_forward(self, ps, stream=None):
         lib = _lib.load()

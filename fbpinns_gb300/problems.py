@@ -380,3 +380,28 @@ class Helmholtz2D(Problem):
         p = all_params["static"]["problem"]
         return {"kind": _lib.PROBLEM_HELMHOLTZ2D, "p": [p["sd"], p["k"]], "n_int": 0, "gauss": p["source"],
                 "d2_group": 3}  # the residual needs only u_xx + u_yy
+
+
+# the constraining functions that the kernels evaluate, by the function itself:
+# a subclass that keeps one is in, one that replaces it is not
+_ANSATZ = {k.constraining_fn: k for k in (HarmonicOscillator1DHardBC, BurgersEquation2D, WaveEquationConstantVelocity3D,
+                                          Poisson2D, Helmholtz2D)}
+
+
+def ansatz_spec(problem, all_params):
+    """fused_spec whose ansatz is problem.constraining_fn, or None where the
+    kernels have none (or its parameters are on a GPU, where reading them
+    would wait for it)."""
+    k = _ANSATZ.get(problem.constraining_fn)
+    if k is None:
+        return None
+    p = all_params["static"]["problem"]
+    if any(torch.is_tensor(v) and v.is_cuda for v in p.values()):
+        return None
+    try:
+        spec = k.fused_spec(all_params)
+    except (KeyError, TypeError, ValueError, AttributeError):  # parameters that only the residual needs
+        return None
+    if spec["kind"] != _lib.PROBLEM_WAVE_C:
+        spec["gauss"] = None  # the residual's
+    return spec

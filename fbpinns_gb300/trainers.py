@@ -28,6 +28,7 @@ from .engine import FBPINNEngine, FBPINNJet, constrained_jets, d2mask_of, jet_in
 from .networks import (fcn_param_count, pack_layers, unpack_layers, engine_network,  # noqa: F401
                        NETWORK_ACTIVATIONS, FCN, SIREN, AdaptiveFCN, AdaptiveSIREN, FourierFCN)
 from .optim import adam_update
+from .problems import ansatz_spec
 from .takes import get_inputs, split_takes, inside_models, grid_of  # noqa: F401  (re-exported API)
 
 logger = logging.getLogger("fbpinns_gb300")
@@ -631,6 +632,9 @@ class FBPINNTrainer:
             setattr(eng, key, (x, ps))
         ps = getattr(eng, key)[1]
         with torch.no_grad():
+            spec = ansatz_spec(problem, all_params)
+            if spec is not None:
+                return eng.solution(ps, spec)
             eng.forward_pairs(ps, z2=False)
             U = eng.pou_forward(ps)
             return problem.constraining_fn(all_params, x, U[:, 0:1])

@@ -926,3 +926,42 @@ def test_fused_step_tail_matches_separate_launches(cuda, n):
     assert out[0][0] == out[1][0]
     for a, b in zip(out[0][1], out[1][1]):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("name", ["ho", "burgers", "poisson", "helmholtz", "wave", "wave_gaussian"])
+@pytest.mark.parametrize("n", [1, 700])
+def test_fused_solution_matches_constraining_fn(cuda, name, n, monkeypatch):
+    """predict by the kernel's ansatz (values only) against the jets' values
+    through the problem's constraining_fn in torch; a subclass with its own
+    constraining_fn takes the torch route.  Both sum the same FP32 products in
+    another order: 1e-5 of the largest value."""
+    from fbpinns_gb300.trainers import FBPINNTrainer
+    src = np.array([[0.1, -0.2, 0.3, 1.0], [0.4, 0.3, 0.2, -0.7]])
+    pcls, pkw, recipe, ls, d2 = {
+        "ho": (PR.HarmonicOscillator1DHardBC, {}, "ho", [1, 32, 32, 1], 1),
+        "burgers": (PR.BurgersEquation2D, {}, "burgers", [2, 16, 16, 1], 1),
+        "poisson": (PR.Poisson2D, {}, "multilevel", [2, 16, 16, 1], 3),
+        "helmholtz": (PR.Helmholtz2D, {}, "multilevel", [2, 8, 8, 1], 3),
+        "wave": (PR.WaveEquationConstantVelocity3D, dict(source=src), "wave", [3, 32, 32, 1], 7),
+        "wave_gaussian": (PR.WaveEquationGaussianVelocity3D, dict(source=src), "wave", [3, 32, 32, 1], 7)}[name]
+    static = decomposition(recipe)
+    eng = _engine(static, random_layers(ls, static["m"], seed=3), d2)
+    ap = {"static": {"problem": pcls.init_params(**pkw)[0]}, "trainable": {}}
+    lo = torch.tensor([-1.0, -1.0, 0.0] if ls[0] == 3 else [-1.0, 0.0] if name == "burgers" else [0.0] * ls[0])
+    x = (lo + (1 - lo) * torch.rand((n, ls[0]), generator=torch.Generator().manual_seed(n))).cuda()
+    assert PR.ansatz_spec(pcls, ap) is not None
+    got = FBPINNTrainer.predict(eng, ap, pcls, x)
+
+    class Own(pcls):
+        @staticmethod
+        def constraining_fn(all_params, x_batch, u):
+            return 2 * pcls.constraining_fn(all_params, x_batch, u)
+
+    assert PR.ansatz_spec(Own, ap) is None
+    own = FBPINNTrainer.predict(eng, ap, Own, x)
+    monkeypatch.setattr(PR, "_ANSATZ", {})
+    ref = FBPINNTrainer.predict(eng, ap, pcls, x)
+    assert got.shape == ref.shape == (n, 1) and got.dtype == ref.dtype
+    scale = max(ref.abs().max().item(), 1.0)
+    assert (got - ref).abs().max().item() <= 1e-5 * scale
+    assert torch.allclose(own, 2 * ref, rtol=1e-6, atol=1e-6 * scale)
