@@ -210,10 +210,44 @@ __device__ __forceinline__ void ansatz(const fbp_problem& P, const float* xp, fl
     }
 }
 
+// The Helmholtz source sum_g amp exp(-|x - m|^2 / (2 s^2)): up to GAUSS_CAP
+// Gaussians staged in shared memory as (mx, my, s^2, amp) and 1 / s^2, so that
+// the quotient is a product and one correction (q - y s^2 is exact to the last
+// bit of y) instead of a division per point and Gaussian: POU + loss of 2.1e6
+// points, 64 Gaussians 472 -> 299 us.
+constexpr int GAUSS_CAP = 128;
+struct Gauss {
+    float4 g;
+    float inv;
+};
+
+template <int XD>
+__device__ __forceinline__ float gauss_source(const fbp_problem& P, const Gauss* __restrict__ gs, const float* xp) {
+    float f = 0.f;
+    if (P.ng <= GAUSS_CAP) {
+#pragma unroll 4
+        for (int g = 0; g < P.ng; ++g) {
+            const float4 v = gs[g].g;
+            const float inv = gs[g].inv, dx = xp[0] - v.x, dy = xp[XD - 1] - v.y;
+            const float q = -0.5f * fmaf(dy, dy, dx * dx);
+            float y = q * inv;
+            y = fmaf(fmaf(-y, v.z, q), inv, y);
+            f = fmaf(v.w, expf(y), f);
+        }
+    } else {
+        for (int g = 0; g < P.ng; ++g) {
+            const float mx = P.gauss[4 * g], my = P.gauss[4 * g + 1], s = P.gauss[4 * g + 2], amp = P.gauss[4 * g + 3];
+            const float dx = xp[0] - mx, dy = xp[XD - 1] - my;
+            f += amp * expf(-0.5f * (dx * dx + dy * dy) / (s * s));
+        }
+    }
+    return f;
+}
+
 // residual r(uc) and dr/duc
 template <int XD, int D2>
-__device__ __forceinline__ float residual(const fbp_problem& P, const float* xp, const float (&u)[JL<XD, D2>::J],
-                                          float (&dr)[JL<XD, D2>::J]) {
+__device__ __forceinline__ float residual(const fbp_problem& P, const Gauss* __restrict__ gs, const float* xp,
+                                          const float (&u)[JL<XD, D2>::J], float (&dr)[JL<XD, D2>::J]) {
     using L = JL<XD, D2>;
     constexpr int J = L::J;
 #pragma unroll
@@ -266,24 +300,14 @@ __device__ __forceinline__ float residual(const fbp_problem& P, const float* xp,
         case FBP_PROBLEM_HELMHOLTZ2D: {  // u_xx + u_yy + k^2 u + f
             if constexpr (XD == 2 && L::LAPI > 0 && L::G == 3) {
                 const float k = P.p[1];
-                float f = 0.f;
-                for (int g = 0; g < P.ng; ++g) {
-                    const float mx = P.gauss[4 * g], my = P.gauss[4 * g + 1], s = P.gauss[4 * g + 2], amp = P.gauss[4 * g + 3];
-                    const float dx = xp[0] - mx, dy = xp[1] - my;
-                    f += amp * expf(-0.5f * (dx * dx + dy * dy) / (s * s));
-                }
+                const float f = gauss_source<XD>(P, gs, xp);
                 r = u[L::LAPI] + k * k * u[0] + f;
                 dr[L::LAPI] = 1.f;
                 dr[0] = k * k;
             }
             if constexpr (XD == 2 && L::sidx(0) > 0 && L::sidx(1) > 0) {
                 const float k = P.p[1];
-                float f = 0.f;
-                for (int g = 0; g < P.ng; ++g) {
-                    const float mx = P.gauss[4 * g], my = P.gauss[4 * g + 1], s = P.gauss[4 * g + 2], amp = P.gauss[4 * g + 3];
-                    const float dx = xp[0] - mx, dy = xp[1] - my;
-                    f += amp * expf(-0.5f * (dx * dx + dy * dy) / (s * s));
-                }
+                const float f = gauss_source<XD>(P, gs, xp);
                 r = u[L::sidx(0)] + u[L::sidx(1)] + k * k * u[0] + f;
                 dr[L::sidx(0)] = 1.f;
                 dr[L::sidx(1)] = 1.f;
@@ -504,7 +528,8 @@ __device__ __forceinline__ double block_sum_double(double v, double* sh) {
 // Constraint, residual and seeds of one point from its unconstrained jets u:
 // returns r^2 and leaves the seed dL/dU (before the 1/npou of the POU sum) in ub.
 template <int XD, int D2>
-__device__ __forceinline__ float point_residual(const fbp_problem& P, float inv_n, const float* __restrict__ x,
+__device__ __forceinline__ float point_residual(const fbp_problem& P, const Gauss* __restrict__ gs, float inv_n,
+                                                const float* __restrict__ x,
                                                 int64_t p, const float (&u)[JL<XD, D2>::J],
                                                 float* __restrict__ U_out, float (&ub)[JL<XD, D2>::J]) {
     constexpr int J = JL<XD, D2>::J;
@@ -530,7 +555,7 @@ __device__ __forceinline__ float point_residual(const fbp_problem& P, float inv_
         for (int c = 0; c < J; ++c) U_out[p * J + c] = uc[c];
     }
     float dr[J];
-    const float r = residual<XD, D2>(P, xp, uc, dr);
+    const float r = residual<XD, D2>(P, gs, xp, uc, dr);
     // seeds: dL/duc = (2 r / n) dr/duc, then the ansatz adjoint
     const float g = 2.0f * r * inv_n;
     float ucb[J];
@@ -586,6 +611,15 @@ __global__ void __launch_bounds__(POU_WARPS * 32) pou_loss_kernel(fbp_problem P,
     constexpr int J = JL<XD, D2>::J, RS = rec_stride(J), NV = 2 * J, SLOTCAP = pou_slotcap(RS);
     __shared__ __align__(16) float table[POU_WARPS][SLOTCAP * RS];
     __shared__ double sh[POU_WARPS];
+    __shared__ Gauss gs[XD == 2 ? GAUSS_CAP : 1];  // the Helmholtz source
+    if (XD == 2 && P.kind == FBP_PROBLEM_HELMHOLTZ2D && P.ng <= GAUSS_CAP) {
+        for (int g = threadIdx.x; g < P.ng; g += blockDim.x) {
+            const float s2 = P.gauss[4 * g + 2] * P.gauss[4 * g + 2];
+            gs[g].g = make_float4(P.gauss[4 * g], P.gauss[4 * g + 1], s2, P.gauss[4 * g + 3]);
+            gs[g].inv = 1.0f / s2;
+        }
+        __syncthreads();
+    }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float* T = table[w];
     const float inv_npou = 1.0f / (float)npou;
@@ -710,7 +744,7 @@ __global__ void __launch_bounds__(POU_WARPS * 32) pou_loss_kernel(fbp_problem P,
             PointPOU<XD, D2>::run(p, npou, pt_off, p_take, pair_out, slot_out, u, s_cap, u_cap, status);
         }
         if (pv) {
-            const float r2 = point_residual<XD, D2>(P, inv_n, x, p, u, U_out, ub);
+            const float r2 = point_residual<XD, D2>(P, gs, inv_n, x, p, u, U_out, ub);
             if (!P.pt_keep || P.pt_keep[p]) {
                 acc += (double)r2;
             } else {  // a point outside every active subdomain: no loss, no seeds
@@ -758,6 +792,8 @@ __global__ void __launch_bounds__(POU_WARPS * 32) pou_loss_kernel(fbp_problem P,
     }
 }
 
+constexpr int TAIL_T = 128;  // threads per CTA: a few thousand parameters reach every SM
+
 __device__ __forceinline__ void loss_sum(const double* __restrict__ part, int np, double scale, double* loss,
                                          double* sh) {
     double a = 0.0;
@@ -771,19 +807,28 @@ __global__ void loss_finalize_kernel(const double* __restrict__ part, int np, do
     loss_sum(part, np, scale, loss, sh);
 }
 
-// Sum of the partials of items [a, b) for one parameter, in item order; eight
-// loads are issued together (a subdomain that holds every point has hundreds
-// of items, and one load at a time is a chain of memory latencies).
+// Sum of the partials of items [a, b) for one parameter, in item order; the
+// loads of sixteen items are issued together (a subdomain that holds every
+// point has hundreds of items, and fewer at a time are a chain of latencies).
 __device__ __forceinline__ float item_sum(const float* __restrict__ p, int a, int b, int P) {
     float s = 0.f;
-    for (int it = a; it < b; it += 8) {
-        float v[8];
+    const float* q = p + (size_t)a * P;
+    int left = b - a;
+    for (; left >= 16; left -= 16, q += 16 * (size_t)P) {
+        float v[16];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = it + u < b ? p[(size_t)(it + u) * P] : 0.f;
+        for (int u = 0; u < 16; ++u) v[u] = __ldcs(q + (size_t)u * P);
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-            if (it + u < b) s += v[u];
+        for (int u = 0; u < 16; ++u) s += v[u];
     }
+    for (; left >= 4; left -= 4, q += 4 * (size_t)P) {
+        float v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = __ldcs(q + (size_t)u * P);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s += v[u];
+    }
+    for (; left > 0; --left, q += P) s += *q;
     return s;
 }
 
@@ -797,14 +842,14 @@ __global__ void grad_reduce_kernel(const float* __restrict__ part, const int32_t
     }
 }
 
-// The end of a training step in one launch: the loss (CTA 0), each parameter's
+// The end of a training step in one launch: the loss (the last CTA), each parameter's
 // gradient from its items' partials, its Adam step, and the step count, which
 // the last CTA to finish increments (every CTA reads the count before it takes
 // its ticket; the ticket is left at zero).  Four launches otherwise
 // (loss_finalize, grad_reduce, adam and the count): a step of the 1D
 // oscillator (15 networks, 200 points) 37.6 -> 34.8 us, of Burgers (128
 // networks, 200^2 points) 79.4 -> 74.3 us.
-__global__ void __launch_bounds__(256) step_tail_kernel(const double* __restrict__ loss_part, int np, double scale,
+__global__ void __launch_bounds__(TAIL_T) step_tail_kernel(const double* __restrict__ loss_part, int np, double scale,
                                                         double* loss, const float* __restrict__ part,
                                                         const int32_t* __restrict__ item_start, int64_t m, int P,
                                                         float* __restrict__ grad, float* __restrict__ theta,
@@ -814,11 +859,13 @@ __global__ void __launch_bounds__(256) step_tail_kernel(const double* __restrict
                                                         int32_t* ticket) {
     __shared__ double sh[32];
     const int c = *(volatile const int32_t*)count_dev + 1;
-    if (blockIdx.x == 0) loss_sum(loss_part, np, scale, loss, sh);
+    const int nb = (int)gridDim.x - 1;  // the last CTA has the loss, the others the parameters
+    if ((int)blockIdx.x == nb) loss_sum(loss_part, np, scale, loss, sh);
     const float bc1 = 1.0f - powf(b1, (float)c);
     const float bc2 = 1.0f - powf(b2, (float)c);
     const int64_t total = m * (int64_t)P;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t i = (int)blockIdx.x < nb ? blockIdx.x * (int64_t)TAIL_T + threadIdx.x : total; i < total;
+         i += (int64_t)nb * TAIL_T) {
         const int64_t j = i / P;
         const int q = (int)(i - j * P);
         const float g = item_sum(part + q, item_start[j], item_start[j + 1], P);
@@ -942,7 +989,7 @@ extern "C" int fbp_pou_loss(int32_t xd, int32_t d2mask, const fbp_problem* prob,
 
 extern "C" int fbp_loss_finalize(const double* loss_part, int32_t n_part, double scale, double* loss, void* stream) {
     FBP_REQUIRE(loss_part && loss && n_part > 0, FBP_ERR_INVALID, "fbp_loss_finalize: bad args");
-    loss_finalize_kernel<<<1, 256, 0, as_stream(stream)>>>(loss_part, n_part, scale, loss);
+    loss_finalize_kernel<<<1, TAIL_T, 0, as_stream(stream)>>>(loss_part, n_part, scale, loss);
     FBP_LAUNCH_CHECK();
     return FBP_OK;
 }
@@ -966,8 +1013,8 @@ extern "C" int fbp_step_tail(const double* loss_part, int32_t n_part, double sca
     FBP_REQUIRE(loss_part && loss && n_part > 0 && grad_part && item_start && grad && theta && m1 && m2 && state &&
                     count_dev && ticket && m > 0 && nparam > 0,
                 FBP_ERR_INVALID, "fbp_step_tail: bad args");
-    const int64_t b = std::min<int64_t>((m * (int64_t)nparam + 255) / 256, (int64_t)sm_count() * 8);
-    step_tail_kernel<<<(int)b, 256, 0, as_stream(stream)>>>(loss_part, n_part, scale, loss, grad_part, item_start, m,
+    const int64_t b = std::min<int64_t>((m * (int64_t)nparam + TAIL_T - 1) / TAIL_T, (int64_t)sm_count() * 16);
+    step_tail_kernel<<<(int)b + 1, TAIL_T, 0, as_stream(stream)>>>(loss_part, n_part, scale, loss, grad_part, item_start, m,
                                                            nparam, grad, theta, m1, m2, state, lr, b1, b2, eps,
                                                            eps_root, count_dev, ticket);
     FBP_LAUNCH_CHECK();

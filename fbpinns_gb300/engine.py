@@ -167,6 +167,20 @@ class PointSet:
         # resident CTAs (otherwise its counter reset costs more than it saves)
         self.chunk, self.fwd_chunk, self.dynamic = work_item_sizes(s_cap, m, eng.sm_count, self.chunk_req,
                                                                    self.fwd_req, eng.adaptive_items)
+        if eng.adaptive_items:
+            # The tensor-core kernels' set-up per item (B operands, the reduction of
+            # the item's sums) is larger and they have fewer, larger CTAs: up to four
+            # times the requested pairs while that leaves 32 adjoint and 16 forward
+            # items per SM.  Steps with 1024 / 4096 pairs, and with up to 4096 / 16384:
+            # Helmholtz, 1.7e7 pairs of 2-32-32-1 networks 9323 and 8672 us,
+            # Poisson, 9.4e6 pairs of 2-16-16-1 networks 2043 and 1962 us
+            adj, fwd, _ = work_item_sizes(s_cap, m, 4 * eng.sm_count, 4 * self.chunk_req, 4 * self.fwd_req)
+            if eng.tc_adjoint:
+                self.chunk = max(self.chunk, adj)
+            if eng.tensor_cores:
+                self.fwd_chunk = max(self.fwd_chunk, fwd)
+            self.fwd_chunk = max(self.fwd_chunk, self.chunk)
+            self.dynamic = s_cap // self.chunk + m > 4 * eng.sm_count
         self.items_cap = s_cap // self.chunk + m + 1
         self.forward_items_cap = s_cap // self.fwd_chunk + m + 1  # the forward queue's items fit in this
         self.items_all = torch.zeros(3 * self.items_cap, **i32)
