@@ -79,7 +79,7 @@ __device__ __forceinline__ void tc_fwd_issue(uint32_t tmem, uint32_t zcol, uint3
 }
 
 template <class C>
-__global__ void __launch_bounds__(TcFwd<C>::T) __maxnreg__(TcFwd<C>::REGS) forward_pairs_tm_kernel(fbp_net net, const float* __restrict__ x,
+__global__ void __maxnreg__(TcFwd<C>::REGS) forward_pairs_tm_kernel(fbp_net net, const float* __restrict__ x,
                                                                            fbp_pairs pr, float* __restrict__ pair_out,
                                                                            int32_t* __restrict__ status) {
     using A = TcFwd<C>;
