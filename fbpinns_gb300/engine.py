@@ -113,6 +113,23 @@ def work_item_sizes(s_cap, m, sms, chunk, forward_chunk, adaptive=True):
     return adj, fwd, s_cap // adj + m > 4 * sms
 
 
+def tc_item_size(s_cap, sms, rebuilt):
+    """Pairs per item, forward and adjoint, of the tensor-core kernels for up to
+    s_cap pairs on sms SMs: their set-up per item (B operands, parameters, the
+    reduction of the item's sums) costs about two tiles of 128 pairs and they
+    have one or two CTAs per SM, so items are whole tiles and about 13 per SM.
+    Where the lists are rebuilt every step, fewer, down to four per SM, until
+    items have six tiles: the CTAs that then stay idle leave the list kernels of
+    the next batch room.  Steps in us by size, the nearest to the rule's marked *:
+    Poisson, 9.4e6 pairs 1024 2043, 2048 1956, 4096 1918, 6144 1893*; Helmholtz,
+    1.7e7 pairs 1024 9323, 4096 8675, 8192 8465*; wave, 4.1e6 pairs 1024 3108,
+    2176 3058*, 3072 3142; SIREN, 1.8e6 pairs 1024 510*, 1536 524, 2048 545;
+    Burgers 256 67*, 512 70; Poisson, 16381 points redrawn 256 144, 512 136,
+    768 119*, 1024 131."""
+    size = max(s_cap // (13 * sms), min(768, s_cap // (4 * sms)) if rebuilt else 0)
+    return max(128, (size + 127) // 128 * 128)
+
+
 class PointSet:
     """Interaction lists, subdomain-major pair order, work queues and jet buffers
     of one set of points ``x`` (n, xd) on the device.
@@ -167,20 +184,14 @@ class PointSet:
         # resident CTAs (otherwise its counter reset costs more than it saves)
         self.chunk, self.fwd_chunk, self.dynamic = work_item_sizes(s_cap, m, eng.sm_count, self.chunk_req,
                                                                    self.fwd_req, eng.adaptive_items)
-        if eng.adaptive_items:
-            # The tensor-core kernels' set-up per item (B operands, the reduction of
-            # the item's sums) is larger and they have fewer, larger CTAs: up to four
-            # times the requested pairs while that leaves 32 adjoint and 16 forward
-            # items per SM.  Steps with 1024 / 4096 pairs, and with up to 4096 / 16384:
-            # Helmholtz, 1.7e7 pairs of 2-32-32-1 networks 9323 and 8672 us,
-            # Poisson, 9.4e6 pairs of 2-16-16-1 networks 2043 and 1962 us
-            adj, fwd, _ = work_item_sizes(s_cap, m, 4 * eng.sm_count, 4 * self.chunk_req, 4 * self.fwd_req)
+        if eng.adaptive_items and self.chunk_req >= 512:
+            size = min(tc_item_size(s_cap, eng.sm_count, self.fixed_caps), 8 * self.chunk_req)
             if eng.tc_adjoint:
-                self.chunk = max(self.chunk, adj)
+                self.chunk = max(self.chunk, size)
+                self.dynamic = s_cap // self.chunk + m > 4 * eng.sm_count
             if eng.tensor_cores:
-                self.fwd_chunk = max(self.fwd_chunk, fwd)
+                self.fwd_chunk = max(self.chunk, size)
             self.fwd_chunk = max(self.fwd_chunk, self.chunk)
-            self.dynamic = s_cap // self.chunk + m > 4 * eng.sm_count
         self.items_cap = s_cap // self.chunk + m + 1
         self.forward_items_cap = s_cap // self.fwd_chunk + m + 1  # the forward queue's items fit in this
         self.items_all = torch.zeros(3 * self.items_cap, **i32)
