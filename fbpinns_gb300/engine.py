@@ -123,7 +123,7 @@ def tc_item_size(s_cap, sms, rebuilt):
     the next batch room.  Steps in us by size, the nearest to the rule's marked *:
     Poisson, 9.4e6 pairs 1024 2043, 2048 1956, 4096 1918, 6144 1893*; Helmholtz,
     1.7e7 pairs 1024 9323, 4096 8675, 8192 8465*; wave, 4.1e6 pairs 1024 3108,
-    2176 3058*, 3072 3142; SIREN, 1.8e6 pairs 1024 510*, 1536 524, 2048 545;
+    2176 3058*, 3072 3142; SIREN, 1.8e6 pairs 1024 510, 1152 528*, 1536 524;
     Burgers 256 67*, 512 70; Poisson, 16381 points redrawn 256 144, 512 136,
     768 119*, 1024 131."""
     size = max(s_cap // (13 * sms), min(768, s_cap // (4 * sms)) if rebuilt else 0)
@@ -696,27 +696,30 @@ def constrained_jets(cfn, all_params, x, U, xd, d2mask, need=None):
     J = U.shape[1]
     out = [None] * J
     u0 = U[:, 0:1]
-    out[0] = cfn(all_params, x, u0)
-    if out[0] is u0:
-        return U
     second = {d: jet_index(xd, d2mask, (d, d)) for d in range(xd) if (d2mask >> d) & 1}
     dims = [d for d in range(xd) if need is None or 1 + d in need or second.get(d) in need]
+    try:
+        if not dims:
+            raise NoRule
+        ud = torch.stack([U[:, 1 + d:2 + d] for d in dims])
+        udd = torch.stack([U[:, second[d]:second[d] + 1] if d in second else torch.zeros_like(u0) for d in dims])
+        same, out[0], yd, ydd = jets(lambda xj, uj: cfn(all_params, xj, uj), x, dims, u0, ud, udd if second else None)
+        if same:
+            return U
+        zeros = torch.zeros_like(out[0])
+        for d in range(xd):
+            i = dims.index(d) if d in dims else None
+            out[1 + d] = zeros if i is None or yd is None else yd[i]
+            if d in second:
+                out[second[d]] = zeros if i is None or ydd is None else ydd[i]
+        return torch.cat(out, dim=1)
+    except NoRule:
+        out[0] = cfn(all_params, x, u0)
+    if out[0] is u0:
+        return U
     for d in set(range(xd)) - set(dims):
         for k in [1 + d] + ([second[d]] if d in second else []):
             out[k] = torch.zeros_like(out[0])
-    if not dims:
-        return torch.cat(out, dim=1)
-    try:
-        ud = torch.stack([U[:, 1 + d:2 + d] for d in dims])
-        udd = torch.stack([U[:, second[d]:second[d] + 1] if d in second else torch.zeros_like(u0) for d in dims])
-        _, yd, ydd = jets(lambda xj, uj: cfn(all_params, xj, uj), x, dims, u0, ud, udd if second else None)
-        for i, d in enumerate(dims):
-            out[1 + d] = torch.zeros_like(out[0]) if yd is None else yd[i]
-            if d in second:
-                out[second[d]] = torch.zeros_like(out[0]) if ydd is None else ydd[i]
-        return torch.cat(out, dim=1)
-    except NoRule:
-        pass
     ones = torch.ones((n, 1), dtype=x.dtype, device=x.device)
     zero = torch.zeros((n, 1), dtype=x.dtype, device=x.device)
     for d in dims:

@@ -209,14 +209,15 @@ class Jet(torch.Tensor):
 
 
 def jets(fn, x, dims, u, ud, udd):
-    """(value, d, dd) of fn(x, u) along the unit directions ``dims`` of x (n, xd),
-    where u has the derivatives ud, udd (directions, n, 1); d and dd as
-    (directions, n, 1), or None for zero.  Raises NoRule where fn makes a call
-    without a rule."""
+    """(same, value, d, dd) of fn(x, u) along the unit directions ``dims`` of x
+    (n, xd), where u has the derivatives ud, udd (directions, n, 1): whether fn
+    returned its u itself, and its value, d and dd as (n, 1) and (directions, n,
+    1), or None for zero.  Raises NoRule where fn makes a call without a rule."""
     e = torch.zeros((len(dims), 1, x.shape[1]), dtype=x.dtype, device=x.device)
     for i, d in enumerate(dims):
         e[i, 0, d] = 1.0
-    y = fn(Jet.make(x, e.expand(-1, x.shape[0], -1), None), Jet.make(u, ud, udd))
+    uj = Jet.make(u, ud, udd)
+    y = fn(Jet.make(x, e.expand(-1, x.shape[0], -1), None), uj)
     if not isinstance(y, torch.Tensor) or y.dtype != u.dtype:
         raise NoRule
-    return (y.v, y.d, y.dd) if isinstance(y, Jet) else (y, None, None)
+    return (y is uj,) + ((y.v, y.d, y.dd) if isinstance(y, Jet) else (y, None, None))

@@ -81,5 +81,5 @@ def test_every_builtin_constraint_has_rules():
         xd, d2, fn, p = CASES[name]
         x = torch.rand((5, xd), dtype=torch.float64)
         z = torch.zeros((xd, 5, 1), dtype=torch.float64)
-        _, d, dd = taylor.jets(lambda a, b: fn(p, a, b), x, list(range(xd)), x[:, 0:1] * 1, z + 1, z)
+        _, _, d, dd = taylor.jets(lambda a, b: fn(p, a, b), x, list(range(xd)), x[:, 0:1] * 1, z + 1, z)
         assert d.shape == dd.shape == (xd, 5, 1) and torch.isfinite(d).all() and math.isfinite(dd.sum().item())
