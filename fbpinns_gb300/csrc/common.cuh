@@ -137,6 +137,32 @@ __device__ __forceinline__ void adam_element(float& theta, float& m1, float& m2,
     theta = theta + (-lr) * (mh / (sqrtf(nh + eps_root) + eps));
 }
 
+// Programmatic dependent launch between the kernels of a step: the next kernel
+// may be set up while the one before it ends, and waits, before it touches
+// global memory, until that one has completed and its writes are visible.  It
+// does nothing for kernels launched without it.  (No kernel lets the next one
+// start early: waiting CTAs then hold registers and tensor memory that the list
+// kernels on the other stream could use -- a step of 16381 redrawn points 118
+// -> 132 us, Burgers 67 -> 72.)  The 1D oscillator's step 35.0 -> 33.0 us.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launches a kernel that begins with pdl_wait, so that its launch overlaps the
+// end of the kernel before it on the stream.
+template <class... P, class... A>
+cudaError_t launch_after(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 inline int jet_size_rt(int xd, int d2) { return 1 + xd + d2_slots(d2); }
 
 }  // namespace fbp

@@ -186,6 +186,7 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait();
     const uint32_t tmem = T.tmem_base;
     const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)n0;  // this thread's lane and columns
     const uint32_t b1h = smem_u32(&T.b1[0][0]), b1l = smem_u32(&T.b1[1][0]);

@@ -58,10 +58,10 @@ int launch_adjoint_tc(const fbp_net& net, const float* x, const fbp_pairs& pr, c
     }
     FBP_REQUIRE(L.res * cols <= 512, FBP_ERR_UNSUPPORTED, "adjoint_tc: %d CTAs/SM x %d TMEM columns > 512", L.res,
                 cols);
-    if (grid <= 0) grid = L.res * sm_count();
+    if (grid <= 0) grid = (int)std::min<int64_t>(L.res * sm_count(), std::max<int64_t>(pr.items_cap, 1));
     if (pr.item_ctr) FBP_CUDA_CHECK(cudaMemsetAsync(pr.item_ctr, 0, sizeof(int32_t), st));
-    adjoint_pairs_tc_kernel<C><<<grid, threads, L.shm, st>>>(net, x, pr, slot_out, grad_part, status);
-    FBP_LAUNCH_CHECK();
+    FBP_CUDA_CHECK(launch_after(adjoint_pairs_tc_kernel<C>, grid, threads, L.shm, st, net, x, pr, slot_out, grad_part,
+                                status));
     return FBP_OK;
 }
 

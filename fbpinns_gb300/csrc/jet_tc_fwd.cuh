@@ -353,7 +353,7 @@ int launch_forward_tm(const fbp_net& net, const float* x, const fbp_pairs& pr, f
                                             (int)shm));
         attr_set[dev].store(true);
     }
-    if (grid <= 0) grid = res * sm_count();
+    if (grid <= 0) grid = (int)std::min<int64_t>(res * sm_count(), std::max<int64_t>(pr.items_cap, 1));
     if (pr.item_ctr) FBP_CUDA_CHECK(cudaMemsetAsync(pr.item_ctr, 0, sizeof(int32_t), st));
     forward_pairs_tm_kernel<C><<<grid, TcFwd<C>::T, shm, st>>>(net, x, pr, pair_out, status);
     FBP_LAUNCH_CHECK();

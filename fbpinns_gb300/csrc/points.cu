@@ -85,6 +85,7 @@ __global__ void cell_count_kernel(const float* __restrict__ x, int64_t n, CellGr
 __global__ void __launch_bounds__(kScanThreads) cell_scan_kernel(const int32_t* __restrict__ count, int ncell,
                                                                  int32_t* __restrict__ start,
                                                                  int32_t* __restrict__ cursor) {
+    pdl_wait();
     __shared__ int32_t warp_sums[kScanThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int per = (ncell + kScanThreads - 1) / kScanThreads;
@@ -122,6 +123,7 @@ __global__ void __launch_bounds__(kScanThreads) cell_scan_kernel(const int32_t* 
 
 __global__ void cell_scatter_kernel(const int32_t* __restrict__ key, int64_t n, int32_t* __restrict__ cursor,
                                     int32_t* __restrict__ idx) {
+    pdl_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         idx[atomicAdd(&cursor[key[i]], 1)] = (int32_t)i;
 }
@@ -133,6 +135,7 @@ __global__ void __launch_bounds__(kOrderWarps * 32) cell_order_kernel(const int3
                                                                       const int32_t* __restrict__ start, int ncell,
                                                                       const float* __restrict__ x_in, int xd,
                                                                       float* __restrict__ x_out) {
+    pdl_wait();
     __shared__ int32_t stage[kOrderWarps][kOrderStage];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int32_t* st = stage[wid];
@@ -234,13 +237,10 @@ extern "C" int fbp_sort_points_cells(const float* x_in, int64_t n, int32_t xd, c
     if (blocks > sm_count() * 8) blocks = sm_count() * 8;
     cell_count_kernel<<<blocks, 256, 0, st>>>(x_in, n, g, key, count);
     FBP_LAUNCH_CHECK();
-    cell_scan_kernel<<<1, kScanThreads, 0, st>>>(count, ncell, start, cursor);
-    FBP_LAUNCH_CHECK();
-    cell_scatter_kernel<<<blocks, 256, 0, st>>>(key, n, cursor, idx);
-    FBP_LAUNCH_CHECK();
+    FBP_CUDA_CHECK(launch_after(cell_scan_kernel, 1, kScanThreads, 0, st, count, ncell, start, cursor));
+    FBP_CUDA_CHECK(launch_after(cell_scatter_kernel, blocks, 256, 0, st, key, n, cursor, idx));
     int oblocks = (ncell + kOrderWarps - 1) / kOrderWarps;
     if (oblocks > sm_count() * 8) oblocks = sm_count() * 8;
-    cell_order_kernel<<<oblocks, kOrderWarps * 32, 0, st>>>(idx, start, ncell, x_in, xd, x_out);
-    FBP_LAUNCH_CHECK();
+    FBP_CUDA_CHECK(launch_after(cell_order_kernel, oblocks, kOrderWarps * 32, 0, st, idx, start, ncell, x_in, xd, x_out));
     return FBP_OK;
 }

@@ -611,6 +611,7 @@ __global__ void __launch_bounds__(POU_WARPS * 32) pou_loss_kernel(fbp_problem P,
     constexpr int J = JL<XD, D2>::J, RS = rec_stride(J), NV = 2 * J, SLOTCAP = pou_slotcap(RS);
     __shared__ __align__(16) float table[POU_WARPS][SLOTCAP * RS];
     __shared__ double sh[POU_WARPS];
+    pdl_wait();
     __shared__ Gauss gs[XD == 2 ? GAUSS_CAP : 1];  // the Helmholtz source
     if (XD == 2 && P.kind == FBP_PROBLEM_HELMHOLTZ2D && P.ng <= GAUSS_CAP) {
         for (int g = threadIdx.x; g < P.ng; g += blockDim.x) {
@@ -858,6 +859,7 @@ __global__ void __launch_bounds__(TAIL_T) step_tail_kernel(const double* __restr
                                                         float eps, float eps_root, int32_t* count_dev,
                                                         int32_t* ticket) {
     __shared__ double sh[32];
+    pdl_wait();
     const int c = *(volatile const int32_t*)count_dev + 1;
     const int nb = (int)gridDim.x - 1;  // the last CTA has the loss, the others the parameters
     if ((int)blockIdx.x == nb) loss_sum(loss_part, np, scale, loss, sh);
@@ -975,10 +977,8 @@ extern "C" int fbp_pou_loss(int32_t xd, int32_t d2mask, const fbp_problem* prob,
     const float inv_n = (float)(1.0 / (double)n);
 #define X(a, b)                                                                                              \
     if (xd == a && d2mask == b) {                                                                            \
-        pou_loss_kernel<a, b><<<g, POU_WARPS * 32, 0, st>>>(*prob, n, npou, inv_n, x, pt_off, np_off, p_take,   \
-                                                             pair_out,                                        \
-                                                    slot_out, U_out, s_cap, u_cap, loss_part, n_part, status); \
-        FBP_LAUNCH_CHECK();                                                                                  \
+        FBP_CUDA_CHECK(launch_after(pou_loss_kernel<a, b>, g, POU_WARPS * 32, 0, st, *prob, n, npou, inv_n, x, pt_off, \
+                                    np_off, p_take, pair_out, slot_out, U_out, s_cap, u_cap, loss_part, n_part, status)); \
         return FBP_OK;                                                                                       \
     }
     FBP_XD_D2_CASES(X)
@@ -1014,9 +1014,8 @@ extern "C" int fbp_step_tail(const double* loss_part, int32_t n_part, double sca
                     count_dev && ticket && m > 0 && nparam > 0,
                 FBP_ERR_INVALID, "fbp_step_tail: bad args");
     const int64_t b = std::min<int64_t>((m * (int64_t)nparam + TAIL_T - 1) / TAIL_T, (int64_t)sm_count() * 16);
-    step_tail_kernel<<<(int)b + 1, TAIL_T, 0, as_stream(stream)>>>(loss_part, n_part, scale, loss, grad_part, item_start, m,
-                                                           nparam, grad, theta, m1, m2, state, lr, b1, b2, eps,
-                                                           eps_root, count_dev, ticket);
-    FBP_LAUNCH_CHECK();
+    FBP_CUDA_CHECK(launch_after(step_tail_kernel, (int)b + 1, TAIL_T, 0, as_stream(stream), loss_part, n_part, scale,
+                                loss, grad_part, item_start, m, nparam, grad, theta, m1, m2, state, lr, b1, b2, eps,
+                                eps_root, count_dev, ticket));
     return FBP_OK;
 }

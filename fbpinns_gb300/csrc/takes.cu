@@ -67,6 +67,7 @@ __global__ void inside_count_kernel(const float* __restrict__ x, int64_t n, fbp_
                                     uint64_t* __restrict__ pt_lvl, int32_t* __restrict__ model_count,
                                     uint64_t* __restrict__ pt_hit, int32_t* __restrict__ pt_cand,
                                     int2* __restrict__ sums) {
+    pdl_wait();
     extern __shared__ int32_t box_count[];
     if constexpr (SHIST) {
         for (int64_t j = threadIdx.x; j < b.m; j += blockDim.x) box_count[j] = 0;
@@ -154,6 +155,7 @@ __global__ void __launch_bounds__(FILL_WARPS * 32)
                        const uint64_t* __restrict__ pt_hit, const int32_t* __restrict__ pt_cand,
                        int32_t* __restrict__ n_take, int32_t* __restrict__ m_take, int32_t* __restrict__ p_take,
                        int32_t* __restrict__ np_take, int64_t s_cap, int64_t u_cap, int32_t* __restrict__ status) {
+    pdl_wait();
     __shared__ int32_t stage[FILL_WARPS][FILL_STAGE];
     __shared__ uint64_t s_lvl[FILL_WARPS][32];
     __shared__ int32_t s_ubase[FILL_WARPS][32];
@@ -347,6 +349,7 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* smem_warp, int& 
 }
 
 __global__ void scan_reduce_kernel(const int32_t* __restrict__ in, int64_t n, int32_t* __restrict__ sums) {
+    pdl_wait();
     __shared__ int sw[33];
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE;
     int s = 0;
@@ -362,6 +365,7 @@ __global__ void scan_reduce_kernel(const int32_t* __restrict__ in, int64_t n, in
 
 // single block: exclusive scan of the tile sums in place, total at sums[nb]
 __global__ void scan_sums_kernel(int32_t* __restrict__ sums, int64_t nb) {
+    pdl_wait();
     __shared__ int sw[33];
     int carry = 0;
     for (int64_t b0 = 0; b0 < nb; b0 += blockDim.x) {
@@ -385,6 +389,7 @@ constexpr int64_t SCAN_FUSED_TILES = 4096;
 // scanned offsets and the total at sums[nb].
 __global__ void scan_down_kernel(const int32_t* __restrict__ in, int64_t n, const int32_t* __restrict__ sums,
                                  int64_t nb, int32_t* __restrict__ out, bool fused) {
+    pdl_wait();
     __shared__ int sw[33];
     __shared__ int tile[SCAN_TILE];
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE;
@@ -434,14 +439,11 @@ int scan_launch(const int32_t* in, int32_t* out, int64_t n, int32_t* sums, cudaS
         return FBP_OK;
     }
     const bool fused = nb <= SCAN_FUSED_TILES;
-    scan_reduce_kernel<<<(unsigned)nb, SCAN_T, 0, st>>>(in, n, sums);
-    FBP_LAUNCH_CHECK();
+    FBP_CUDA_CHECK(launch_after(scan_reduce_kernel, (int)nb, SCAN_T, 0, st, in, n, sums));
     if (!fused) {
-        scan_sums_kernel<<<1, 1024, 0, st>>>(sums, nb);
-        FBP_LAUNCH_CHECK();
+        FBP_CUDA_CHECK(launch_after(scan_sums_kernel, 1, 1024, 0, st, sums, nb));
     }
-    scan_down_kernel<<<(unsigned)nb, SCAN_T, 0, st>>>(in, n, sums, nb, out, fused);
-    FBP_LAUNCH_CHECK();
+    FBP_CUDA_CHECK(launch_after(scan_down_kernel, (int)nb, SCAN_T, 0, st, in, n, sums, nb, out, fused));
     return FBP_OK;
 }
 
@@ -504,6 +506,7 @@ __global__ void sort_hist_kernel(const int32_t* __restrict__ key, const int32_t*
                                  const uint8_t* __restrict__ pt_keep, const int32_t* __restrict__ s_dev,
                                  int64_t s_cap, int64_t m, int64_t nchunks, int64_t chn,
                                  int32_t* __restrict__ hist) {
+    pdl_wait();
     extern __shared__ int cnt[];
     const int64_t s = min((int64_t)*s_dev, s_cap);
     for (int64_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
@@ -547,6 +550,7 @@ __global__ void __launch_bounds__(SCATTER_W * 32)
                         const int32_t* __restrict__ s_dev, int64_t s_cap, int64_t m, int64_t nchunks,
                         int64_t chn, const int32_t* __restrict__ hoff, int4* __restrict__ sd_rec,
                         int32_t* __restrict__ sd_start) {
+    pdl_wait();
     extern __shared__ int run[];  // [W][m]: per-warp counts, then running offsets
     // sd_start[j] = hoff[j * nchunks] (start of bucket j), sd_start[m] = s
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j <= m; j += (int64_t)gridDim.x * blockDim.x)
@@ -645,6 +649,7 @@ __global__ void __launch_bounds__(WORK_T) work_kernel(const int32_t* __restrict_
                                                       int32_t* __restrict__ items, int32_t* __restrict__ item_start,
                                                       int32_t* __restrict__ n_items, int64_t cap,
                                                       int32_t* __restrict__ status) {
+    pdl_wait();
     __shared__ int sw[33];
     __shared__ int2 s_item[WORK_T];  // first item and number of items of the CTA's subdomains
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -759,18 +764,17 @@ static int launch_count(const float* x, int64_t n, const fbp_boxes* boxes, int32
     const int t = shist ? COUNT_T : LIST_CHUNK;
     const int g = shist ? grid_for(n, t, COUNT_CTAS) : grid_for(n, t);
     const size_t shm = shist ? (size_t)boxes->m * sizeof(int32_t) : 0;
-#define X(D)                                                                                                         \
-    if (boxes->xd == D) {                                                                                            \
-        if (shist)                                                                                                   \
-            inside_count_kernel<D, true><<<g, t, shm, st>>>(x, n, *boxes, pt_count, pt_nlvl, pt_lvl, model_count,    \
-                                                            pt_hit, pt_cand, sums);                                  \
-        else                                                                                                         \
-            inside_count_kernel<D, false><<<g, t, 0, st>>>(x, n, *boxes, pt_count, pt_nlvl, pt_lvl, model_count,     \
-                                                           pt_hit, pt_cand, sums);                                   \
+#define X(D)                                                                                                        \
+    if (boxes->xd == D) {                                                                                           \
+        if (shist)                                                                                                  \
+            FBP_CUDA_CHECK(launch_after(inside_count_kernel<D, true>, g, t, shm, st, x, n, *boxes, pt_count, pt_nlvl, \
+                                        pt_lvl, model_count, pt_hit, pt_cand, sums));                               \
+        else                                                                                                        \
+            FBP_CUDA_CHECK(launch_after(inside_count_kernel<D, false>, g, t, 0, st, x, n, *boxes, pt_count, pt_nlvl, \
+                                        pt_lvl, model_count, pt_hit, pt_cand, sums));                               \
     }
     X(1) X(2) X(3)
 #undef X
-    FBP_LAUNCH_CHECK();
     return FBP_OK;
 }
 
@@ -782,17 +786,16 @@ static int launch_fill(const float* x, int64_t n, const fbp_boxes* boxes, int32_
 #define X(D)                                                                                                        \
     if (boxes->xd == D) {                                                                                           \
         if (sums)                                                                                                   \
-            inside_fill_kernel<D, true><<<g, FILL_WARPS * 32, 0, st>>>(                                             \
-                x, n, *boxes, pt_off, np_off, pt_count, sums, pt_lvl, pt_hit, pt_cand, n_take, m_take, p_take,      \
-                np_take, s_cap, u_cap, status);                                                                     \
+            FBP_CUDA_CHECK(launch_after(inside_fill_kernel<D, true>, g, FILL_WARPS * 32, 0, st, x, n, *boxes, pt_off, \
+                                        np_off, pt_count, sums, pt_lvl, pt_hit, pt_cand, n_take, m_take, p_take,    \
+                                        np_take, s_cap, u_cap, status));                                            \
         else                                                                                                        \
-            inside_fill_kernel<D, false><<<g, FILL_WARPS * 32, 0, st>>>(                                            \
-                x, n, *boxes, pt_off, np_off, nullptr, nullptr, pt_lvl, pt_hit, pt_cand, n_take, m_take, p_take,    \
-                np_take, s_cap, u_cap, status);                                                                     \
+            FBP_CUDA_CHECK(launch_after(inside_fill_kernel<D, false>, g, FILL_WARPS * 32, 0, st, x, n, *boxes, pt_off, \
+                                        np_off, nullptr, nullptr, pt_lvl, pt_hit, pt_cand, n_take, m_take, p_take,  \
+                                        np_take, s_cap, u_cap, status));                                            \
     }
     X(1) X(2) X(3)
 #undef X
-    FBP_LAUNCH_CHECK();
     return FBP_OK;
 }
 
@@ -943,16 +946,15 @@ static int sort_pairs(const int32_t* m_take, const int32_t* n_take, const int32_
             cudaFuncSetAttribute(sort_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(shm * sw)));
     if (nch > 0) {
         const int g = (int)std::min<int64_t>(nch, (int64_t)sm_count() * 8);
-        sort_hist_kernel<<<g, 256, shm, st>>>(m_take, n_take, pt_keep, s_dev, s_cap, m, nch, chn, hist);
-        FBP_LAUNCH_CHECK();
+        FBP_CUDA_CHECK(launch_after(sort_hist_kernel, g, 256, shm, st, m_take, n_take, pt_keep, s_dev, s_cap, m, nch, chn,
+                                    hist));
     }
     int rc = scan_launch(hist, hoff, hn, sums, st);
     if (rc) return rc;
     if (nch > 0) {
         const int g = (int)std::min<int64_t>(nch, (int64_t)sm_count() * 32 / sw);
-        sort_scatter_kernel<<<g, 32 * sw, shm * sw, st>>>(m_take, n_take, p_take, pt_keep, s_dev, s_cap, m, nch,
-                                                          chn, hoff, reinterpret_cast<int4*>(sd_rec), sd_start);
-        FBP_LAUNCH_CHECK();
+        FBP_CUDA_CHECK(launch_after(sort_scatter_kernel, g, 32 * sw, shm * sw, st, m_take, n_take, p_take, pt_keep, s_dev,
+                                    s_cap, m, nch, chn, hoff, reinterpret_cast<int4*>(sd_rec), sd_start));
     } else {
         FBP_CUDA_CHECK(cudaMemsetAsync(sd_start, 0, (size_t)(m + 1) * sizeof(int32_t), st));
     }
@@ -1003,8 +1005,7 @@ extern "C" int fbp_build_work(const int32_t* sd_start, int64_t m, const uint8_t*
     FBP_REQUIRE(scratch && scratch_bytes >= fbp_work_scratch_bytes(m), FBP_ERR_CAPACITY,
                 "fbp_build_work: scratch too small");
     cudaStream_t st = as_stream(stream);
-    work_kernel<<<(unsigned)((m + WORK_T - 1) / WORK_T), WORK_T, 0, st>>>(sd_start, m, select, chunk, items, item_start,
-                                                                        n_items, items_cap, status);
-    FBP_LAUNCH_CHECK();
+    FBP_CUDA_CHECK(launch_after(work_kernel, (int)((m + WORK_T - 1) / WORK_T), WORK_T, 0, st, sd_start, m, select, chunk,
+                                items, item_start, n_items, items_cap, status));
     return FBP_OK;
 }
