@@ -358,75 +358,92 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
             tc_fence_after();
             // ---- tanh jets of layer 2 and their adjoint -> z2bar ----
             {
-                float acc[J][8];
-#pragma unroll
-                for (int c = 0; c < J; ++c) tmem_ld8(mine + A::cZ + c * H, acc[c]);
-                tmem_wait_ld();
-                if constexpr (A::OVER) {  // every thread has read its z before z2bar takes the columns
-                    tc_fence_before();
-                    __syncthreads();
-                    tc_fence_after();
-                }
                 float ob[J];
 #pragma unroll
                 for (int c = 0; c < J; ++c) ob[c] = T.xo[buf][XD + c][r];
                 if (h == 0) g3b += ob[0];
+                // eight neurons at a time, or four where z's columns are taken by z2bar:
+                // that wait for every thread's z would keep all J x 8 in registers
+                constexpr int NH = A::OVER ? 4 : 8;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int k = n0 + 2 * q;
-                    float2 z[J];
+                for (int half = 0; half < 8 / NH; ++half) {
+                    float acc[J][NH];
 #pragma unroll
-                    for (int c = 0; c < J; ++c) z[c] = make_float2(acc[c][2 * q], acc[c][2 * q + 1]);
-                    z[0] = add2(z[0], *reinterpret_cast<const float2*>(&S.b2[k]));
-                    float2 a, tp;
-                    F::template first<true>(S, k, z[0], a, tp);
-                    const float2 tpp = F::template second<true>(S, k, F::template m2<true>(a, tp));
-                    const float2 tppp = F::template third<true>(S, k, tp);
-                    // the sensitivities of sigma' and sigma'' over W3: P = sum_d ob_d z_d +
-                    // sum_s ob_s z_s, Q = sum_s ob_s sum_d z_d^2; then W3-bar += ob_0 a +
-                    // tp P + tpp Q, z2bar_0 = W3 (ob_0 tp + tpp P + tppp Q), z2bar_d =
-                    // W3 (ob_d tp + 2 ob_s tpp z_d), z2bar_s = W3 ob_s tp
-                    const float2 w3 = *reinterpret_cast<const float2*>(&S.W3[k]);
-                    const float2 wtp = mul2(w3, tp), w4 = mul2(dup2(2.0f), mul2(w3, tpp));
-                    float2 P = mul2(dup2(ob[1]), z[1]), Q = dup2(0.f), zb[J];
-#pragma unroll
-                    for (int d = 1; d < XD; ++d) P = fma2(dup2(ob[1 + d]), z[1 + d], P);
-#pragma unroll
-                    for (int d = 0; d < XD; ++d) zb[1 + d] = mul2(dup2(ob[1 + d]), wtp);
-#pragma unroll
-                    for (int s = 0; s < NS; ++s) {
-                        const float2 os = dup2(ob[1 + XD + s]), o4 = mul2(os, w4);
-                        float2 q2 = dup2(0.f);  // sum of z_d^2 over the slot's dims
-                        bool first = true;
-#pragma unroll
-                        for (int d = 0; d < XD; ++d)
-                            if ((C::slot_dims(s) >> d) & 1) {
-                                q2 = first ? mul2(z[1 + d], z[1 + d]) : fma2(z[1 + d], z[1 + d], q2);
-                                first = false;
-                                zb[1 + d] = fma2(o4, z[1 + d], zb[1 + d]);
-                            }
-                        P = fma2(os, z[1 + XD + s], P);
-                        Q = s == 0 ? mul2(os, q2) : fma2(os, q2, Q);
-                        zb[1 + XD + s] = mul2(os, wtp);
+                    for (int c = 0; c < J; ++c) {
+                        if constexpr (NH == 8) tmem_ld8(mine + A::cZ + c * H, acc[c]);
+                        else tmem_ld4(mine + A::cZ + c * H + half * NH, acc[c]);
                     }
-                    float2 s3 = fma2(tp, P, fma2(dup2(ob[0]), a, sum[A::iW3][q]));
-                    float2 z0 = fma2(tpp, P, mul2(dup2(ob[0]), tp));
-                    if constexpr (NS > 0) {
-                        s3 = fma2(tpp, Q, s3);
-                        z0 = fma2(tppp, Q, z0);
-                    }
-                    zb[0] = mul2(w3, z0);
-                    sum[A::iW3][q] = s3;
-                    sum[A::iB2][q] = add2(sum[A::iB2][q], zb[0]);
+                    tmem_wait_ld();
 #pragma unroll
-                    for (int c = 0; c < J; ++c) acc[c][2 * q] = zb[c].x, acc[c][2 * q + 1] = zb[c].y;
+                    for (int qq = 0; qq < NH / 2; ++qq) {
+                        const int q = half * (NH / 2) + qq, k = n0 + 2 * q;
+                        float2 z[J];
+#pragma unroll
+                        for (int c = 0; c < J; ++c) z[c] = make_float2(acc[c][2 * qq], acc[c][2 * qq + 1]);
+                        z[0] = add2(z[0], *reinterpret_cast<const float2*>(&S.b2[k]));
+                        float2 a, tp;
+                        F::template first<true>(S, k, z[0], a, tp);
+                        const float2 tpp = F::template second<true>(S, k, F::template m2<true>(a, tp));
+                        const float2 tppp = F::template third<true>(S, k, tp);
+                        // the sensitivities of sigma' and sigma'' over W3: P = sum_d ob_d z_d +
+                        // sum_s ob_s z_s, Q = sum_s ob_s sum_d z_d^2; then W3-bar += ob_0 a +
+                        // tp P + tpp Q, z2bar_0 = W3 (ob_0 tp + tpp P + tppp Q), z2bar_d =
+                        // W3 (ob_d tp + 2 ob_s tpp z_d), z2bar_s = W3 ob_s tp
+                        const float2 w3 = *reinterpret_cast<const float2*>(&S.W3[k]);
+                        const float2 wtp = mul2(w3, tp), w4 = mul2(dup2(2.0f), mul2(w3, tpp));
+                        float2 P = mul2(dup2(ob[1]), z[1]), Q = dup2(0.f), zb[J];
+#pragma unroll
+                        for (int d = 1; d < XD; ++d) P = fma2(dup2(ob[1 + d]), z[1 + d], P);
+#pragma unroll
+                        for (int d = 0; d < XD; ++d) zb[1 + d] = mul2(dup2(ob[1 + d]), wtp);
+#pragma unroll
+                        for (int s = 0; s < NS; ++s) {
+                            const float2 os = dup2(ob[1 + XD + s]), o4 = mul2(os, w4);
+                            float2 q2 = dup2(0.f);  // sum of z_d^2 over the slot's dims
+                            bool first = true;
+#pragma unroll
+                            for (int d = 0; d < XD; ++d)
+                                if ((C::slot_dims(s) >> d) & 1) {
+                                    q2 = first ? mul2(z[1 + d], z[1 + d]) : fma2(z[1 + d], z[1 + d], q2);
+                                    first = false;
+                                    zb[1 + d] = fma2(o4, z[1 + d], zb[1 + d]);
+                                }
+                            P = fma2(os, z[1 + XD + s], P);
+                            Q = s == 0 ? mul2(os, q2) : fma2(os, q2, Q);
+                            zb[1 + XD + s] = mul2(os, wtp);
+                        }
+                        float2 s3 = fma2(tp, P, fma2(dup2(ob[0]), a, sum[A::iW3][q]));
+                        float2 z0 = fma2(tpp, P, mul2(dup2(ob[0]), tp));
+                        if constexpr (NS > 0) {
+                            s3 = fma2(tpp, Q, s3);
+                            z0 = fma2(tppp, Q, z0);
+                        }
+                        zb[0] = mul2(w3, z0);
+                        sum[A::iW3][q] = s3;
+                        sum[A::iB2][q] = add2(sum[A::iB2][q], zb[0]);
+#pragma unroll
+                        for (int c = 0; c < J; ++c) acc[c][2 * qq] = zb[c].x, acc[c][2 * qq + 1] = zb[c].y;
+                    }
+#pragma unroll
+                    for (int c = 0; c < J; ++c) {
+#pragma unroll
+                        for (int i = 0; i < NH; i += 4)
+                            *reinterpret_cast<float4*>(zrow + c * H + half * NH + i) =
+                                make_float4(acc[c][i], acc[c][i + 1], acc[c][i + 2], acc[c][i + 3]);
+                        if constexpr (NH == 8) tmem_st_split8(mine + A::zcol(c), H, acc[c]);
+                    }
                 }
+                if constexpr (A::OVER) {
+                    tc_fence_before();
+                    __syncthreads();  // every thread has read its z
+                    tc_fence_after();
 #pragma unroll
-                for (int c = 0; c < J; ++c) {
-                    *reinterpret_cast<float4*>(zrow + c * H) = make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
-                    *reinterpret_cast<float4*>(zrow + c * H + 4) =
-                        make_float4(acc[c][4], acc[c][5], acc[c][6], acc[c][7]);
-                    tmem_st_split8(mine + A::zcol(c), H, acc[c]);
+                    for (int c = 0; c < J; ++c) {  // this thread's own row
+                        const float4 u = *reinterpret_cast<const float4*>(zrow + c * H);
+                        const float4 v = *reinterpret_cast<const float4*>(zrow + c * H + 4);
+                        const float zc[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+                        tmem_st_split8(mine + A::zcol(c), H, zc);
+                    }
                 }
             }
             tmem_wait_st();
