@@ -41,8 +41,10 @@ WIDTH = 2.9
 LR = 1e-3
 SEED = 0
 # DRAM bytes (read + write) of one adjoint launch and the pairs it covered, from an ncu
-# capture of this workload at 2^16 points: layer 2 recomputed, and z-jets read from the
-# forward's store (the forward then writes 256 B per pair more)
+# capture of this workload at 2^16 points: the tensor-core kernel, the FMA kernel with layer 2
+# recomputed, and the FMA kernel reading the forward's z-jets (the forward then writes 256 B per
+# pair more)
+ADJ_DRAM_TC = (52.576000e6 + 0.339456e6, 2342389)
 ADJ_DRAM_RECOMPUTE = (52.580352e6 + 0.155392e6, 2342389)
 ADJ_DRAM_STORED = (689.641984e6 + 3.272704e6, 2342389)
 METRIC = "FBPINN train steps/s, fused adjoint vs plain GPU step, at matched test L1 error"
@@ -457,9 +459,9 @@ def run_fused(args, world, rank, local):
     dom = max(("forward_pairs", "adjoint_pairs"), key=lambda k: timings[k])
     ach = (fl_adj if dom == "adjoint_pairs" else fl_fwd) / (timings[dom] * 1e-3) / 1e12
     # DRAM traffic of the adjoint per launch: ncu dram__bytes_read.sum + dram__bytes_write.sum of
-    # adjoint_pairs_kernel<Cfg<2,16,16,11>> in one capture of this workload at 2^16 points, scaled
+    # the adjoint kernel of Cfg<2,16,16,11> in one capture of this workload at 2^16 points, scaled
     # by this run's pairs (traffic grows with the pairs); per variant (bytes, pairs of the capture)
-    adj_dram = ADJ_DRAM_STORED if ps.zs is not None else ADJ_DRAM_RECOMPUTE
+    adj_dram = (ADJ_DRAM_TC if eng.tc_adjoint else ADJ_DRAM_STORED if ps.zs is not None else ADJ_DRAM_RECOMPUTE)
     traffic = adj_dram[0] / adj_dram[1] * pairs if (dom == "adjoint_pairs" and J == 4 and adj_dram) else None
     roofline = {"bound": "fp32", "kernel": dom, "achieved": ach, "peak": best, "unit": "TFLOP/s", "frac": ach / best,
                 "peak_source": "FP32 FMA probe (fbp_fma_probe) measured in this run; MEASURED_PEAKS.json has no FP32 figure",
@@ -555,12 +557,10 @@ def run_fused(args, world, rank, local):
         except Exception as ex:  # reported, not hidden
             cpu["agreement"] = {"error": repr(ex)[:200]}
 
-    # launches of our kernels in one step (counted from the C-ABI calls of the step body; each
-    # scan of up to 4096 tiles of 2048 is two launches, all of them at this size): sample (1),
-    # cell order (4), inside count (1), pair and slot offsets (2 + 2), fill (1), subdomain sort
-    # (hist 1, scan 2, scatter 1, starts 1), two work queues (count 1, scan 2, fill 1 each),
-    # forward, POU/loss, loss finalize, adjoint, gradient reduce, Adam + step count (1+1+1+1+1+2)
-    per_step = 1 + (4 if eng.cell_order else 0) + 1 + 4 + 1 + 5 + 2 * 4 + 7
+    # launches of our kernels in one step (the C-ABI calls of the step body, as the profiler lists
+    # them at this size): sample (1), cell order (4), lists: count, fill (2), subdomain sort
+    # (hist 1, scan 2, scatter 1), two work queues (1 each), forward, POU/loss, adjoint, tail
+    per_step = 1 + (4 if eng.cell_order else 0) + 2 + 4 + 2 + 4
     if rank == 0:
         line = {"metric": METRIC, "value": value, "unit": "steps/s", "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": ms_max, "higher_is_better": True, "scaling": "weak",
@@ -573,7 +573,7 @@ def run_fused(args, world, rank, local):
                            "grid": eng.launch_grid, "forward_grid": eng.forward_grid,
                            "autotuned": getattr(eng, "tuned", None),
                            "forward_kernel": "tcgen05 3xTF32" if eng.tensor_cores else "fp32 fma",
-                           "adjoint_kernel": "tcgen05 3xTF32 layer-2 recompute + fp32 fma" if eng.tc_adjoint
+                           "adjoint_kernel": "tcgen05 3xTF32 + mma.sync 3xTF32 weight gradient" if eng.tc_adjoint
                            else ("fp32 fma, layer-2 z-jets stored by the forward" if ps.zs is not None
                                  else "fp32 fma, layer 2 recomputed"),
                            "jet": "u, grad u, u_xx, u_yy" if args.per_dim_jets else "u, grad u, laplacian u",
@@ -718,11 +718,13 @@ def main():
     ap.add_argument("--forward-chunk", type=int, default=0, help="pairs per forward work item (0: 4 x --chunk)")
     ap.add_argument("--grid", type=int, default=0)
     ap.add_argument("--fma-forward", action="store_true", help="forward jets on the CUDA-core FMA kernel")
-    ap.add_argument("--tc-adjoint", action="store_true",
-                    help="adjoint with the layer-2 recompute on the tensor cores (fbp_adjoint_pairs_tc)")
+    ap.add_argument("--tc-adjoint", action="store_const", const=True, default=None,
+                    help="adjoint on the tensor cores (fbp_adjoint_pairs_tc; the default where it is compiled)")
+    ap.add_argument("--fma-adjoint", dest="tc_adjoint", action="store_const", const=False,
+                    help="adjoint on the CUDA-core FMA kernel")
     ap.add_argument("--store-z2", action="store_const", const=True, default=None,
                     help="the forward stores the layer-2 z-jets and the adjoint reads them instead of recomputing "
-                         "(default: only for hidden layers at least 32 wide, so not for this workload)")
+                         "(on the FMA kernel; default: not for this workload)")
     ap.add_argument("--no-cell-order", dest="cell_order", action="store_false",
                     help="keep each drawn batch in the sampler's order (default: Morton cell order)")
     ap.add_argument("--per-dim-jets", action="store_true",

@@ -36,6 +36,9 @@ import tempfile
 import torch
 
 CACHE_ENV = "FBPINNS_GB300_AUTOTUNE_CACHE"
+# part of the cache key; raised when the kernels or the candidates change so
+# that a choice stored for the old ones is measured again
+KERNELS = 2
 
 
 def cache_path():
@@ -57,7 +60,7 @@ def config_key(engine, n, pipelined):
     return "|".join(str(v) for v in (props.name, props.multi_processor_count, engine.layer_sizes, engine.activation,
                                      engine.d2mask, int(engine.tensor_cores), int(getattr(engine, "tc_adjoint", 0)),
                                      int(bool(getattr(engine, "z2_rows", 0))), int(bool(getattr(engine, "cell_order", 0))),
-                                     engine.m, int(n), int(bool(pipelined))))
+                                     engine.m, int(n), int(bool(pipelined)), f"k{KERNELS}"))
 
 
 def _load_cache(path):
@@ -85,10 +88,12 @@ def _store_cache(path, key, entry):
         return repr(ex)
 
 
-def default_candidates(s, m, sms):
+def default_candidates(s, m, sms, tc_sizes=()):
     """Around the pair-count heuristic (``engine.work_item_sizes`` with the
     requested 1024 / 4096): adjoint items of half, once and twice its size,
-    forward items of 1, 2 and 4 times the adjoint's (at most 8192)."""
+    forward items of 1, 2 and 4 times the adjoint's (at most 8192); then
+    ``tc_sizes``, each for both queues (the tensor-core kernels' own rule, whose
+    items are longer: their set-up per item is about two tiles)."""
     from .engine import work_item_sizes
     adj, _, _ = work_item_sizes(s, m, sms, 1024, 4096)
     out = []
@@ -96,7 +101,7 @@ def default_candidates(s, m, sms):
         for k in (1, 2, 4):
             if (a, min(a * k, 8192)) not in out:
                 out.append((a, min(a * k, 8192)))
-    return out
+    return out + [(t, t) for t in tc_sizes if (t, t) not in out]
 
 
 def _apply(engine, choice):
@@ -137,7 +142,13 @@ def tune_work_items(engine, x, caps=None, candidates=None, reps=3, use_cache=Tru
     probe = engine.points(x)
     s, n = probe.s, probe.n
     if candidates is None:
-        candidates = default_candidates(s, engine.m, engine.sm_count)
+        from .engine import tc_item_size
+        tc_sizes = ()
+        if engine.tc_adjoint:
+            # what a point set takes without the autotuner, and half of it
+            t = min(8192, tc_item_size(caps[0] if caps else s, engine.sm_count, caps is not None))
+            tc_sizes = (t, max(128, t // 256 * 128))
+        candidates = default_candidates(s, engine.m, engine.sm_count, tc_sizes)
     if pipelined and caps is None:
         caps = (int(probe.s * 1.25) + 1024, int(probe.u * 1.25) + 1024)
     del probe

@@ -336,6 +336,15 @@ def test_autotune_candidates_follow_the_pair_count():
     assert all(f <= 8192 and f >= a for a, f in default_candidates(10 ** 9, 4096, 152))
 
 
+def test_autotune_candidates_hold_the_tensor_core_sizes():
+    """The sizes of the tensor-core kernels' own rule come after the pair-count
+    ones, each once and for both queues."""
+    from fbpinns_gb300.autotune import default_candidates
+    base = default_candidates(314_672, 128, 152)
+    assert default_candidates(314_672, 128, 152, (768, 384)) == base + [(768, 768), (384, 384)]
+    assert (256, 256) in base and default_candidates(314_672, 128, 152, (256, 256)) == base
+
+
 def test_constrained_jets_identity_and_needed_components():
     """constrained_jets (the jets of constraining_fn(u) for the generic step):
     exact against closed forms for the HO hard-constraint ansatz
