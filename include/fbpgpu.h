@@ -341,9 +341,9 @@ int fbp_forward_pairs(const fbp_net* net, const float* x, const fbp_pairs* pairs
 
 /* Same records as fbp_forward_pairs, with layer 2 of every jet component on
  * the 5th-generation tensor cores (tcgen05, TF32 operands split hi + lo, three
- * products, FP32 accumulation in tensor memory).  Compiled for xd = 2 with two
- * 16-wide hidden layers only (FBP_ERR_UNSUPPORTED otherwise; see
- * fbp_has_tc_shape for the jet masks and activations).  A kernel that
+ * products, FP32 accumulation in tensor memory).  Compiled for two hidden
+ * layers of 16 or 32 neurons and the dimensions, jet masks and activations
+ * that fbp_has_tc_shape knows (FBP_ERR_UNSUPPORTED otherwise).  A kernel that
  * times out waiting for its MMAs sets FBP_STATUS_TC_TIMEOUT in *status and
  * leaves its remaining pairs unwritten.  Same reference functions as
  * fbp_forward_pairs. */
@@ -409,12 +409,13 @@ int fbp_loss_finalize(const double* loss_part, int32_t n_part, double scale,
 int fbp_adjoint_pairs(const fbp_net* net, const float* x, const fbp_pairs* pairs,
                       const float* slot_out, float* grad_part, int32_t grid, void* stream);
 
-/* fbp_adjoint_pairs with the layer-2 recompute on the tensor cores: per tile
- * of 128 pairs the jets z_c = W2 v_c of the forward are J tcgen05 GEMMs
- * (TF32 operands split hi + lo, three products, FP32 accumulation in TMEM),
- * and the CUDA cores run the rest of the adjoint.  tanh networks xd-16-16-1
- * (fbp_has_tc_adjoint_shape); the same gradient partials up to FP32
- * rounding.  Bounded waits as fbp_forward_pairs_tc (FBP_STATUS_TC_TIMEOUT in
+/* fbp_adjoint_pairs with its layer-2 contractions on the tensor cores: per
+ * tile of 128 pairs the jets z_c = W2 v_c and the transposed products with
+ * their adjoints are tcgen05 GEMMs (TF32 operands split hi + lo, three
+ * products, FP32 accumulation in TMEM), and the sums over the pairs are
+ * warp-level MMAs of the same split.  Two hidden layers of 16 or 32 neurons,
+ * tanh, sin or adaptive (fbp_has_tc_adjoint_shape); the same gradient partials
+ * up to FP32 rounding; fbp_pairs.zs is not read.  Bounded waits as fbp_forward_pairs_tc (FBP_STATUS_TC_TIMEOUT in
  * *status; FBP_STATUS_TC_TEST_NO_MMA exercises that path).
  * Replaces XLA's reverse-mode transpose of the model (fbpinns/trainers.py:292). */
 int fbp_adjoint_pairs_tc(const fbp_net* net, const float* x, const fbp_pairs* pairs,
