@@ -57,6 +57,8 @@ struct TcAdj {
     static constexpr int NPT = H / 8;      // threads per pair
     static constexpr int T = 128 * NPT;    // threads per CTA
     static constexpr int NW = T / 32;
+    // the first second-derivative slot sums more than one dim
+    static constexpr bool SUMS = NS > 0 && (C::slot_dims(0) & (C::slot_dims(0) - 1)) != 0;
     static constexpr int NA = NS > 0 ? 3 : 2;  // A operands a, tp (, tpp); also the GEMM 2 groups
     static constexpr int OP = 2 * H;           // TMEM columns of an operand: hi, lo
     // TMEM columns: [A operands | z | (z2bar operands past the NA-th) | T].  z2bar
@@ -362,9 +364,13 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
 #pragma unroll
                 for (int c = 0; c < J; ++c) ob[c] = T.xo[buf][XD + c][r];
                 if (h == 0) g3b += ob[0];
-                // eight neurons at a time, or four where z's columns are taken by z2bar:
-                // that wait for every thread's z would keep all J x 8 in registers
-                constexpr int NH = A::OVER ? 4 : 8;
+                // eight neurons at a time, or four, with z2bar split for TMEM from its row
+                // afterwards, where z's columns are taken by z2bar (that wait for every
+                // thread's z would keep all J x 8 in registers) and where a slot sums
+                // several dims (its z_d^2 and P take registers too).  Steps in us, eight
+                // and four: Laplacian jets, Helmholtz 8452 8399, SIREN 528 522, Poisson
+                // of 16381 points 119 117.5; u_xx alone, Burgers 69.0 69.8
+                constexpr int NH = A::OVER || A::SUMS ? 4 : 8;
 #pragma unroll
                 for (int half = 0; half < 8 / NH; ++half) {
                     float acc[J][NH];
@@ -437,6 +443,8 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
                     tc_fence_before();
                     __syncthreads();  // every thread has read its z
                     tc_fence_after();
+                }
+                if constexpr (NH == 4) {
 #pragma unroll
                     for (int c = 0; c < J; ++c) {  // this thread's own row
                         const float4 u = *reinterpret_cast<const float4*>(zrow + c * H);
