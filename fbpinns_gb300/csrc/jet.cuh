@@ -147,11 +147,13 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
 
-// sin and cos of two values: x - j pi/2 with pi/2 in three parts (Cody and
-// Waite), then their Taylor polynomials to r^9 and r^10 on [-pi/4, pi/4]
-// (remainders below 2e-9 and 2e-10), exchanged and negated by the quadrant j
-// mod 4.  Arguments beyond 1e4 (and NaN) take sincosf.  On neurons in pairs
-// about a third of the instructions of two sincosf calls.
+// sin and cos of two values: x - j pi/2 with pi/2 as the sum of three floats,
+// each the remainder rounded (Cody and Waite), then their Taylor polynomials to
+// r^9 and r^10 on [-pi/4, pi/4] (remainders below 2e-9 and 2e-10), exchanged and
+// negated by the quadrant j mod 4.  Arguments beyond 1e4 (and NaN) take sincosf.
+// On neurons in pairs about a third of the instructions of two sincosf calls.
+// (One at a time in the FMA kernels it loses to sincosf: FourierFCN 2-16-32-1
+// on 2^18 points 7.05 -> 7.34 ms a step.)
 __device__ __forceinline__ void sincos2(float2 x, float2& sn, float2& cs) {
     if (!(fmaxf(fabsf(x.x), fabsf(x.y)) <= 1e4f)) {
         sincosf(x.x, &sn.x, &cs.x);
