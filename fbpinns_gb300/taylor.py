@@ -10,6 +10,11 @@ direction gives.  The jvp's ops on zero tangents go through Python meta
 kernels, about 0.3 ms each: 72 ms a step for the wave equation's constraint,
 where the rules take 4.  A call without a rule raises ``NoRule`` and the
 caller uses the jvp.
+
+A ``Jet`` holds no data of its own, so whatever reaches past the rules (vmap,
+torch.func, TorchScript, C++ extensions) has nothing to compute on and ends up
+in ``Jet.__torch_dispatch__``, which refuses as well; a refusal that the
+function or TorchScript turns into something else is still on the trace.
 """
 
 import torch
@@ -183,29 +188,67 @@ PLAIN = {getattr(T, k).__get__ for k in ("shape", "dtype", "device", "ndim", "is
      torch.zeros_like, torch.ones_like, T.new_zeros, T.new_ones}
 
 
+class _Trace:
+    """One evaluation of a function on Jets: whether it made a call that has no rule."""
+
+    def __init__(self):
+        self.refused = False
+
+    def refuse(self):
+        self.refused = True
+        raise NoRule
+
+
+def _trace_in(args):
+    """The trace of a Jet among the arguments (nested ones too), or None."""
+    for a in args.values() if isinstance(args, dict) else args:
+        t = a.trace if isinstance(a, Jet) else _trace_in(a) if isinstance(a, (tuple, list, dict)) else None
+        if t is not None:
+            return t
+    return None
+
+
+def _refuse(*args):
+    t = _trace_in(args)
+    if t is not None:
+        t.refuse()
+    raise NoRule
+
+
 class Jet(torch.Tensor):
     """A tensor with derivative stacks; made by ``Jet.make``."""
 
     @staticmethod
-    def make(v, d, dd):
-        j = v.as_subclass(Jet)
-        j.__dict__.update(v=v, d=d, dd=dd)
+    def make(v, d, dd, trace=None):
+        j = torch.Tensor._make_wrapper_subclass(Jet, v.shape, dtype=v.dtype, device=v.device)
+        j.__dict__.update(v=v, d=d, dd=dd, trace=trace)
         return j
 
     @classmethod
+    def __torch_dispatch__(cls, func, types, args=(), kwargs=None):
+        _refuse(args, kwargs or {})
+
+    @classmethod
     def __torch_function__(cls, func, types, args=(), kwargs=None):
-        if not all(t in (Jet, torch.Tensor, torch.nn.Parameter) for t in types):
-            raise NoRule
+        kwargs = kwargs or {}
+        trace = _trace_in(args) or _trace_in(kwargs)
+        if trace is None or not all(t in (Jet, torch.Tensor, torch.nn.Parameter) for t in types):
+            _refuse(args, kwargs)
         with torch._C.DisableTorchFunctionSubclass():
             if func in PLAIN:
-                return func(*(a.v if isinstance(a, Jet) else a for a in args), **(kwargs or {}))
+                return func(*(a.v if isinstance(a, Jet) else a for a in args), **kwargs)
             rule = RULES.get(func)
             if rule is None:
-                raise NoRule
+                trace.refuse()
             try:
-                return rule(*args, **(kwargs or {}))
-            except (TypeError, AttributeError) as e:  # an argument that the rule does not take (alpha=, out=, dtype=)
-                raise NoRule from e
+                out = rule(*args, **kwargs)
+            except NoRule:
+                trace.refuse()
+            except (TypeError, AttributeError):  # an argument that the rule does not take (alpha=, out=, dtype=)
+                trace.refuse()
+            if isinstance(out, Jet):
+                out.trace = trace
+            return out
 
 
 def jets(fn, x, dims, u, ud, udd):
@@ -216,8 +259,14 @@ def jets(fn, x, dims, u, ud, udd):
     e = torch.zeros((len(dims), 1, x.shape[1]), dtype=x.dtype, device=x.device)
     for i, d in enumerate(dims):
         e[i, 0, d] = 1.0
-    uj = Jet.make(u, ud, udd)
-    y = fn(Jet.make(x, e.expand(-1, x.shape[0], -1), None), uj)
-    if not isinstance(y, torch.Tensor) or y.dtype != u.dtype:
+    trace = _Trace()
+    uj = Jet.make(u, ud, udd, trace)
+    try:
+        y = fn(Jet.make(x, e.expand(-1, x.shape[0], -1), None, trace), uj)
+    except Exception:
+        if trace.refused:  # what TorchScript makes of a refusal, or fn's answer to one
+            raise NoRule from None
+        raise
+    if trace.refused or not isinstance(y, torch.Tensor) or y.dtype != u.dtype:
         raise NoRule
     return (y is uj,) + ((y.v, y.d, y.dd) if isinstance(y, Jet) else (y, None, None))

@@ -7,6 +7,7 @@ import math
 import numpy as np
 import pytest
 import torch
+import torch.utils.checkpoint
 
 from fbpinns_gb300 import engine, problems as PR, taylor
 
@@ -83,3 +84,100 @@ def test_every_builtin_constraint_has_rules():
         z = torch.zeros((xd, 5, 1), dtype=torch.float64)
         _, _, d, dd = taylor.jets(lambda a, b: fn(p, a, b), x, list(range(xd)), x[:, 0:1] * 1, z + 1, z)
         assert d.shape == dd.shape == (xd, 5, 1) and torch.isfinite(d).all() and math.isfinite(dd.sum().item())
+
+
+@torch.jit.script
+def _scripted(x, u):
+    return torch.tanh(x[:, 0:1]) * u
+
+
+_traced = torch.jit.trace(lambda x, u: torch.tanh(x[:, 0:1]) * u, (W[:, :2], W[:, :1]))
+
+
+def _caught(x, u):
+    try:
+        return torch.atan(x[:, 0:1]) * u
+    except BaseException:
+        return 0 * u
+
+
+_T = torch.func
+PAST_THE_RULES = {  # calls that do not come (only) through __torch_function__
+    "vmap": lambda p, x, u: torch.vmap(lambda a, b: torch.tanh(a[0:1]) * b)(x, u),
+    "vmap_closure": lambda p, x, u: torch.vmap(lambda b: b * 2)(u) * torch.tanh(x[:, 0:1]),
+    "script": lambda p, x, u: _scripted(x, u),
+    "trace": lambda p, x, u: _traced(x, u),
+    "func_vjp": lambda p, x, u: _T.vjp(lambda a: a * a * x[:, 0:1], u)[1](torch.ones_like(u))[0] * u,
+    "func_vjp_value": lambda p, x, u: _T.vjp(lambda a: a * a, u)[0] * x[:, 0:1],
+    "func_grad": lambda p, x, u: _T.grad(lambda a: (a * a * a).sum())(u) * x[:, 0:1],
+    "func_grad_closure": lambda p, x, u: _T.grad(lambda a: (a * x[:, 0:1]).sum())(torch.zeros_like(u)) * u,
+    "func_jvp": lambda p, x, u: _T.jvp(lambda a: a * a, (u,), (torch.ones_like(u),))[1] * x[:, 0:1],
+    "caught": lambda p, x, u: _caught(x, u),
+}
+
+
+def _jets_and_grad(fn, x, U, d2, seed, grad=True):
+    with torch.set_grad_enabled(grad):
+        y = engine.constrained_jets(fn, None, x, U, x.shape[1], d2)
+    assert y.requires_grad or not grad
+    return y.detach(), torch.autograd.grad((y * seed).sum(), U)[0] if grad else None
+
+
+@pytest.mark.parametrize("grad", [True, False])
+@pytest.mark.parametrize("name", sorted(PAST_THE_RULES))
+def test_constraints_that_reach_past_the_rules(name, grad, monkeypatch):
+    """Jets and gradient are those of the nested jvp, with gradients on and off."""
+    fn, (x, U, seed) = PAST_THE_RULES[name], _xu()
+    y, dy = _jets_and_grad(fn, x, U, 3, seed, grad)
+    with monkeypatch.context() as m:
+        m.setattr(taylor, "RULES", {})
+        m.setattr(taylor, "PLAIN", set())
+        ref, dref = _jets_and_grad(fn, x, U, 3, seed, grad)
+    assert ref[:, 1:].abs().max() > 0.1
+    torch.testing.assert_close(y, ref, rtol=1e-11, atol=1e-11)
+    if grad:
+        torch.testing.assert_close(dy, dref, rtol=1e-11, atol=1e-11)
+
+
+def _xu():
+    g = torch.Generator().manual_seed(3)
+    return (torch.rand((17, 2), generator=g, dtype=torch.float64),
+            torch.randn((17, 5), generator=g, dtype=torch.float64, requires_grad=True),
+            torch.randn((17, 5), generator=g, dtype=torch.float64))
+
+
+@pytest.mark.parametrize("outer", ["vmap", "grad", "jvp", "dual", "hooks", "checkpoint"])
+def test_jets_under_outer_transforms(outer):
+    """constrained_jets itself inside a transform gives what it gives outside."""
+    fn = CASES["rules"][2]
+    p = torch.zeros((17, 1), dtype=torch.float64)
+    x, U, seed = _xu()
+
+    def jets(V):
+        return engine.constrained_jets(fn, p, x, V, 2, 3)
+
+    y, dy = jets(U).detach(), torch.autograd.grad((jets(U) * seed).sum(), U)[0]
+    V = U.detach()
+    if outer == "vmap":
+        got, want = torch.vmap(jets)(torch.stack([V, 2 * V])), torch.stack([y, jets(2 * V)])
+    elif outer == "grad":
+        got, want = _T.grad(lambda v: (jets(v) * seed).sum())(V), dy
+    elif outer == "jvp":
+        got, want = (_T.jvp(jets, (V,), (seed,))[1] * seed).sum(), None
+    elif outer == "dual":
+        with torch.autograd.forward_ad.dual_level():
+            t = torch.autograd.forward_ad.unpack_dual(jets(torch.autograd.forward_ad.make_dual(V, seed))).tangent
+        got, want = (t * seed).sum(), None
+    elif outer == "hooks":
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t.clone(), lambda t: t):
+            z = jets(U)
+        got, want = torch.autograd.grad((z * seed).sum(), U)[0], dy
+    else:
+        z = torch.utils.checkpoint.checkpoint(jets, U, use_reentrant=False)
+        got, want = torch.autograd.grad((z * seed).sum(), U)[0], dy
+    if want is None:  # seed . J seed from the reverse mode
+        W2 = U.detach().requires_grad_(True)
+        h = torch.zeros_like(y, requires_grad=True)
+        g, = torch.autograd.grad((jets(W2) * h).sum(), W2, create_graph=True)
+        want = (torch.autograd.grad((g * seed).sum(), h)[0] * seed).sum()
+    torch.testing.assert_close(got, want, rtol=1e-11, atol=1e-11)
