@@ -189,14 +189,20 @@ PLAIN = {getattr(T, k).__get__ for k in ("shape", "dtype", "device", "ndim", "is
 
 
 class _Trace:
-    """One evaluation of a function on Jets: whether it made a call that has no rule."""
+    """One evaluation of a function on Jets: the grad mode that it began in, and
+    whether it made a call that has no rule."""
 
     def __init__(self):
-        self.refused = False
+        self.grad, self.refused = torch.is_grad_enabled(), False
 
     def refuse(self):
         self.refused = True
         raise NoRule
+
+    def same_modes(self):
+        """False inside a custom autograd.Function (which turns forward mode off,
+        and its own derivatives are then wanted) and under another grad mode."""
+        return torch.is_grad_enabled() == self.grad and torch._C._is_fwd_grad_enabled()
 
 
 def _trace_in(args):
@@ -232,7 +238,8 @@ class Jet(torch.Tensor):
     def __torch_function__(cls, func, types, args=(), kwargs=None):
         kwargs = kwargs or {}
         trace = _trace_in(args) or _trace_in(kwargs)
-        if trace is None or not all(t in (Jet, torch.Tensor, torch.nn.Parameter) for t in types):
+        if trace is None or not trace.same_modes() or \
+                not all(t in (Jet, torch.Tensor, torch.nn.Parameter) for t in types):
             _refuse(args, kwargs)
         with torch._C.DisableTorchFunctionSubclass():
             if func in PLAIN:
@@ -260,6 +267,8 @@ def jets(fn, x, dims, u, ud, udd):
     for i, d in enumerate(dims):
         e[i, 0, d] = 1.0
     trace = _Trace()
+    if not trace.same_modes():
+        raise NoRule
     uj = Jet.make(u, ud, udd, trace)
     try:
         y = fn(Jet.make(x, e.expand(-1, x.shape[0], -1), None, trace), uj)

@@ -86,6 +86,47 @@ def test_every_builtin_constraint_has_rules():
         assert d.shape == dd.shape == (xd, 5, 1) and torch.isfinite(d).all() and math.isfinite(dd.sum().item())
 
 
+class _Square(torch.autograd.Function):
+    """u^2 with its own derivatives, usable under torch.func."""
+
+    @staticmethod
+    def forward(u):
+        return u * u
+
+    @staticmethod
+    def setup_context(ctx, inputs, output):
+        ctx.save_for_backward(*inputs)
+        ctx.save_for_forward(*inputs)
+
+    @staticmethod
+    def backward(ctx, g):
+        return 2 * ctx.saved_tensors[0] * g
+
+    @staticmethod
+    def jvp(ctx, t):
+        return 2 * ctx.saved_tensors[0] * t
+
+
+class _Through(torch.autograd.Function):
+    """Returns its input, with another derivative than the identity's."""
+
+    @staticmethod
+    def forward(u):
+        return u
+
+    @staticmethod
+    def setup_context(ctx, inputs, output):
+        pass
+
+    @staticmethod
+    def backward(ctx, g):
+        return 3 * g
+
+    @staticmethod
+    def jvp(ctx, t):
+        return 3 * t
+
+
 @torch.jit.script
 def _scripted(x, u):
     return torch.tanh(x[:, 0:1]) * u
@@ -101,6 +142,12 @@ def _caught(x, u):
         return 0 * u
 
 
+def _partly_no_grad(x, u):
+    with torch.no_grad():
+        a = torch.tanh(x[:, 0:1]) * u
+    return a + u * x[:, 0:1]
+
+
 _T = torch.func
 PAST_THE_RULES = {  # calls that do not come (only) through __torch_function__
     "vmap": lambda p, x, u: torch.vmap(lambda a, b: torch.tanh(a[0:1]) * b)(x, u),
@@ -112,7 +159,12 @@ PAST_THE_RULES = {  # calls that do not come (only) through __torch_function__
     "func_grad": lambda p, x, u: _T.grad(lambda a: (a * a * a).sum())(u) * x[:, 0:1],
     "func_grad_closure": lambda p, x, u: _T.grad(lambda a: (a * x[:, 0:1]).sum())(torch.zeros_like(u)) * u,
     "func_jvp": lambda p, x, u: _T.jvp(lambda a: a * a, (u,), (torch.ones_like(u),))[1] * x[:, 0:1],
+    "function": lambda p, x, u: _Square.apply(u) * x[:, 0:1],
+    "function_and_u": lambda p, x, u: _Square.apply(u) * x[:, 0:1] + u,
+    "function_through": lambda p, x, u: _Through.apply(u) * x[:, 0:1],
+    "function_through_alone": lambda p, x, u: _Through.apply(u),
     "caught": lambda p, x, u: _caught(x, u),
+    "partly_no_grad": lambda p, x, u: _partly_no_grad(x, u),
 }
 
 
