@@ -121,7 +121,20 @@ def _div(a, b):
         w = v / b
         return Jet.make(w, _full(None if d is None else _pad(d, w.dim()) / b, w),
                         _full(None if dd is None else _pad(dd, w.dim()) / b, w))
-    return _times(a, _reciprocal(b))
+    # from w v = u: the quotient itself, not u (1 / v), which overflows where v is
+    # tiny and rounds twice
+    (u, ud, udd), (v, vd, vdd) = _parts(a), _parts(b)
+    w = u / v
+    n = w.dim()
+
+    def over_v(s):
+        return None if s is None else _full(_pad(s, n) / v, w)
+
+    def minus(s, t):
+        return _sum(None if s is None else _pad(s, n), None if t is None else -t)
+    d = over_v(minus(ud, _mul(vd, w, n)))
+    cross = None if d is None or vd is None else 2.0 * (d * _pad(vd, n))
+    return Jet.make(w, d, over_v(minus(udd, _sum(cross, _mul(vdd, w, n)))))
 
 
 def _pow(a, p):

@@ -233,3 +233,30 @@ def test_jets_under_outer_transforms(outer):
         g, = torch.autograd.grad((jets(W2) * h).sum(), W2, create_graph=True)
         want = (torch.autograd.grad((g * seed).sum(), h)[0] * seed).sum()
     torch.testing.assert_close(got, want, rtol=1e-11, atol=1e-11)
+
+
+def test_quotient_of_jets_where_the_reciprocal_overflows():
+    """u / v of jets with v below the reciprocal of the largest number: the
+    value and the derivatives along u of the direct quotient."""
+    x, U, _ = _xu()
+    U = U.detach()[:, :4]
+    s = 2.0 ** -1040
+
+    def fn(p, x, u):
+        return (u * s) / (torch.exp(x[:, 1:2]) * s)
+    y = engine.constrained_jets(fn, None, x, U, 2, 1)
+    u, v = U[:, 0] * s, torch.exp(x[:, 1]) * s
+    assert torch.equal(y[:, 0], u / v) and torch.isfinite(y).all()
+    torch.testing.assert_close(y[:, 1], (U[:, 1] * s) / v, rtol=1e-9, atol=0)
+
+
+def _quotient(p, x, u):
+    return (u * (x[:, 0:1] + 1)) / (x[:, 1:2] * 3 + 1)
+
+
+def test_quotient_of_jets_rounds_once():
+    """The value in float32 is the one that the function itself gives."""
+    x, U, _ = _xu()
+    x, U = x.float(), U.detach().float()[:, :4]
+    y = engine.constrained_jets(_quotient, None, x, U, 2, 1)
+    assert torch.equal(y[:, 0:1], _quotient(None, x, U[:, 0:1]))
