@@ -139,7 +139,8 @@ def _div(a, b):
 
 def _pow(a, p):
     """a ** p for an integer p >= 1 (other powers: the jvp)."""
-    if not isinstance(a, Jet) or isinstance(p, bool) or not isinstance(p, (int, float)) or p != int(p) or p < 1:
+    if not isinstance(a, Jet) or isinstance(p, bool) or not isinstance(p, (int, float)) or not 1 <= p < 2 ** 31 \
+            or p != int(p):
         raise NoRule
     p = int(p)
     if p == 1:
@@ -165,9 +166,10 @@ def _reduce(a, dim=None, keepdim=False):
     if dim is None or not isinstance(a, Jet):
         raise NoRule
     dims = dim if isinstance(dim, (tuple, list)) else (dim,)
-    if not dims or not all(type(i) is int for i in dims):
+    n = a.v.dim()
+    if not dims or not all(type(i) is int and -n <= i < n for i in dims):
         raise NoRule
-    dims = [i % a.v.dim() if a.v.dim() else 0 for i in dims]
+    dims = [i % n for i in dims]
     up = [i + 1 for i in dims]
     return Jet.make(a.v.sum(dims, keepdim=keepdim), None if a.d is None else a.d.sum(up, keepdim=keepdim),
                     None if a.dd is None else a.dd.sum(up, keepdim=keepdim))

@@ -260,3 +260,24 @@ def test_quotient_of_jets_rounds_once():
     x, U = x.float(), U.detach().float()[:, :4]
     y = engine.constrained_jets(_quotient, None, x, U, 2, 1)
     assert torch.equal(y[:, 0:1], _quotient(None, x, U[:, 0:1]))
+
+
+@pytest.mark.parametrize("call", [lambda x, u: (x * u).sum(2, keepdim=True), lambda x, u: (x * u).sum((0, -3))[:, None],
+                                  lambda x, u: torch.sum(x * u, (1, -1), keepdim=True)])
+def test_wrong_dims_of_a_sum_are_refused(call):
+    """As the plain call does: an IndexError out of range, a RuntimeError for a dim given twice."""
+    x, U, _ = _xu()
+    with pytest.raises((IndexError, RuntimeError)) as plain:
+        call(x, U[:, 0:1])
+    with pytest.raises(plain.type):
+        engine.constrained_jets(lambda p, x, u: call(x, u) * u, None, x, U, 2, 3)
+
+
+@pytest.mark.parametrize("p", [float("inf"), 2.0 ** 40])
+def test_powers_beyond_the_rule_go_to_the_jvp(p, monkeypatch):
+    x, U, _ = _xu()
+    y = engine.constrained_jets(lambda q, x, u: u + torch.tanh(x[:, 0:1]) ** p, None, x, U, 2, 3)
+    with monkeypatch.context() as m:
+        m.setattr(taylor, "RULES", {})
+        ref = engine.constrained_jets(lambda q, x, u: u + torch.tanh(x[:, 0:1]) ** p, None, x, U, 2, 3)
+    torch.testing.assert_close(y, ref, rtol=1e-11, atol=1e-11, equal_nan=True)
