@@ -892,6 +892,27 @@ struct XDispatch;
     X(1, 0) X(1, 1) X(2, 0) X(2, 1) X(2, 2) X(2, 3) X(2, 11) X(3, 0) X(3, 1) X(3, 2) X(3, 3) X(3, 4) X(3, 5) X(3, 6) \
         X(3, 7) X(3, 55)
 
+// Dims that a problem kind's ansatz and residual are written for (0: any); both
+// leave zeros at any other number.
+static int problem_dims(int kind) {
+    switch (kind) {
+        case FBP_PROBLEM_HO_HARDBC: return 1;
+        case FBP_PROBLEM_BURGERS:
+        case FBP_PROBLEM_POISSON2D:
+        case FBP_PROBLEM_HELMHOLTZ2D: return 2;
+        case FBP_PROBLEM_WAVE_C: return 3;
+        default: return 0;
+    }
+}
+
+static int check_problem(const char* what, const fbp_problem* prob, int32_t xd) {
+    const int dims = problem_dims(prob->kind);
+    FBP_REQUIRE(dims == 0 || dims == xd, FBP_ERR_UNSUPPORTED, "%s: problem kind %d is for xd=%d, not %d", what,
+                prob->kind, dims, xd);
+    FBP_REQUIRE(prob->ng == 0 || prob->gauss, FBP_ERR_INVALID, "%s: null gaussians", what);
+    return FBP_OK;
+}
+
 static int grid_pts(int64_t n) {
     int64_t b = (n + POU_T - 1) / POU_T;
     const int64_t cap = (int64_t)sm_count() * 8;
@@ -926,7 +947,7 @@ extern "C" int fbp_pou_solution(int32_t xd, int32_t d2mask, const fbp_problem* p
                                 float* out, int64_t s_cap, int32_t* status, void* stream) {
     FBP_REQUIRE(prob && pt_off && out && status && npou > 0 && (x || n == 0), FBP_ERR_INVALID,
                 "fbp_pou_solution: bad args");
-    FBP_REQUIRE(prob->ng == 0 || prob->gauss, FBP_ERR_INVALID, "fbp_pou_solution: null gaussians");
+    if (const int rc = check_problem("fbp_pou_solution", prob, xd)) return rc;
     if (n == 0) return FBP_OK;
     cudaStream_t st = as_stream(stream);
     // 64 threads per CTA: the 10^4 points of a test grid reach every SM
@@ -967,8 +988,8 @@ extern "C" int fbp_pou_loss(int32_t xd, int32_t d2mask, const fbp_problem* prob,
                             double* loss_part, int32_t n_part, int32_t* status, void* stream) {
     FBP_REQUIRE(prob && x && pt_off && np_off && loss_part && status && npou > 0, FBP_ERR_INVALID,
                 "fbp_pou_loss: bad args");
+    if (const int rc = check_problem("fbp_pou_loss", prob, xd)) return rc;
     FBP_REQUIRE(n > 0, FBP_ERR_INVALID, "fbp_pou_loss: no points");
-    FBP_REQUIRE(prob->ng == 0 || prob->gauss, FBP_ERR_INVALID, "fbp_pou_loss: null gaussians");
     // CTAs of POU_WARPS warps, each warp 32 points at a time
     const int64_t ctas = ((n + 31) / 32 + POU_WARPS - 1) / POU_WARPS;
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>(ctas, (int64_t)sm_count() * 8));

@@ -382,18 +382,22 @@ class Helmholtz2D(Problem):
                 "d2_group": 3}  # the residual needs only u_xx + u_yy
 
 
-# the constraining functions that the kernels evaluate, by the function itself:
-# a subclass that keeps one is in, one that replaces it is not
-_ANSATZ = {k.constraining_fn: k for k in (HarmonicOscillator1DHardBC, BurgersEquation2D, WaveEquationConstantVelocity3D,
-                                          Poisson2D, Helmholtz2D)}
+# the constraining functions that the kernels evaluate, by the function itself (a
+# subclass that keeps one is in, one that replaces it is not), with the number of
+# dims that the kernels have each for
+_ANSATZ = {k.constraining_fn: (k, xd) for k, xd in (
+    (HarmonicOscillator1DHardBC, 1), (BurgersEquation2D, 2), (WaveEquationConstantVelocity3D, 3), (Poisson2D, 2),
+    (Helmholtz2D, 2))}
 
 
-def ansatz_spec(problem, all_params):
-    """fused_spec whose ansatz is problem.constraining_fn, or None where the
-    kernels have none (or its parameters are on a GPU, where reading them
-    would wait for it)."""
-    k = _ANSATZ.get(problem.constraining_fn)
-    if k is None:
+def ansatz_spec(problem, all_params, xd=None):
+    """fused_spec whose ansatz is problem.constraining_fn at points of xd dims
+    (None: as many as the problem's own), or None where the kernels have none:
+    the functions read their first columns only, so a problem with a parameter
+    as a further input dim can keep one, which the kernels cannot evaluate there
+    (or the parameters are on a GPU, where reading them would wait for it)."""
+    k, dims = next((v for f, v in _ANSATZ.items() if f is problem.constraining_fn), (None, None))
+    if k is None or xd not in (None, dims):
         return None
     p = all_params["static"]["problem"]
     if any(torch.is_tensor(v) and v.is_cuda for v in p.values()):

@@ -632,7 +632,7 @@ class FBPINNTrainer:
             setattr(eng, key, (x, ps))
         ps = getattr(eng, key)[1]
         with torch.no_grad():
-            spec = ansatz_spec(problem, all_params)
+            spec = ansatz_spec(problem, all_params, eng.xd)
             if spec is not None:
                 return eng.solution(ps, spec)
             eng.forward_pairs(ps, z2=False)
