@@ -399,13 +399,16 @@ def ansatz_spec(problem, all_params, xd=None):
     k, dims = next((v for f, v in _ANSATZ.items() if f is problem.constraining_fn), (None, None))
     if k is None or xd not in (None, dims):
         return None
-    p = all_params["static"]["problem"]
-    if any(torch.is_tensor(v) and v.is_cuda for v in p.values()):
-        return None
     try:
+        if any(torch.is_tensor(v) and v.is_cuda for v in all_params["static"]["problem"].values()):
+            return None
         spec = k.fused_spec(all_params)
-    except (KeyError, TypeError, ValueError, AttributeError):  # parameters that only the residual needs
+        # as the kernels take them: numbers, and a table of Gaussians of four columns
+        spec["p"] = [float(v) for v in spec["p"]]
+        spec["n_int"] = 0  # the residual's, as is Helmholtz's table
+        spec["gauss"] = torch.as_tensor(spec["gauss"], dtype=torch.float32) if spec["kind"] == _lib.PROBLEM_WAVE_C else None
+    except Exception:  # arrays, or parameters that only the residual needs: constraining_fn takes what it can use
         return None
-    if spec["kind"] != _lib.PROBLEM_WAVE_C:
-        spec["gauss"] = None  # the residual's
+    if spec["gauss"] is not None and (spec["gauss"].dim() != 2 or spec["gauss"].shape[1] != 4):
+        return None
     return spec
