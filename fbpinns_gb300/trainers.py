@@ -623,21 +623,31 @@ class FBPINNTrainer:
 
     @staticmethod
     def predict(eng, all_params, problem, x):
-        """FBPINN solution at points x with all subdomains (the test-step inference)."""
+        """FBPINN solution at points x with all subdomains (the test-step inference).
+
+        The interaction lists of the last points are kept, with a copy of those
+        points (the caller may write to x between calls), and used again for
+        points of the same values."""
         x = torch.as_tensor(x, dtype=torch.float32).to(eng.device)
-        key = "_test_points"
-        cache = getattr(eng, key, None)
-        if cache is None or cache[0] is not x and not torch.equal(cache[0], x):
-            ps = eng.points(x)
-            setattr(eng, key, (x, ps))
-        ps = getattr(eng, key)[1]
         with torch.no_grad():
             spec = ansatz_spec(problem, all_params, eng.xd)
-            if spec is not None:
-                return eng.solution(ps, spec)
-            eng.forward_pairs(ps, z2=False)
-            U = eng.pou_forward(ps)
-            return problem.constraining_fn(all_params, x, U[:, 0:1])
+
+            def solution(ps):
+                if spec is not None:
+                    return eng.solution(ps, spec)
+                eng.forward_pairs(ps, z2=False)
+                U = eng.pou_forward(ps)
+                return problem.constraining_fn(all_params, ps.x, U[:, 0:1])
+
+            ps = getattr(eng, "_test_points", None)
+            if ps is not None and ps.x.shape == x.shape:
+                # compared on the device; read after the launches, which do not wait for it
+                same = (ps.x == x).all()
+                u = solution(ps)
+                if same.item():
+                    return u
+            eng._test_points = eng.points(x.clone())
+            return solution(eng._test_points)
 
 
 class PINNTrainer(FBPINNTrainer):

@@ -558,3 +558,53 @@ def test_helmholtz_reference_field_convergence():
     assert e[1] < 1e-3 and 3.5 < e[0] / e[1] < 4.5, e
     r = diffs(40 * math.pi, (200, 400, 800))
     assert min(r) > 0.3, r
+
+
+class _FakeEngine:
+    """The parts of an engine that predict uses, on the CPU: lists of the points
+    that points() was called with, a solution that tells which these were."""
+
+    device, xd = "cpu", 2
+
+    def __init__(self):
+        self.built = 0
+
+    def points(self, x):
+        from types import SimpleNamespace
+        self.built += 1
+        return SimpleNamespace(x=x, lists=x.clone())
+
+    def forward_pairs(self, ps, z2=True):
+        pass
+
+    def pou_forward(self, ps):
+        return ps.lists.sum(1, keepdim=True)
+
+
+def test_predict_follows_points_written_in_place():
+    """Points that the caller writes to between calls (through torch, or a
+    pointer, which leaves no version) get lists of their own; points of the
+    same values keep theirs."""
+    from fbpinns_gb300.problems import Problem
+    from fbpinns_gb300.trainers import FBPINNTrainer
+
+    class Own(Problem):
+        @staticmethod
+        def constraining_fn(all_params, x_batch, u):
+            return u + 10 * x_batch[:, 0:1]
+
+    def check(x, built):
+        u = FBPINNTrainer.predict(eng, {"static": {"problem": {}}}, Own, x)
+        assert torch.equal(u, x.sum(1, keepdim=True) + 10 * x[:, 0:1]) and eng.built == built
+
+    eng = _FakeEngine()
+    x = torch.rand((7, 2))
+    check(x, 1)
+    check(x, 1)
+    check(x.clone(), 1)
+    x.add_(1)
+    check(x, 2)
+    x.numpy()[3, 1] = 5.0
+    check(x, 3)
+    check(x[:5], 4)
+    check(x, 5)
