@@ -122,8 +122,9 @@ class PointTakes:
         assert x.is_cuda and x.dtype == torch.float32 and x.shape == (self.n, self.grid.xd)
         x = x.contiguous()
         # the status word is sticky: cleared only by reset_status()
-        if count_models:
-            self._counts[:-1].zero_()
+        if count_models:  # on the launches' stream: both are added to
+            with torch.cuda.stream(stream):
+                self._counts[:-1].zero_()
         hit, cand = (_lib.ptr(self.pt_hit), _lib.ptr(self.pt_cand)) if self.use_hit_masks else (None, None)
         sums, nb = _lib.ptr(self._sums), self._sums.numel() * 4
         _lib.check(lib.fbp_inside_count_chunks(_lib.ptr(x), self.n, C.byref(b), _lib.ptr(self.pt_count),

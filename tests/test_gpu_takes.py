@@ -261,3 +261,27 @@ def test_work_queue_of_many_subdomains(cuda, m):
         np.testing.assert_array_equal(_np(items)[:3 * k].reshape(-1, 3), np.array(ref, dtype=np.int64).reshape(-1, 3)[:k])
         first = np.concatenate([[0], np.cumsum([sum(1 for r in ref if r[0] == j) for j in range(m)])])
         np.testing.assert_array_equal(_np(istart), np.minimum(first, limit))
+
+
+@pytest.mark.parametrize("sized", [False, True])
+def test_lists_on_another_stream_than_the_current(cuda, sized):
+    """build(x, stream=s) with the box counts while the current stream is busy:
+    clearing the counts and chunk sums belongs to s, before its count pass."""
+    g = T.grid_of(decomposition("multilevel"))
+    n = 5000
+    x = torch.rand((n, 2), generator=torch.Generator().manual_seed(n)).cuda()
+    ref = T.PointTakes(g, n)
+    s, u = ref.build(x)
+    t = T.PointTakes(g, n, *((s, u) if sized else ()))
+    t.build(x)  # leaves counts and sums
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(50_000_000)  # tens of milliseconds
+    sizes = t.build(x, stream=side)
+    torch.cuda.synchronize()
+    t.check_status()
+    assert sizes == (None if sized else (s, u))
+    for k in ("pt_off", "np_off", "model_count"):
+        assert torch.equal(getattr(t, k), getattr(ref, k)), k
+    for k, c in (("n_take", s), ("m_take", s), ("p_take", s), ("np_take", u)):
+        assert torch.equal(getattr(t, k)[:c], getattr(ref, k)[:c]), k
