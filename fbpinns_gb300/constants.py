@@ -106,7 +106,9 @@ class Constants(ConstantsBase):
         self.autotune = True           # measure the work-item sizes on the first batch (fused step)
         self.launch_grid = 0           # CTAs of the persistent jet kernels (0 = 4 per SM)
         self.use_graph = True          # capture the step in a CUDA graph
-        self.tensor_cores = None       # forward jets on tcgen05 (3xTF32): None = where compiled, True, False
+        # jets and adjoint on tcgen05 (3xTF32): None = where compiled, True = the forward
+        # required, False = FP32 FMA kernels for both
+        self.tensor_cores = None
         self.store_z2 = None           # forward stores the layer-2 z-jets for the FMA adjoint: None = its hidden >= 32
         self.pair_headroom = 1.25      # pair-buffer capacity factor for resampled steps
         self.device_schedule = True    # fused step: follow scheduler changes on the device (no re-capture)

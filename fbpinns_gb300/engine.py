@@ -378,12 +378,15 @@ class FBPINNEngine:
         self.tensor_cores = (tc_ok and self.act != _lib.ACT_FOURIER) if tensor_cores is None else bool(tensor_cores)
         # adjoint with its layer-2 recompute and W2^T products on the tensor cores
         # (fbp_adjoint_pairs_tc): None = where it is compiled and the caller does not
-        # ask for stored z-jets; True = required; False = the FMA kernel
+        # ask for stored z-jets or, with tensor_cores=False, for FP32 kernels;
+        # True = required; False = the FMA kernel
         tca_ok = bool(_lib.load().fbp_has_tc_adjoint_shape(self.xd, self.h1, self.h2, self.d2mask, self.act))
         if tc_adjoint and not tca_ok:
             raise _lib.FBPLibraryError(f"no tensor-core adjoint kernel for layer sizes {ls} ({activation}, "
                                        f"d2mask {self.d2mask}); compiled: xd-16-16-1 and xd-32-32-1 networks")
-        self.tc_adjoint = tca_ok and (not store_z2 if tc_adjoint is None else bool(tc_adjoint))
+        if tc_adjoint is None:
+            tc_adjoint = not store_z2 and (tensor_cores is None or tensor_cores)
+        self.tc_adjoint = tca_ok and bool(tc_adjoint)
         # store_z2: the forward of a training step stores the layer-2 z-jets of
         # every pair (J * h2 floats) and the FMA adjoint reads them instead of
         # recomputing layer 2 (h1 multiply-adds per stored value); a point set

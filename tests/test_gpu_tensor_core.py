@@ -310,3 +310,20 @@ def test_tensor_core_adjoint_other_activations(cuda, act, d2, n):
     assert torch.isfinite(grads[1]).all()
     err = (grads[1] - grads[0]).abs().max(1).values / grads[0].abs().max(1).values.clamp(min=1e-30)
     assert err.max().item() <= TC_TOL, err.tolist()
+
+
+@pytest.mark.parametrize("ls,d2", [([2, 16, 16, 1], 3 | 8), ([3, 32, 32, 1], 7 | _lib.D2_GROUP(3))])
+def test_fp32_kernels_for_forward_and_adjoint_by_one_option(cuda, ls, d2):
+    """tensor_cores=False, which is all that a configuration has, selects the
+    FMA kernels for both unless the adjoint is asked for by itself."""
+    static = decomposition("wave" if ls[0] == 3 else "multilevel")
+
+    def choice(**kw):
+        eng = FBPINNEngine(static, ls, d2, **kw)
+        return eng.tensor_cores, eng.tc_adjoint
+
+    assert choice() == (True, True)
+    assert choice(tensor_cores=False) == (False, False)
+    assert choice(tensor_cores=False, tc_adjoint=True) == (False, True)
+    assert choice(tc_adjoint=False) == (True, False)
+    assert choice(store_z2=True) == (True, False)
