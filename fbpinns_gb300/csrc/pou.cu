@@ -214,17 +214,32 @@ __device__ __forceinline__ void ansatz(const fbp_problem& P, const float* xp, fl
 // Gaussians staged in shared memory as (mx, my, s^2, amp) and 1 / s^2, so that
 // the quotient is a product and one correction (q - y s^2 is exact to the last
 // bit of y) instead of a division per point and Gaussian: POU + loss of 2.1e6
-// points, 64 Gaussians 472 -> 299 us.
+// points, 64 Gaussians 472 -> 299 us.  Only where nothing in it can overflow:
+// centres and points up to GAUSS_FAR, widths s^2 in [2^-80, 2^80]; elsewhere
+// (a width of zero, say) gs is null or the point is far, and it divides.
 constexpr int GAUSS_CAP = 128;
+constexpr float GAUSS_FAR = 1e6f;
 struct Gauss {
     float4 g;
     float inv;
 };
 
+// Stages the table; the calling CTA's verdict on all of it.
+__device__ __forceinline__ const Gauss* stage_gauss(const fbp_problem& P, Gauss* gs) {
+    bool ok = P.ng <= GAUSS_CAP;
+    for (int g = threadIdx.x; ok && g < P.ng; g += blockDim.x) {
+        const float mx = P.gauss[4 * g], my = P.gauss[4 * g + 1], s2 = P.gauss[4 * g + 2] * P.gauss[4 * g + 2];
+        gs[g].g = make_float4(mx, my, s2, P.gauss[4 * g + 3]);
+        gs[g].inv = 1.0f / s2;
+        ok = s2 >= 0x1p-80f && s2 <= 0x1p80f && fabsf(mx) <= GAUSS_FAR && fabsf(my) <= GAUSS_FAR;
+    }
+    return __syncthreads_and(ok) ? gs : nullptr;
+}
+
 template <int XD>
 __device__ __forceinline__ float gauss_source(const fbp_problem& P, const Gauss* __restrict__ gs, const float* xp) {
     float f = 0.f;
-    if (P.ng <= GAUSS_CAP) {
+    if (gs && fabsf(xp[0]) <= GAUSS_FAR && fabsf(xp[XD - 1]) <= GAUSS_FAR) {
 #pragma unroll 4
         for (int g = 0; g < P.ng; ++g) {
             const float4 v = gs[g].g;
@@ -612,15 +627,9 @@ __global__ void __launch_bounds__(POU_WARPS * 32) pou_loss_kernel(fbp_problem P,
     __shared__ __align__(16) float table[POU_WARPS][SLOTCAP * RS];
     __shared__ double sh[POU_WARPS];
     pdl_wait();
-    __shared__ Gauss gs[XD == 2 ? GAUSS_CAP : 1];  // the Helmholtz source
-    if (XD == 2 && P.kind == FBP_PROBLEM_HELMHOLTZ2D && P.ng <= GAUSS_CAP) {
-        for (int g = threadIdx.x; g < P.ng; g += blockDim.x) {
-            const float s2 = P.gauss[4 * g + 2] * P.gauss[4 * g + 2];
-            gs[g].g = make_float4(P.gauss[4 * g], P.gauss[4 * g + 1], s2, P.gauss[4 * g + 3]);
-            gs[g].inv = 1.0f / s2;
-        }
-        __syncthreads();
-    }
+    __shared__ Gauss gauss_table[XD == 2 ? GAUSS_CAP : 1];  // the Helmholtz source
+    const Gauss* gs = nullptr;
+    if (XD == 2 && P.kind == FBP_PROBLEM_HELMHOLTZ2D) gs = stage_gauss(P, gauss_table);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float* T = table[w];
     const float inv_npou = 1.0f / (float)npou;

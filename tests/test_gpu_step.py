@@ -965,3 +965,35 @@ def test_fused_solution_matches_constraining_fn(cuda, name, n, monkeypatch):
     scale = max(ref.abs().max().item(), 1.0)
     assert (got - ref).abs().max().item() <= 1e-5 * scale
     assert torch.allclose(own, 2 * ref, rtol=1e-6, atol=1e-6 * scale)
+
+
+@pytest.mark.parametrize("table", ["ordinary", "capacity", "beyond", "zero_width", "tiny_width", "huge_width", "far_centre"])
+def test_helmholtz_source_over_all_widths(cuda, table):
+    """With all parameters zero the residual is the source, so the loss is the
+    mean of its square: against torch's float32 division, for tables up to and
+    beyond the staged one and for widths and centres that leave float32's
+    range squared.  Points sit on a centre and off it.  Sums of up to 129
+    float32 terms of size 1 with errors of an ulp or two of the exponent (below
+    100 where the term is not zero): 2e-5 of the loss."""
+    rng = np.random.default_rng(5)
+    n = {"capacity": 128, "beyond": 129}.get(table, 3)
+    t = np.concatenate([rng.uniform(0.1, 0.9, (n, 2)), rng.uniform(0.02, 0.1, (n, 1)), rng.uniform(0.5, 1, (n, 1))], 1)
+    t[0, :2] = 0.25, 0.75
+    odd = {"zero_width": (2, 0.0), "tiny_width": (2, 1e-20), "huge_width": (2, 1e20), "far_centre": (0, 1e25)}.get(table)
+    if odd:
+        t[0, odd[0]] = odd[1]
+    x = torch.as_tensor(rng.uniform(0, 1, (300, 2)), dtype=torch.float32)
+    if table != "zero_width":  # (0 / 0 on its centre)
+        x[7] = torch.tensor([0.25, 0.75])
+    static = decomposition("multilevel")
+    eng = FBPINNEngine(static, [2, 16, 16, 1], 3 | _lib.D2_LAPLACIAN)
+    eng.set_theta(torch.zeros_like(eng.theta))
+    p = PR.Helmholtz2D.init_params(source=t)[0]
+    eng.set_problem(PR.Helmholtz2D.fused_spec({"static": {"problem": p}}))
+    ps = eng.points(x.cuda())
+    eng.forward_pairs(ps)
+    loss = eng.pou_loss(ps).item()
+    ps.check_status()
+    ref = (PR.gaussian_sum(p["source"], x).double() ** 2).mean().item()
+    assert np.isfinite(ref) and ref > 1e-4
+    assert abs(loss - ref) <= 2e-5 * ref
