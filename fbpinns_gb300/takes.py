@@ -67,6 +67,14 @@ def grid_of(static, device="cuda"):
     return g
 
 
+def check_sizes(s, u):
+    """Pairs and slots of a point set are counted and addressed in int32."""
+    if max(s, u) >= 1 << 31:
+        raise _lib.FBPLibraryError(f"interaction lists: {s} pairs and {u} (point, level) slots, at most {(1 << 31) - 1}"
+                                   " of each; use fewer points at a time")
+    return s, u
+
+
 class PointTakes:
     """Interaction lists of one point set, built by count -> scan -> fill.
 
@@ -97,6 +105,7 @@ class PointTakes:
         self.status = self._counts[pad + nsum:]
         self.s_cap = s_cap
         self.u_cap = u_cap
+        check_sizes(s_cap or 0, u_cap or 0)
         self._alloc(s_cap or 0, u_cap or 0)
 
     def _alloc(self, s_cap, u_cap):
@@ -138,7 +147,7 @@ class PointTakes:
             h = self._counts.cpu().numpy() if count_models else None
             tot = (h[-1 - nb // 4:-1] if count_models else self._sums.cpu().numpy()).reshape(-1, 2)[:-1]
             self.model_counts = h[:self.grid.m] if count_models else None
-            s, u = int(tot[:, 0].sum(dtype=np.int64)), int(tot[:, 1].sum(dtype=np.int64))
+            s, u = check_sizes(*(int(v) for v in tot.sum(0, dtype=np.int64)))
             self._alloc(s, u)
             s_cap, u_cap = s, u
             sizes = (s, u)

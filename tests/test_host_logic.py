@@ -608,3 +608,12 @@ def test_predict_follows_points_written_in_place():
     check(x, 3)
     check(x[:5], 4)
     check(x, 5)
+
+
+def test_lists_beyond_int32_are_refused():
+    """Offsets into the lists are int32: a larger total is an error, not a wrapped offset."""
+    from fbpinns_gb300 import _lib, takes
+    assert takes.check_sizes(2 ** 31 - 1, 0) == (2 ** 31 - 1, 0)
+    for s, u in ((2 ** 31, 1), (1, 2 ** 31), (2 ** 33, 2 ** 33)):
+        with pytest.raises(_lib.FBPLibraryError):
+            takes.check_sizes(s, u)
