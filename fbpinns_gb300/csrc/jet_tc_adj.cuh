@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(TcAdj<C>::T, 32 / C::H1) adjoint_pairs_tc_kern
                 const int p2 = sp + 2 * (lane & 3);
                 const float* zr = &T.zb[p2 * A::ZS + sk];
                 const float* ar = &T.a1[p2 * A::AS + sn + (lane >> 2)];
-                const float* tr = A::SINL ? &T.tp1[p2 * A::AS + sn + (lane >> 2)] : nullptr;
+                const float* tr = A::SINL ? &T.tp1[p2 * A::AS + sn + (lane >> 2)] : ar;  // (read for sine only)
 #pragma unroll 1
                 for (int p = 0; p < np; p += 8, zr += 8 * A::ZS, ar += 8 * A::AS, tr += 8 * A::AS) {
                     float bh[NA][A::NQ][2], bl[NA][A::NQ][2];
