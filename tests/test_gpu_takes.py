@@ -285,3 +285,39 @@ def test_lists_on_another_stream_than_the_current(cuda, sized):
         assert torch.equal(getattr(t, k), getattr(ref, k)), k
     for k, c in (("n_take", s), ("m_take", s), ("p_take", s), ("np_take", u)):
         assert torch.equal(getattr(t, k)[:c], getattr(ref, k)[:c]), k
+
+
+@pytest.mark.parametrize("hits", [True, False])
+@pytest.mark.parametrize("n", [1, 255, 257, 4097, 400_001])
+def test_separate_count_scans_and_fill_give_the_same_lists(cuda, n, hits):
+    """fbp_inside_count, two fbp_scan_i32 and fbp_inside_fill, one by one,
+    against PointTakes.build (which counts and fills by chunks): both offsets
+    and all four lists."""
+    import ctypes as C
+    from fbpinns_gb300 import _lib
+    lib, P, st = _lib.load(), _lib.ptr, _lib.stream_ptr()
+    g = T.grid_of(decomposition("multilevel"))
+    x = (torch.rand((n, 2), generator=torch.Generator().manual_seed(n)) * 3 - 1).cuda()
+    t = T.PointTakes(g, n)
+    t.use_hit_masks = hits
+    s, u = t.build(x)
+    t.check_status()
+    b = g.boxes()
+    i32 = dict(dtype=torch.int32, device="cuda")
+    count, nlvl, cand = (torch.full((n,), -1, **i32) for _ in range(3))
+    lvl, hit = (torch.full((n,), -1, dtype=torch.int64, device="cuda") for _ in range(2))
+    hit_p, cand_p = (P(hit), P(cand)) if hits else (None, None)
+    _lib.check(lib.fbp_inside_count(P(x), n, C.byref(b), P(count), P(nlvl), P(lvl), None, hit_p, cand_p, st))
+    pt_off, np_off = (torch.full((n + 1,), -1, **i32) for _ in range(2))
+    nb = int(lib.fbp_scan_scratch_bytes(n))
+    scratch = torch.empty(nb // 4 + 1, **i32)
+    for src, dst in ((count, pt_off), (nlvl, np_off)):
+        _lib.check(lib.fbp_scan_i32(P(src), P(dst), n, P(scratch), nb, st))
+    assert torch.equal(pt_off, t.pt_off) and torch.equal(np_off, t.np_off)
+    n_take, m_take, p_take = (torch.full((max(s, 1),), -1, **i32) for _ in range(3))
+    np_take, status = torch.full((max(u, 1),), -1, **i32), torch.zeros(1, **i32)
+    _lib.check(lib.fbp_inside_fill(P(x), n, C.byref(b), P(pt_off), P(np_off), P(lvl), hit_p, cand_p, P(n_take), P(m_take),
+                                   P(p_take), P(np_take), s, u, P(status), st))
+    assert int(status.item()) == 0
+    for a, k, c in ((n_take, "n_take", s), (m_take, "m_take", s), (p_take, "p_take", s), (np_take, "np_take", u)):
+        assert torch.equal(a[:c], getattr(t, k)[:c]), k

@@ -327,3 +327,86 @@ def test_fp32_kernels_for_forward_and_adjoint_by_one_option(cuda, ls, d2):
     assert choice(tensor_cores=False, tc_adjoint=True) == (False, True)
     assert choice(tc_adjoint=False) == (True, False)
     assert choice(store_z2=True) == (True, False)
+
+
+@pytest.mark.parametrize("act", ["sin", "adaptive_tanh", "adaptive_sin"])
+@pytest.mark.parametrize("n", [1, 127, 129, 2000])
+def test_tensor_core_kernels_of_1d_networks_other_activations(cuda, act, n):
+    """1-32-32-1 SIREN and adaptive networks, which the engine gives the
+    tensor-core kernels by default: records and gradients (activation
+    parameters included) against the FMA kernels for the same seeds, at the
+    edges of the 128-pair tiles.  Records to TC_TOL of each component's
+    largest over 2000 points, gradients to TC_TOL of each network's largest."""
+    from helpers import boxes_static
+    static = boxes_static(np.array([[0.0], [-0.5], [0.3]], dtype=np.float32),
+                          np.array([[1.0], [1.2], [0.9]], dtype=np.float32))
+    gen = torch.Generator().manual_seed(11)
+    scale = math.sqrt(6.0) if act in ("sin", "adaptive_sin") else 1.0
+    nx = {"sin": 0, "adaptive_tanh": 1, "adaptive_sin": 2}[act]
+    layers = [tuple([(w * scale).float(), (b * scale).float()] +
+                    [(0.5 + torch.rand(b.shape, generator=gen, dtype=torch.float64)).float() for _ in range(nx)])
+              for w, b in random_layers([1, 32, 32, 1], 3, 17)]
+    x = torch.rand((2000, 1), generator=torch.Generator().manual_seed(n))
+    seeds = torch.randn((6144, 8), generator=torch.Generator().manual_seed(1)).cuda()
+
+    def run(fma, x):
+        eng = FBPINNEngine(static, [1, 32, 32, 1], 1, chunk=1024, activation=act,
+                           **(dict(tensor_cores=False, tc_adjoint=False, store_z2=False) if fma else {}))
+        assert fma or eng.tc_adjoint
+        eng.set_theta(pack_layers(layers))
+        ps = eng.points(x)
+        ps.pair_out.fill_(float("nan"))
+        eng.forward_pairs(ps)
+        rec = ps.pair_out[:ps.s].clone()
+        ps.slot_out.copy_(seeds[:ps.slot_out.shape[0], :ps.slot_out.shape[1]])
+        ps.grad_part.fill_(float("nan"))
+        grad = eng.adjoint(ps).clone()
+        torch.cuda.synchronize()
+        ps.check_status()
+        return rec, grad, eng.J
+
+    top = run(True, x)[0].abs().max(0).values
+    (r0, g0, J), (r1, g1, _) = run(True, x[:n]), run(False, x[:n])
+    assert torch.isfinite(r1[:, :2 * J]).all() and torch.isfinite(g1).all()
+    err = ((r1 - r0).abs().max(0).values / top.clamp(min=1e-30))[:2 * J]
+    assert err.max().item() <= TC_TOL, err.tolist()
+    err = (g1 - g0).abs().max(1).values / g0.abs().max(1).values.clamp(min=1e-30)
+    assert err.max().item() <= TC_TOL, err.tolist()
+
+
+def test_sine_of_pairs_over_its_range(cuda):
+    """The tensor-core kernels' sine and cosine against float64, up to and
+    across the argument (1e4) from which they call sincosf.  One 2-16-16-1
+    SIREN per argument v: layer 2's first neuron is sin(v + sin(x_n)), the only
+    one with an output weight, at a box centre with half widths of one, where
+    the window is one: u = sin v and du/dx = cos v.
+
+    Bound, as absolute error: v - j pi/2 is rounded three times below 1 (3 x
+    2^-25, times |cos| <= 0.88 where it is above a half), the polynomials once
+    at their end (2^-25) and by about 1e-8 inside: 1.25e-7.  Beyond 1e4
+    sincosf's 2 ulp are as much."""
+    from helpers import boxes_static
+    rng = np.random.default_rng(2)
+    k = np.arange(0, 6360, 53)
+    v = np.concatenate([rng.uniform(-10, 10, 1500), rng.uniform(-1e4, 1e4, 1500), k * (math.pi / 2),
+                        k * (math.pi / 2) + math.pi / 4, -k * (math.pi / 4),
+                        [0.0, -0.0, 1e-30, 1e4, -1e4, np.nextafter(np.float32(1e4), np.float32(2e4)), 12345.678, -3e5, 1e7]])
+    v = torch.as_tensor(v.astype(np.float32))
+    m = len(v)
+    static = boxes_static(np.full((m, 2), -1.0, np.float32), np.full((m, 2), 1.0, np.float32))
+    w1, b1 = torch.zeros((m, 16, 2)), torch.zeros((m, 16))
+    w2, b2 = torch.zeros((m, 16, 16)), torch.zeros((m, 16))
+    w3, b3 = torch.zeros((m, 1, 16)), torch.zeros((m, 1))
+    w1[:, 0, 0], w2[:, 0, 0], b2[:, 0], w3[:, 0, 0] = 1.0, 1.0, v, 1.0
+    b2[:, 1] = v.flip(0)  # its partner in the pair is another argument
+    eng = FBPINNEngine(static, [2, 16, 16, 1], 1, activation="sin", tensor_cores=True)
+    eng.set_theta(pack_layers([(w1, b1), (w2, b2), (w3, b3)]))
+    ps = eng.points(torch.zeros((1, 2)))
+    eng.forward_pairs(ps)
+    torch.cuda.synchronize()
+    ps.check_status()
+    rec = ps.pair_out[:ps.s].double().cpu()
+    assert ps.s == m and torch.equal(ps.takes.m_take[:m].cpu(), torch.arange(m, dtype=torch.int32))
+    assert torch.equal(rec[:, eng.J], torch.ones(m, dtype=torch.float64))
+    assert (rec[:, 0] - torch.sin(v.double())).abs().max().item() <= 1.25e-7
+    assert (rec[:, 1] - torch.cos(v.double())).abs().max().item() <= 1.25e-7
