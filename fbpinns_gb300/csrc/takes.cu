@@ -995,15 +995,13 @@ extern "C" int fbp_train_mask(const int32_t* pt_off, const int32_t* m_take, int6
     return FBP_OK;
 }
 
-extern "C" size_t fbp_work_scratch_bytes(int64_t m) { return (size_t)(m + 1) * sizeof(int32_t) * 2 + scan_scratch(m) + 256; }
+extern "C" size_t fbp_work_scratch_bytes(int64_t) { return 0; }
 
 extern "C" int fbp_build_work(const int32_t* sd_start, int64_t m, const uint8_t* select, int32_t chunk,
                               int32_t* items, int32_t* item_start, int32_t* n_items, int64_t items_cap,
-                              int32_t* status, void* scratch, size_t scratch_bytes, void* stream) {
+                              int32_t* status, void*, size_t, void* stream) {
     FBP_REQUIRE(sd_start && items && item_start && n_items && status && m > 0 && chunk > 0, FBP_ERR_INVALID,
                 "fbp_build_work: bad args");
-    FBP_REQUIRE(scratch && scratch_bytes >= fbp_work_scratch_bytes(m), FBP_ERR_CAPACITY,
-                "fbp_build_work: scratch too small");
     cudaStream_t st = as_stream(stream);
     FBP_CUDA_CHECK(launch_after(work_kernel, (int)((m + WORK_T - 1) / WORK_T), WORK_T, 0, st, sd_start, m, select, chunk,
                                 items, item_start, n_items, items_cap, status));

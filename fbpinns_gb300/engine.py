@@ -177,7 +177,6 @@ class PointSet:
         self.sd_pair, self.sd_point, self.sd_slot = self.sd_rec[:, 0], self.sd_rec[:, 1], self.sd_rec[:, 2]
         lib = _lib.load()
         self.sort_scratch = torch.empty(int(lib.fbp_sort_scratch_bytes(s_cap, m)) // 4 + 1, **i32)
-        self.work_scratch = torch.empty(int(lib.fbp_work_scratch_bytes(m)) // 4 + 1, **i32)
         # Work-item sizes: the requested ones, cut (to powers of two) so that a
         # small step still gives every SM several adjoint items and a few
         # forward items; a dynamic schedule only when there are more items than
@@ -257,17 +256,15 @@ class PointSet:
         eng = self.eng
         lib = _lib.load()
         st = _lib.stream_ptr(stream)
-        ws = self.work_scratch.numel() * 4
         _lib.check(lib.fbp_build_work(_lib.ptr(self.sd_start), eng.m, None, self.fwd_chunk, _lib.ptr(self.items_all),
                                       _lib.ptr(self.item_start_all), _lib.ptr(self.n_items_all), self.items_cap,
-                                      _lib.ptr(t_status(self)), _lib.ptr(self.work_scratch), ws, st),
-                   "fbp_build_work")
+                                      _lib.ptr(t_status(self)), None, 0, st), "fbp_build_work")
         active = eng.active if state is None else state
         self.adj_select = active.contiguous()
         _lib.check(lib.fbp_build_work(_lib.ptr(self.sd_start), eng.m, _lib.ptr(self.adj_select), self.chunk,
                                       _lib.ptr(self.items_act), _lib.ptr(self.item_start_act),
-                                      _lib.ptr(self.n_items_act), self.items_cap, _lib.ptr(t_status(self)),
-                                      _lib.ptr(self.work_scratch), ws, st), "fbp_build_work")
+                                      _lib.ptr(self.n_items_act), self.items_cap, _lib.ptr(t_status(self)), None, 0,
+                                      st), "fbp_build_work")
 
     def pairs_struct(self, adjoint=False, z2=True):
         """The launch's fbp_pairs; z2: pass the stored layer-2 z-jets buffer

@@ -324,7 +324,8 @@ int fbp_sort_pairs(const int32_t* m_take, const int32_t* n_take, const int32_t* 
 
 /* Work queue: each subdomain with select[j] != 0 (NULL = all) contributes
  * ceil(count/chunk) items (subdomain, begin, count) in subdomain order.
- * Also writes item_start (m+1): the first item of each subdomain. */
+ * Also writes item_start (m+1): the first item of each subdomain.  The one
+ * launch needs no scratch (0 bytes; scratch may be null and is not read). */
 size_t fbp_work_scratch_bytes(int64_t m);
 int fbp_build_work(const int32_t* sd_start, int64_t m, const uint8_t* select, int32_t chunk,
                    int32_t* items, int32_t* item_start, int32_t* n_items, int64_t items_cap,
