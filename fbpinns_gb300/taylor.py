@@ -236,13 +236,16 @@ def _refuse(*args):
     raise NoRule
 
 
+_wrapper = torch.Tensor._make_wrapper_subclass
+
+
 class Jet(torch.Tensor):
     """A tensor with derivative stacks; made by ``Jet.make``."""
 
     @staticmethod
     def make(v, d, dd, trace=None):
-        j = torch.Tensor._make_wrapper_subclass(Jet, v.shape, dtype=v.dtype, device=v.device)
-        j.__dict__.update(v=v, d=d, dd=dd, trace=trace)
+        j = _wrapper(Jet, v.shape, dtype=v.dtype, device=v.device)
+        j.v, j.d, j.dd, j.trace = v, d, dd, trace
         return j
 
     @classmethod
@@ -252,13 +255,17 @@ class Jet(torch.Tensor):
     @classmethod
     def __torch_function__(cls, func, types, args=(), kwargs=None):
         kwargs = kwargs or {}
-        trace = _trace_in(args) or _trace_in(kwargs)
-        if trace is None or not trace.same_modes() or \
-                not all(t in (Jet, torch.Tensor, torch.nn.Parameter) for t in types):
+        for a in args:
+            if type(a) is Jet:
+                trace = a.trace
+                break
+        else:
             _refuse(args, kwargs)
+        if not trace.same_modes() or not _TYPES.issuperset(types):
+            trace.refuse()
         with torch._C.DisableTorchFunctionSubclass():
             if func in PLAIN:
-                return func(*(a.v if isinstance(a, Jet) else a for a in args), **kwargs)
+                return func(*(a.v if type(a) is Jet else a for a in args), **kwargs)
             rule = RULES.get(func)
             if rule is None:
                 trace.refuse()
@@ -268,9 +275,11 @@ class Jet(torch.Tensor):
                 trace.refuse()
             except (TypeError, AttributeError):  # an argument that the rule does not take (alpha=, out=, dtype=)
                 trace.refuse()
-            if isinstance(out, Jet):
-                out.trace = trace
+            out.trace = trace
             return out
+
+
+_TYPES = {Jet, torch.Tensor, torch.nn.Parameter}
 
 
 def jets(fn, x, dims, u, ud, udd):
