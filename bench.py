@@ -463,8 +463,20 @@ def run_fused(args, world, rank, local):
     # by this run's pairs (traffic grows with the pairs); per variant (bytes, pairs of the capture)
     adj_dram = (ADJ_DRAM_TC if eng.tc_adjoint else ADJ_DRAM_STORED if ps.zs is not None else ADJ_DRAM_RECOMPUTE)
     traffic = adj_dram[0] / adj_dram[1] * pairs if (dom == "adjoint_pairs" and J == 4 and adj_dram) else None
-    roofline = {"bound": "fp32", "kernel": dom, "achieved": ach, "peak": best, "unit": "TFLOP/s", "frac": ach / best,
-                "peak_source": "FP32 FMA probe (fbp_fma_probe) measured in this run; MEASURED_PEAKS.json has no FP32 figure",
+    # A tensor-core kernel's contractions against the split-TF32 rate: half the measured bf16 rate
+    # over three products per useful one.  That is not what bounds it (its elementwise work fills
+    # half the issue slots: profiles/), so the FP32 probe's fraction stands beside it.
+    if eng.tc_adjoint if dom == "adjoint_pairs" else eng.tensor_cores:
+        try:
+            with open(os.path.join(os.path.dirname(os.path.abspath(__file__)), "MEASURED_PEAKS.json")) as f:
+                bf16, src = float(json.load(f)["bf16_tflops"]), "measured bf16 (MEASURED_PEAKS.json) / 6"
+        except (OSError, KeyError, ValueError):
+            bf16, src = 1900.0, "fallback bf16 1900 / 6"
+        bound, peak, src = "tensor", bf16 / 6, src + ": TF32 at half the bf16 rate, three products (3xTF32)"
+    else:
+        bound, peak, src = "fp32", best, "FP32 FMA probe (fbp_fma_probe) measured in this run"
+    roofline = {"bound": bound, "kernel": dom, "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak,
+                "peak_source": src, "fp32_probe_tflops": best, "frac_of_fp32_probe": ach / best,
                 "traffic": traffic,
                 "traffic_source": "ncu DRAM bytes of the adjoint at 2^16 points scaled by pairs" if traffic else None,
                 "kernel_ms": {k: round(v, 4) for k, v in timings.items()},

@@ -131,7 +131,9 @@ class PointTakes:
         assert x.is_cuda and x.dtype == torch.float32 and x.shape == (self.n, self.grid.xd)
         x = x.contiguous()
         # the status word is sticky: cleared only by reset_status()
-        if count_models:  # on the launches' stream: both are added to
+        if count_models and stream is None:
+            self._counts[:-1].zero_()
+        elif count_models:  # on the launches' stream, as both are added to
             with torch.cuda.stream(stream):
                 self._counts[:-1].zero_()
         hit, cand = (_lib.ptr(self.pt_hit), _lib.ptr(self.pt_cand)) if self.use_hit_masks else (None, None)
@@ -147,7 +149,7 @@ class PointTakes:
             h = self._counts.cpu().numpy() if count_models else None
             tot = (h[-1 - nb // 4:-1] if count_models else self._sums.cpu().numpy()).reshape(-1, 2)[:-1]
             self.model_counts = h[:self.grid.m] if count_models else None
-            s, u = check_sizes(*(int(v) for v in tot.sum(0, dtype=np.int64)))
+            s, u = check_sizes(int(tot[:, 0].sum(dtype=np.int64)), int(tot[:, 1].sum(dtype=np.int64)))
             self._alloc(s, u)
             s_cap, u_cap = s, u
             sizes = (s, u)
