@@ -122,6 +122,17 @@ __global__ void fma_probe_kernel(float* sink, int iters) {
     if (s == 12345.678f) sink[threadIdx.x] = s;  // keeps the chains live
 }
 
+// *differs = 1 where any word differs (a word of host memory, so that the host
+// needs no copy to read it; all writers write the same).  Two reads of 80 KB for
+// a test grid of 10^4 points: the launch is its whole cost.
+__global__ void differs_kernel(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b, int64_t n,
+                               int32_t* differs) {
+    bool d = false;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        d |= a[i] != b[i];
+    if (__syncthreads_or(d) && threadIdx.x == 0) *(volatile int32_t*)differs = 1;
+}
+
 __global__ void tanh_probe_kernel(const float* __restrict__ x, float* __restrict__ y, int64_t n) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         y[i] = tanh_fast(x[i]);
@@ -197,6 +208,16 @@ extern "C" int fbp_fma_probe(float* sink, int32_t blocks, int32_t iters, double*
     fma_probe_kernel<<<blocks, 256, 0, as_stream(stream)>>>(sink, iters);
     FBP_LAUNCH_CHECK();
     *flops_out = 2.0 * 8.0 * (double)iters * 256.0 * (double)blocks;
+    return FBP_OK;
+}
+
+extern "C" int fbp_differs(const float* a, const float* b, int64_t n, int32_t* differs, void* stream) {
+    FBP_REQUIRE(differs && n >= 0 && ((a && b) || n == 0), FBP_ERR_INVALID, "fbp_differs: bad args");
+    if (n == 0) return FBP_OK;
+    const int blocks = (int)std::min<int64_t>((n + 255) / 256, (int64_t)sm_count() * 8);
+    differs_kernel<<<blocks, 256, 0, as_stream(stream)>>>(reinterpret_cast<const uint32_t*>(a),
+                                                          reinterpret_cast<const uint32_t*>(b), n, differs);
+    FBP_LAUNCH_CHECK();
     return FBP_OK;
 }
 

@@ -162,6 +162,7 @@ class PointSet:
         self.takes = PointTakes(g, self.n, s_cap=s_cap, u_cap=u_cap)
         self.fixed_caps = caps is not None
         self._sized = False
+        self._differs = None  # start_compare's pinned word and event
         if caps is not None:
             self._allocate(int(s_cap), int(u_cap))
         self.rebuild()
@@ -284,6 +285,25 @@ class PointSet:
         if z2 and self.zs is not None:
             p.zs, p.zs_cap = _lib.ptr(self.zs), self.zs.shape[1]
         return p
+
+    def start_compare(self, x):
+        """Starts a comparison of x (n, xd float32, on the device) with this set's
+        points, word by word, on the current stream; the returned call waits for
+        it, and for nothing launched after it, and says whether they are equal."""
+        if self._differs is None:
+            self._differs = torch.zeros(1, dtype=torch.int32, pin_memory=True), torch.cuda.Event()
+        word, done = self._differs
+        differs = C.c_int32.from_address(word.data_ptr())
+        differs.value = 0
+        x = x.contiguous()
+        _lib.check(_lib.load().fbp_differs(_lib.ptr(x), _lib.ptr(self.x), x.numel(), _lib.ptr(word), _lib.stream_ptr()),
+                   "fbp_differs")
+        done.record()
+
+        def equal():
+            done.synchronize()
+            return differs.value == 0
+        return equal
 
     def subdomain_counts(self):
         """Pairs per subdomain (from the subdomain-major order), int64 on the device."""

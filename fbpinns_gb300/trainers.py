@@ -626,8 +626,8 @@ class FBPINNTrainer:
         """FBPINN solution at points x with all subdomains (the test-step inference).
 
         The interaction lists of the last points are kept, with a copy of those
-        points (the caller may write to x between calls), and used again for
-        points of the same values."""
+        points (the caller may write to x between calls, through a pointer too),
+        and used again for points of the same values."""
         x = torch.as_tensor(x, dtype=torch.float32).to(eng.device)
         with torch.no_grad():
             spec = ansatz_spec(problem, all_params, eng.xd)
@@ -639,15 +639,21 @@ class FBPINNTrainer:
                 U = eng.pou_forward(ps)
                 return problem.constraining_fn(all_params, ps.x, U[:, 0:1])
 
-            ps = getattr(eng, "_test_points", None)
-            if ps is not None and ps.x.shape == x.shape:
-                # compared on the device; read after the launches, which do not wait for it
-                same = (ps.x == x).all()
-                u = solution(ps)
-                if same.item():
+            source, ps = getattr(eng, "_test_points", (None, None))
+            if ps is not None and x.is_cuda and torch.cuda.is_current_stream_capturing():
+                # the host cannot see the values: a captured call is for the points of
+                # the last call, if that was with the same tensor
+                if x is source:
+                    return solution(ps)
+            elif ps is not None and ps.x.shape == x.shape:
+                equal = ps.start_compare(x)
+                u = solution(ps)  # launched meanwhile, and thrown away if they are not
+                if equal():
+                    eng._test_points = (x, ps)
                     return u
-            eng._test_points = eng.points(x.clone())
-            return solution(eng._test_points)
+            ps = eng.points(x.clone())
+            eng._test_points = (x, ps)
+            return solution(ps)
 
 
 class PINNTrainer(FBPINNTrainer):

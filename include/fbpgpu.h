@@ -489,6 +489,12 @@ int fbp_graph_exec_destroy(void* exec);
  * flop count of the launch. */
 int fbp_fma_probe(float* sink, int32_t blocks, int32_t iters, double* flops_out, void* stream);
 
+/* *differs = 1 where any of the n 32-bit words of a and b differ, else left as it
+ * is; differs may be pinned host memory.  For interaction lists that are kept
+ * with the points they were built for.  No counterpart in the reference, which
+ * finds the points' subdomains again (fbpinns/trainers.py:727-765). */
+int fbp_differs(const float* a, const float* b, int64_t n, int32_t* differs, void* stream);
+
 /* Evaluates the device tanh used inside the jet kernels, y[i] = tanh(x[i]),
  * so that its error can be checked against a reference tanh.  No counterpart
  * in the reference (which calls jnp.tanh, fbpinns/networks.py:64). */

@@ -997,3 +997,64 @@ def test_helmholtz_source_over_all_widths(cuda, table):
     ref = (PR.gaussian_sum(p["source"], x).double() ** 2).mean().item()
     assert np.isfinite(ref) and ref > 1e-4
     assert abs(loss - ref) <= 2e-5 * ref
+
+
+def test_predict_follows_points_on_the_device(cuda):
+    """Points written to in place between calls, by torch and by a kernel of
+    this library, against a fresh engine; a captured call replays with the
+    points of the call before it."""
+    from fbpinns_gb300.trainers import FBPINNTrainer
+    static = decomposition("multilevel")
+    layers = random_layers([2, 16, 16, 1], static["m"], seed=3)
+    ap = {"static": {"problem": PR.Poisson2D.init_params()[0]}, "trainable": {}}
+    eng = _engine(static, layers, 3)
+
+    def fresh(x):
+        return FBPINNTrainer.predict(_engine(static, layers, 3), ap, PR.Poisson2D, x.clone())
+
+    def live(x):
+        return FBPINNTrainer.predict(eng, ap, PR.Poisson2D, x)
+
+    x = torch.rand((701, 2), generator=torch.Generator().manual_seed(1)).cuda()
+    first = fresh(x)
+    assert first.abs().max() > 1e-3
+    for _ in range(2):
+        assert torch.equal(live(x), first)
+    x.copy_(x.flip(0))
+    assert torch.equal(live(x), first.flip(0))
+    x[700, 1] = 0.123
+    assert torch.equal(live(x), fresh(x))
+    eng.sample(x, 5, 0, [0.0, 0.0], [1.0, 1.0])
+    assert torch.equal(live(x), fresh(x))
+    wide = torch.zeros((701, 3), device="cuda")
+    wide[:, 1:] = x
+    assert torch.equal(live(wide[:, 1:]), fresh(x))  # (rows that are not packed, at an odd address)
+    ref = live(x)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = live(x)
+    out.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, 700_001])
+def test_points_compared_word_by_word(cuda, n):
+    """fbp_differs: equal (NaN too), the first or last word another, a sign of zero."""
+    lib, word = _lib.load(), torch.zeros(1, dtype=torch.int32).pin_memory()
+    a = torch.rand(n, generator=torch.Generator().manual_seed(n)).cuda()
+    a[n // 2] = float("nan")
+    a[0] = 0.0
+
+    def differs(b):
+        word.zero_()
+        _lib.check(lib.fbp_differs(_lib.ptr(a), _lib.ptr(b), n, _lib.ptr(word), _lib.stream_ptr()))
+        torch.cuda.synchronize()
+        return word.item()
+
+    assert differs(a.clone()) == 0
+    for i, v in ((0, -0.0), (n - 1, 2.0)):
+        b = a.clone()
+        b[i] = v
+        assert differs(b) == 1

@@ -572,7 +572,8 @@ class _FakeEngine:
     def points(self, x):
         from types import SimpleNamespace
         self.built += 1
-        return SimpleNamespace(x=x, lists=x.clone())
+        kept = x.clone()
+        return SimpleNamespace(x=x, lists=kept, start_compare=lambda y: lambda: torch.equal(x, y))
 
     def forward_pairs(self, ps, z2=True):
         pass
