@@ -627,9 +627,13 @@ __global__ void __launch_bounds__(POU_WARPS * 32) pou_loss_kernel(fbp_problem P,
     __shared__ __align__(16) float table[POU_WARPS][SLOTCAP * RS];
     __shared__ double sh[POU_WARPS];
     pdl_wait();
-    __shared__ Gauss gauss_table[XD == 2 ? GAUSS_CAP : 1];  // the Helmholtz source
+    // the Helmholtz source, with the jets that its residual takes
+    constexpr bool SOURCE = XD == 2 && (JL<XD, D2>::G == 3 || (JL<XD, D2>::sidx(0) > 0 && JL<XD, D2>::sidx(1) > 0));
+    __shared__ Gauss gauss_table[SOURCE ? GAUSS_CAP : 1];
     const Gauss* gs = nullptr;
-    if (XD == 2 && P.kind == FBP_PROBLEM_HELMHOLTZ2D) gs = stage_gauss(P, gauss_table);
+    if constexpr (SOURCE) {
+        if (P.kind == FBP_PROBLEM_HELMHOLTZ2D) gs = stage_gauss(P, gauss_table);
+    }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float* T = table[w];
     const float inv_npou = 1.0f / (float)npou;
