@@ -101,7 +101,9 @@ class Constants(ConstantsBase):
         self.engine = "fused"          # "fused" (CUDA adjoint + fused loss) or "plain" (torch autograd)
         self.resample = False          # redraw uniform collocation points every step on the device
         self.device = "cuda"
-        self.chunk = 1024              # pairs per adjoint work item
+        # pairs per adjoint work item (the size used follows the pair count: fewer for
+        # few pairs, and from 512 up to 8 times as many on the tensor-core kernels)
+        self.chunk = 1024
         self.forward_chunk = None      # pairs per forward work item (None: 4 x chunk)
         self.autotune = True           # measure the work-item sizes on the first batch (fused step)
         self.launch_grid = 0           # CTAs of the persistent jet kernels (0 = 4 per SM)

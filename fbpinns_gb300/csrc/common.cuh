@@ -143,7 +143,9 @@ __device__ __forceinline__ void adam_element(float& theta, float& m1, float& m2,
 // does nothing for kernels launched without it.  (No kernel lets the next one
 // start early: waiting CTAs then hold registers and tensor memory that the list
 // kernels on the other stream could use -- a step of 16381 redrawn points 118
-// -> 132 us, Burgers 67 -> 72.)  The 1D oscillator's step 35.0 -> 33.0 us.
+// -> 132 us, Burgers 67 -> 72.)  The forward is launched without it, and under
+// the dynamic schedule the adjoint follows the memset of its item counter, so
+// neither overlaps the end of a kernel.  The 1D oscillator's step 35.0 -> 33.0 us.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Launches a kernel that begins with pdl_wait, so that its launch overlaps the

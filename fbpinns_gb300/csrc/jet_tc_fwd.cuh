@@ -22,7 +22,7 @@
 // and the tile's two barriers.  Measured on a GB300: 2.34e6 pairs of 2-16-16-1
 // networks, J = 4, 0.161 -> 0.137 ms (operands in shared memory, one thread per
 // pair); a training step of 4096 networks 2-32-32-1 on 2.1e6 points 11.9 ->
-// 10.0 ms, of 900 networks 3-32-32-1 (J = 6) on 58^3 points 4.40 -> 3.47 ms, of
+// 9.5 ms, of 900 networks 3-32-32-1 (J = 6) on 58^3 points 4.40 -> 3.15 ms, of
 // 341 SIRENs or AdaptiveFCNs 2-16-16-1 on 65537 points 582 -> 570 and 530 -> 509
 // us (FMA kernel before).
 #pragma once

@@ -123,9 +123,9 @@ def tc_item_size(s_cap, sms, rebuilt):
     the next batch room.  Steps in us by size, the nearest to the rule's marked *:
     Poisson, 9.4e6 pairs 1024 2043, 2048 1956, 4096 1918, 6144 1893*; Helmholtz,
     1.7e7 pairs 1024 9323, 4096 8675, 8192 8465*; wave, 4.1e6 pairs 1024 3108,
-    2176 3058*, 3072 3142; SIREN, 1.8e6 pairs 1024 510, 1152 528*, 1536 524;
-    Burgers 256 67*, 512 70; Poisson, 16381 points redrawn 256 144, 512 136,
-    768 119*, 1024 131."""
+    2176 3058*, 3072 3142; Burgers 256 67*, 512 70; Poisson, 16381 points redrawn
+    256 144, 512 136, 768 119*, 1024 131.  Not the best for SIREN, 1.8e6 pairs:
+    1024 510, 1152 528*, 1536 524."""
     size = max(s_cap // (13 * sms), min(768, s_cap // (4 * sms)) if rebuilt else 0)
     return max(128, (size + 127) // 128 * 128)
 
@@ -154,7 +154,8 @@ class PointSet:
             self.pt_keep = torch.zeros(max(self.n, 1), dtype=torch.uint8, device=g.device)
             self.n_keep = torch.zeros(1, dtype=torch.int32, device=g.device)
         # requested pairs per adjoint / forward work item (the sizes used are set
-        # with the buffers: smaller for small pair counts, see _allocate)
+        # with the buffers: smaller for small pair counts, larger on the tensor-core
+        # kernels, see _allocate)
         self.chunk_req = int(chunk or engine.chunk)
         self.fwd_req = max(self.chunk_req, engine.forward_chunk)
         self.select = select
