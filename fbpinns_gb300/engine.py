@@ -713,6 +713,9 @@ def constrained_jets(cfn, all_params, x, U, xd, d2mask, need=None):
     returned.  ``need`` (optional jet indices) limits the work to the dims
     whose components are needed; the other components are zero.
     """
+    if torch.is_inference_mode_enabled():  # it turns forward mode off: the jvp's tangents would be zero
+        with torch.inference_mode(False), torch.no_grad():
+            return constrained_jets(cfn, all_params, x.clone(), U.clone(), xd, d2mask, need)
     n = x.shape[0]
     J = U.shape[1]
     out = [None] * J

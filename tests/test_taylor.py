@@ -281,3 +281,15 @@ def test_powers_beyond_the_rule_go_to_the_jvp(p, monkeypatch):
         m.setattr(taylor, "RULES", {})
         ref = engine.constrained_jets(lambda q, x, u: u + torch.tanh(x[:, 0:1]) ** p, None, x, U, 2, 3)
     torch.testing.assert_close(y, ref, rtol=1e-11, atol=1e-11, equal_nan=True)
+
+
+@pytest.mark.parametrize("name", ["burgers", "no_rule", "vmap", "function"])
+def test_jets_in_inference_mode(name):
+    """Where forward mode is off, by the rules and by the jvp, as outside."""
+    fn, p = (CASES[name][2:] if name in CASES else (PAST_THE_RULES[name], None))
+    x, U, _ = _xu()
+    ref = engine.constrained_jets(fn, p, x, U.detach(), 2, 3)
+    assert ref[:, 1:].abs().max() > 0.1
+    with torch.inference_mode():
+        y = engine.constrained_jets(fn, p, x * 1, U * 1, 2, 3)
+    torch.testing.assert_close(y, ref, rtol=1e-11, atol=1e-11)
